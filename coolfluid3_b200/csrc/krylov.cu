@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "persist.h"
 #include "spmv_node.cuh"
 
 namespace ufem {
@@ -62,6 +63,9 @@ struct KrylovWork {
   // its convergence.
   int bicg_expect[2] = {0, 0};
   int cg_expect[2] = {0, 0};   // the same for CG
+  // One-launch solves (persist.cu) per operator type: the plan of this system.
+  PersistPlan pplan[2];
+  int pplan_nc[2] = {-1, -1};  // the coarse aggregates it has room for (-1: no plan yet)
   bool use_graph = true;   // false for the allocation-free solve (instantiation allocates)
   cudaStream_t capture_stream = nullptr;
   int cg_nblk = 0;             // blocks of the fused CG kernels (more than nblk: they are latency-bound)
@@ -76,7 +80,7 @@ struct KrylovWork {
   int32_t* agg_rows = nullptr; // the members of each aggregate, ascending
   double* ainv = nullptr;      // nc x nc, row-major
   double* cvec = nullptr;      // nc: R^T r
-  double* yvec = nullptr;      // nc: Ac^-1 R^T r
+  double* yvec = nullptr;      // 2 nc: Ac^-1 R^T r (the persistent BiCGStab keeps two)
   // Two-level preconditioner of the coupled system (precond 4): point Jacobi
   // plus the same piecewise-constant correction on aggregates of pressure rows
   // (agg .. yvec above, built for the coupled rows).  Its coarse matrix, the
@@ -105,9 +109,6 @@ struct KrylovWork {
 
 namespace {
 
-// dctl slots
-constexpr int kBnorm = 0, kBeta = 1, kEst = 2, kHnext = 3, kTrue = 4;
-constexpr int kRho = 5, kRhoOld = 6, kAlpha = 7, kOmega = 8, kRhV = 9, kTS = 10, kTT = 11, kR2 = 12, kScale = 13;
 constexpr int kRedThreads = 256;
 // Blocks of the vector kernels and their reductions for n rows: one per 1024
 // rows, at most 4 a B200 SM (enough loads in flight to stream the vectors).
@@ -1447,6 +1448,84 @@ int gmres(ufem_ns_handle* h, const MT* vals, const BT* b, VT* x, VT* V, VT* w, V
   }
 }
 
+// The persistent solver's plan for this system and operator type (persist.cu).
+const PersistPlan& persist_plan_of(ufem_ns_handle* h, KrylovWork& kw, bool f32, int nc) {
+  if (kw.pplan_nc[f32] != nc) {
+    kw.pplan[f32] = persist_plan(h->start_h.data(), h->adj_h.data(), h->N, h->neq, f32, nc);
+    kw.pplan_nc[f32] = nc;
+  }
+  return kw.pplan[f32];
+}
+
+// Runs a one-launch solve to its end: kPersistIters iterations a launch (the
+// other streams' kernels get the SMs in between), as many launches as the
+// previous solve needed before the host's first look at the flags.
+constexpr int kPersistIters = 256;
+int solve_persist(KrylovWork& kw, const PersistSolve& a, const PersistPlan& plan, bool use_cg, int& expect,
+                  cudaStream_t st, SolveResult& res) {
+  res = SolveResult();
+  int rc;
+  bool first = true;
+  for (int reps = 1 + std::max(0, expect - 1) / kPersistIters, run = 0; run < a.maxit || first; reps = 1) {
+    for (int k = 0; k < reps; ++k, run += kPersistIters) {
+      rc = use_cg ? persist_cg(a, plan, first, kPersistIters, st) : persist_bicgstab(a, plan, first, kPersistIters, st);
+      if (rc) return rc;
+      first = false;
+    }
+    UFEM_CUDA_TRY(cudaMemcpyAsync(kw.h_ictl, kw.ictl, 8 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    UFEM_CUDA_TRY(cudaMemcpyAsync(kw.h_dctl, kw.dctl, 16 * sizeof(double), cudaMemcpyDeviceToHost, st));
+    UFEM_CUDA_TRY(cudaStreamSynchronize(st));
+    if (kw.h_ictl[kFlagLate]) return set_error(UFEM_ERR_CUDA, "a grid barrier of the Krylov solve ran out of time");
+    if (kw.h_ictl[0]) break;
+  }
+  res.iters = kw.h_ictl[3];
+  res.status = kw.h_ictl[2];
+  expect = res.iters;
+  const double bnorm = kw.h_dctl[kBnorm];
+  if (bnorm == 0.0) {  // a zero RHS has the zero solution
+    UFEM_CUDA_TRY(cudaMemsetAsync(a.x, 0, size_t(a.N) * a.neq * sizeof(double), st));
+    res.converged = true;
+    res.status = 0;
+    return UFEM_OK;
+  }
+  res.relres = bnorm > 0.0 ? kw.h_dctl[kTrue] / bnorm : NAN;  // a non-finite ||b|| never counts as converged
+  res.converged = res.relres <= a.tol;
+  if (res.converged) res.status = 0;
+  else if (res.status == 0) res.status = 1;
+  return UFEM_OK;
+}
+
+template <typename MT>
+PersistSolve persist_args(const ufem_ns_handle* h, const KrylovWork& kw, const MT* vals, const double* b, double* x,
+                          int pkind, double tol, int maxit) {
+  PersistSolve a;
+  a.N = h->N;
+  a.neq = h->neq;
+  a.start = h->d_start;
+  a.adj = h->d_adj;
+  a.vals = vals;
+  a.f32 = std::is_same<MT, float>::value;
+  a.diagpos = h->d_diagpos;
+  a.b = b;
+  a.x = x;
+  a.jacobi = pkind != 0;
+  if (pkind == 3 || pkind == 4) {
+    a.nc = kw.nc;
+    a.agg = kw.agg;
+    a.agg_ptr = kw.agg_ptr;
+    a.agg_rows = kw.agg_rows;
+    a.ainv = kw.ainv;
+    a.cvec = kw.cvec;
+    a.yvec = kw.yvec;
+  }
+  a.part = kw.part;
+  a.dctl = kw.dctl;
+  a.ictl = kw.ictl;
+  a.tol = tol;
+  a.maxit = maxit;
+  return a;
+}
+
 // Right-preconditioned BiCGStab with device-side scalars; the host checks the
 // done flag between blocks of iterations of growing length.
 template <typename VT, typename MT, typename BT>
@@ -1457,6 +1536,20 @@ int bicgstab(ufem_ns_handle* h, KrylovWork& kw, const MT* vals, const BT* b, VT*
   const int nblk = kw.nblk;
   const unsigned g1 = unsigned(nblk);
   int rc;
+  const double alpha_max = std::is_same<VT, float>::value ? 1e20 : 1e150;
+  if (pkind != 2) {
+    const bool f32 = std::is_same<MT, float>::value;
+    const PersistPlan& plan = persist_plan_of(h, kw, f32, pkind == 3 || pkind == 4 ? kw.nc : 0);
+    if (plan.form != kPersistNone) {
+      PersistSolve a = persist_args<MT>(h, kw, vals, b, x, pkind, tol, maxit);
+      a.r = r;
+      a.rh = rh;
+      a.q = p;
+      a.v = v;
+      a.alpha_max = alpha_max;
+      return solve_persist(kw, a, plan, false, kw.bicg_expect[f32], st, res);
+    }
+  }
   if ((rc = setup_precond<VT, MT>(h, pkind, vals, dinv, st))) return rc;
   res = SolveResult();
   if ((rc = spmv<VT, MT>(h, vals, x, v, nullptr, st))) return rc;
@@ -1468,7 +1561,6 @@ int bicgstab(ufem_ns_handle* h, KrylovWork& kw, const MT* vals, const BT* b, VT*
   fill_kernel<VT><<<g1, kRedThreads, 0, st>>>(n, VT(0), v);
   bicg_init_kernel<<<1, 1, 0, st>>>(kw.dctl, kw.ictl, tol);
   UFEM_CUDA_TRY(cudaGetLastError());
-  const double alpha_max = std::is_same<VT, float>::value ? 1e20 : 1e150;
   // the reductions with their scalar updates folded in (three launches fewer an
   // iteration), where the workspace has the fold counter (not the
   // allocation-free solve's)
@@ -1646,6 +1738,17 @@ int cg(ufem_ns_handle* h, KrylovWork& kw, const MT* vals, const BT* b, VT* x, VT
   const int nblk = kw.nblk;
   const unsigned g1 = unsigned(nblk);
   int rc;
+  if (pkind != 2) {
+    const bool f32 = std::is_same<MT, float>::value;
+    const PersistPlan& plan = persist_plan_of(h, kw, f32, pkind == 3 || pkind == 4 ? kw.nc : 0);
+    if (plan.form != kPersistNone) {
+      PersistSolve a = persist_args<MT>(h, kw, vals, b, x, pkind, tol, maxit);
+      a.r = r;
+      a.q = p;
+      a.v = z;
+      return solve_persist(kw, a, plan, true, kw.cg_expect[f32], st, res);
+    }
+  }
   if ((rc = setup_precond<VT, MT>(h, pkind, vals, dinv, st))) return rc;
   res = SolveResult();
   if ((rc = spmv<VT, MT>(h, vals, x, q, nullptr, st))) return rc;
@@ -1855,7 +1958,7 @@ int coupled_coarse_build(ufem_ns_handle* h, int max_side_2d, int max_side_3d) {
   int rc;
   if ((rc = dalloc(&kw.agg, agg.size())) || (rc = dalloc(&kw.agg_ptr, ptr.size())) ||
       (rc = dalloc(&kw.agg_rows, std::max<size_t>(rows.size(), 1))) || (rc = dalloc(&kw.ainv, size_t(nc) * nc)) ||
-      (rc = dalloc(&kw.cvec, size_t(nc))) || (rc = dalloc(&kw.yvec, size_t(nc))) ||
+      (rc = dalloc(&kw.cvec, size_t(nc))) || (rc = dalloc(&kw.yvec, size_t(2) * nc)) ||
       (rc = dalloc(&kw.cp_pos, std::max<size_t>(pos.size(), 1))) || (rc = dalloc(&kw.cp_seg, seg.size())) ||
       (rc = dalloc(&kw.cp_dst, std::max<size_t>(dst.size(), 1))) || (rc = dalloc(&kw.acd, size_t(nc) * nc)))
     return rc;
@@ -2274,7 +2377,7 @@ int krylov_set_coarse(ufem_ns_handle* h, const std::vector<int32_t>& agg, int nc
   if (!spd_inverse(A, nc)) return UFEM_OK;  // nc stays 0: the caller falls back to point Jacobi
   if ((rc = dalloc(&kw.agg, size_t(h->nrows))) || (rc = dalloc(&kw.agg_ptr, ptr.size())) ||
       (rc = dalloc(&kw.agg_rows, std::max<size_t>(rows.size(), 1))) || (rc = dalloc(&kw.ainv, A.size())) ||
-      (rc = dalloc(&kw.cvec, size_t(nc))) || (rc = dalloc(&kw.yvec, size_t(nc))))
+      (rc = dalloc(&kw.cvec, size_t(nc))) || (rc = dalloc(&kw.yvec, size_t(2) * nc)))
     return rc;
   UFEM_CUDA_TRY(cudaMemcpy(kw.agg, agg.data(), agg.size() * 4, cudaMemcpyHostToDevice));
   UFEM_CUDA_TRY(cudaMemcpy(kw.agg_ptr, ptr.data(), ptr.size() * 4, cudaMemcpyHostToDevice));
