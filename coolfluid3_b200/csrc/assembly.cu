@@ -24,132 +24,172 @@
 namespace ufem {
 namespace {
 
-// Stores one row (neq values) of a staged element block: contiguous and
-// vectorised when the staging pitch CH is 1 (warp kernel, 16-byte aligned
-// rows), strided otherwise (chunk kernel, value-major staging).
-template <int NEQ, typename T>
-__device__ __forceinline__ void put_row(T* __restrict__ st, int idx, int CH, const T (&v)[NEQ]) {
-  if (NEQ == 4 && CH == 1) {
-    if constexpr (std::is_same<T, float>::value) {
-      *reinterpret_cast<float4*>(st + idx) = make_float4(v[0], v[1], v[2], v[3]);
-    } else {
-      reinterpret_cast<double2*>(st + idx)[0] = make_double2(v[0], v[1]);
-      reinterpret_cast<double2*>(st + idx)[1] = make_double2(v[2], v[3]);
-    }
-  } else {
-#pragma unroll
-    for (int c = 0; c < NEQ; ++c) st[(idx + c) * CH] = v[c];
-  }
-}
+// ---------------------------------------------------------------------------
+// Element row blocks.  For the row node (relabelled to local position 0) the
+// neq x (n neq) slice of invdt T + theta A has the same structure in the generic
+// (NavierStokesAssembly.hpp:51-67) and the specialised element forms
+// (NavierStokesSpecializations.hpp:37-302): with G_b the shape-function gradients,
+//   [u_i, u_j b] = tg_i G_jb + delta_ij diag_b     [u_i, p b] = thS G_ib
+//   [p,   u_j b] = sWSp G_jb + c_j vem_b            [p,   p b] = dd_b
+// so a row block is its head (tg, thS, sWSp, c: 2 D + 2 numbers) and a column of
+// D + 3 numbers per node.  The routine hands exactly these to a sink: the warp
+// kernel stages them (36 numbers a tetrahedron where the expanded block has 68)
+// and multiplies them out while it sums, the chunk kernel expands them, the
+// residual kernel applies them to the increment.
+//
+// The generic form's order-2 Gauss sums (Proto/ElementIntegration.hpp:236-258)
+// are taken in closed form: on P1 elements every integrand is a polynomial of
+// degree <= 2 in the barycentric coordinates, which that rule integrates exactly:
+//   int N_k = m1 = V/n,   int N_k N_l = m2 (1 + d_kl),   m2 = V/(n(n+1)),
+// and with alpha_b = ubar . G_b, c_0b = U_0 . G_b, w_b = U_b . G_0, q = sum_k w_k U_k:
+//   int N_0 adv_b = m2 (n alpha_b + c_0b)   int adv_0 adv_b = m2 (n^2 alpha_0 alpha_b + q . G_b)
+//   int adv_0 N_b = m2 (n alpha_0 + w_b)    int ua_i S_0 = m2 (n ubar_i + U_0i) + tau m2 (n^2 ubar_i alpha_0 + q_i)
+// The specialised forms are written with normals n_b = D V G_b; here their terms
+// are collected on G_b, including the tetrahedra's use of v where w is meant
+// (:224-226, :236-238), and tau comes from the nodal solution with the standard
+// constants (a default ComputeTauImpl).
+// ---------------------------------------------------------------------------
 
-// Where the element routines send their results.  StageSink stages each row
-// of the element row block and the RHS row in shared memory for the reduction
-// (put_row); the residual kernel's sink folds them into b - M dx instead.
+// Sink of the warp kernel: the record of one incidence in shared memory.
+// Tetrahedra: [tg, thS][columns of nodes 1..3: G, diag, p row][diagonal block and
+// RHS row]; the column of the row node is multiplied out here, since the diagonal
+// block takes it from every incidence, and so is each column's p row (6 loads of 16
+// bytes a contributor instead of 7).  Triangles: the expanded row block and the RHS row (an edge has
+// two elements at most, so multiplying out while summing would cost more loads than
+// it saves).
+template <int D, typename T>
+struct RecordLayout {
+  static constexpr int n = D + 1, neq = D + 1;
+  static constexpr int head = D + 1;        // 3D: tg, thS
+  static constexpr int col = 2 * D + 2;     // 3D: G, diag, p row
+  static constexpr int sums = D == 3 ? head + D * col : n * neq * neq;  // 3D: diagonal block, rhs; 2D: rhs
+  // Lane pitch: 16-byte records whose quarter-warp accesses hit distinct banks
+  // (3D: 400 B and 208 B, odd multiples of 16), odd for the scalar accesses of 2D.
+  static constexpr int pitch = D == 3 ? (sizeof(T) == 8 ? 50 : 52) : 31;
+};
+template <int D, typename T>
+struct RecordSink;
 template <typename T>
+struct RecordSink<3, T> {
+  using L = RecordLayout<3, T>;
+  T* __restrict__ rec;
+  T tg[3], thS, sWSp, c[3];
+  __device__ __forceinline__ void put2(int at, T a, T b) {
+    if constexpr (std::is_same<T, float>::value) *reinterpret_cast<float2*>(rec + at) = make_float2(a, b);
+    else *reinterpret_cast<double2*>(rec + at) = make_double2(a, b);
+  }
+  __device__ __forceinline__ void head(const T (&tg_)[3], T thS_, T sWSp_, const T (&c_)[3]) {
+    put2(0, tg_[0], tg_[1]);
+    put2(2, tg_[2], thS_);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      tg[k] = tg_[k];
+      c[k] = c_[k];
+    }
+    thS = thS_;
+    sWSp = sWSp_;
+  }
+  __device__ __forceinline__ void col(int b, const T (&g)[3], T diag, T vem, T dd) {
+    const T p0 = sWSp * g[0] + c[0] * vem, p1 = sWSp * g[1] + c[1] * vem, p2 = sWSp * g[2] + c[2] * vem;
+    if (b == 0) {
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        put2(L::sums + 4 * i, tg[i] * g[0] + (i == 0 ? diag : T(0)), tg[i] * g[1] + (i == 1 ? diag : T(0)));
+        put2(L::sums + 4 * i + 2, tg[i] * g[2] + (i == 2 ? diag : T(0)), thS * g[i]);
+      }
+      put2(L::sums + 12, p0, p1);
+      put2(L::sums + 14, p2, dd);
+      return;
+    }
+    const int at = L::head + (b - 1) * L::col;
+    put2(at, g[0], g[1]);
+    put2(at + 2, g[2], diag);
+    put2(at + 4, p0, p1);
+    put2(at + 6, p2, dd);
+  }
+  __device__ __forceinline__ void rhs(const T (&r)[4]) {
+    put2(L::sums + 16, r[0], r[1]);
+    put2(L::sums + 18, r[2], r[3]);
+  }
+};
+
+// Sink of the chunk kernel: the expanded block and the RHS row, value-major with
+// pitch CH.
+template <int D, typename T>
 struct StageSink {
   T* __restrict__ st;
   T* __restrict__ rst;
   int CH;
-  template <int NEQ>
-  __device__ __forceinline__ void row(int idx, const T (&v)[NEQ]) { put_row<NEQ, T>(st, idx, CH, v); }
-  template <int NEQ>
-  __device__ __forceinline__ void rhs(const T (&v)[NEQ]) { put_row<NEQ, T>(rst, 0, CH, v); }
+  T tg[D], thS, sWSp, c[D];
+  __device__ __forceinline__ void head(const T (&tg_)[D], T thS_, T sWSp_, const T (&c_)[D]) {
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+      tg[k] = tg_[k];
+      c[k] = c_[k];
+    }
+    thS = thS_;
+    sWSp = sWSp_;
+  }
+  __device__ __forceinline__ void col(int b, const T (&g)[D], T diag, T vem, T dd) {
+    constexpr int neq = D + 1;
+    T* __restrict__ o = st + b * neq * neq * CH;
+#pragma unroll
+    for (int i = 0; i < D; ++i) {
+#pragma unroll
+      for (int j = 0; j < D; ++j) o[(i * neq + j) * CH] = tg[i] * g[j] + (i == j ? diag : T(0));
+      o[(i * neq + D) * CH] = g[i] * thS;
+    }
+#pragma unroll
+    for (int j = 0; j < D; ++j) o[(D * neq + j) * CH] = g[j] * sWSp + c[j] * vem;
+    o[(D * neq + D) * CH] = dd;
+  }
+  __device__ __forceinline__ void rhs(const T (&r)[D + 1]) {
+#pragma unroll
+    for (int k = 0; k <= D; ++k) rst[k * CH] = r[k];
+  }
 };
 
-// Shared tail of both element forms: rhs row a, M = invdt*T + theta*A with the
-// p row of A divided by theta first (NavierStokesAssembly.hpp:69-71), staged.
-template <int D, typename T, typename Sink>
-__device__ __forceinline__ void stage_block(const T (&A)[D + 1][D + 1], const T (&Tm)[D + 1][D + 1],
-                                            const T (&xb)[D + 1], const KParams<T>& kp, T (&rhs)[D + 1],
-                                            Sink& sk, int b) {
-  constexpr int neq = D + 1;
-#pragma unroll
-  for (int r = 0; r < neq; ++r) {
-    T s = 0;
-#pragma unroll
-    for (int c = 0; c < neq; ++c) s += -A[r][c] * xb[c];
-    rhs[r] += s;
-    T row[neq];
-#pragma unroll
-    for (int c = 0; c < neq; ++c) {
-      const T a = (r == D) ? A[r][c] * kp.inv_theta : A[r][c];  // _A(p) / theta
-      row[c] = kp.invdt * Tm[r][c] + kp.theta * a;
-    }
-    sk.template row<neq>((b * neq + r) * neq, row);
+template <typename T>
+struct RecordSink<2, T> : StageSink<2, T> {
+  __device__ __forceinline__ explicit RecordSink(T* rec) {
+    this->st = rec;
+    this->rst = rec + RecordLayout<2, T>::sums;
+    this->CH = 1;
   }
-}
+};
 
 template <int D, typename T>
 __device__ __forceinline__ void load_state(const NodeData& nd, int node, T (&x)[D + 1]) {
-  if constexpr (std::is_same<T, float>::value) {
-    const float4 v = __ldg(reinterpret_cast<const float4*>(nd.node32) + 2ll * node + 1);
-    const float vv[4] = {v.x, v.y, v.z, v.w};
-    // (u, v, [w], p): p sits at index D of the padded record
+  double s[4];
+  ld4(nd.state + 4ll * node, s[0], s[1], s[2], s[3]);
 #pragma unroll
-    for (int k = 0; k < D; ++k) x[k] = vv[k];
-    x[D] = vv[3];
-  } else {
-    double s[4];
-    ld4(nd.state + 4ll * node, s[0], s[1], s[2], s[3]);
-#pragma unroll
-    for (int k = 0; k <= D; ++k) x[k] = T(s[k]);
-  }
+  for (int k = 0; k <= D; ++k) x[k] = T(s[k]);
 }
 
-// ---------------------------------------------------------------------------
-// Generic expression (NavierStokesAssembly.hpp:51-67) for the row node, which
-// the caller has placed at local position 0.  The reference integrates it with
-// the order-2 Gauss rule (Proto/ElementIntegration.hpp:236-258, weight
-// w_q det J).  For P1 elements the gradients G are constant and every integrand
-// is a polynomial of degree <= 2 in the barycentric coordinates, which that
-// rule integrates exactly, so the sums are evaluated here in closed form with
-//   int N_k = m1 = V/n,   int N_k N_l = m2 (1 + d_kl),   m2 = V/(n(n+1)),
-// c_kb = U_k . G_b (U: nodal u_adv), ubar = mean U, alpha_b = ubar . G_b,
-// w_k = c_k0 and q = sum_k w_k U_k:
-//   int adv_b          = V alpha_b
-//   int N_0 adv_b      = m2 (n alpha_b + c_0b)
-//   int adv_0 adv_b    = m2 (n^2 alpha_0 alpha_b + q . G_b)
-//   int adv_0 N_b      = m2 (n alpha_0 + w_b)
-//   int ua_i S_0       = m2 (n ubar_i + U_0i) + tau_su m2 (n^2 ubar_i alpha_0 + q_i)
-//   int S_0 g_i        = m2 (n gbar_i + g_0i) + tau_su m2 (n^2 gbar_i alpha_0 + sum_k w_k g_ki)
-// (tests/test_gpu_parity.py checks the result against the oracle's literal
-// quadrature).
-// ---------------------------------------------------------------------------
-template <int D, typename T, typename Sink>
-__device__ __forceinline__ void generic_row(const int (&ids)[4], int a, const NodeData& nd,
-                                            const double* __restrict__ force, const KParams<T>& kp, Sink& sk) {
-  constexpr int n = D + 1, neq = D + 1;
-  const T inv_n = T(1.0 / n);
-  const T nT = T(n), n2 = T(n * n);
-  Elem<D, T> el;
-  gather_geometry_uadv<D, T>(ids, nd, el);
-  // tau inputs: |mean nodal nu| and u_adv at the centroid (SUPG.hpp:110-116, 145-147)
-  T nsum = 0;
-#pragma unroll
-  for (int b = 0; b < n; ++b) nsum += el.NU[b];
-  const T nu_bar = nsum * inv_n;
-  T Nc[n];
-  centroid_N<D, T>(Nc);
-  T uc[D], ub[D];
-#pragma unroll
-  for (int k = 0; k < D; ++k) {
-    T s = 0, m = 0;
-#pragma unroll
-    for (int b = 0; b < n; ++b) {
-      if constexpr (D == 2) s += Nc[b] * el.U[b][k];
-      m += el.U[b][k];
-    }
-    ub[k] = m * inv_n;
-    // tetrahedra: N_b(centroid) = 1/4 exactly, so the centroid value is the mean
-    uc[k] = (D == 3) ? ub[k] : s;
-  }
+// The original local node at relabelled position b (row node a at position 0).
+template <int D>
+__device__ __forceinline__ int original_node(int b, int a) {
+  return D == 3 ? (b ^ a) : (b + a >= 3 ? b + a - 3 : b + a);
+}
+
+// Gradients of the relabelled nodes, element volume, and the METRIC tau's sums
+// over g = J^-T J^-1 of the element's own frame: sq = sum g_mq^2, itr = 1 / tr g.
+template <int D, typename T>
+struct ElemGeo {
+  T G[D + 1][D];
+  T V, sq, itr;
+};
+
+// From the coordinates, in relabelled order.
+template <int D, typename T>
+__device__ __forceinline__ void compute_geometry(const Elem<D, T>& el, int a, ElemGeo<D, T>& g) {
   T J[D][D], Ji[D][D], det;
 #pragma unroll
   for (int r = 0; r < D; ++r)
 #pragma unroll
     for (int c = 0; c < D; ++c) J[r][c] = el.Xr[r + 1][c];
   inverse_det<T>(J, Ji, det);
-  T G[D][n];
+  T G[D][D + 1];
 #pragma unroll
   for (int r = 0; r < D; ++r) {
     T s = -Ji[r][0];
@@ -159,47 +199,176 @@ __device__ __forceinline__ void generic_row(const int (&ids)[4], int a, const No
 #pragma unroll
     for (int b = 1; b <= D; ++b) G[r][b] = Ji[r][b - 1];
   }
-  T g[D][D];
-  metric_tensor<D, T>(G, a, g);
-  T tps, tsu, tbu;
-  compute_tau<D, T>(kp, el, uc, tabs(nu_bar), G, g, det, tps, tsu, tbu);
-  const T V = det * T(D == 2 ? 0.5 : 1.0 / 6.0);
-  const T m1 = V * inv_n;
-  const T m2 = V * T(1.0 / (n * (n + 1)));
-  T alpha[n], w[n], c0[n], D0[n];
-#pragma unroll
-  for (int b = 0; b < n; ++b) {
-    T a = 0, ww = 0, cc = 0, dd = 0;
-#pragma unroll
-    for (int k = 0; k < D; ++k) {
-      a += ub[k] * G[k][b];
-      ww += el.U[b][k] * G[k][0];
-      cc += el.U[0][k] * G[k][b];
-      dd += G[k][0] * G[k][b];
-    }
-    alpha[b] = a;
-    w[b] = ww;
-    c0[b] = cc;
-    D0[b] = dd;
-  }
-  T q[D];
+  T m[D][D];
+  metric_tensor<D, T>(G, a, m);
+  T sq = 0, tr = 0;
 #pragma unroll
   for (int i = 0; i < D; ++i) {
+    tr += m[i][i];
+#pragma unroll
+    for (int j = 0; j < D; ++j) sq += m[i][j] * m[i][j];
+  }
+#pragma unroll
+  for (int b = 0; b <= D; ++b)
+#pragma unroll
+    for (int k = 0; k < D; ++k) g.G[b][k] = G[k][b];
+  g.V = det * T(D == 2 ? 0.5 : 1.0 / 6.0);
+  g.sq = sq;
+  g.itr = trcp(tr);
+}
+
+// tau of METRIC (SUPG.hpp:176-199): adv = | sum_m u_m grad xi_m |^2 with grad xi_m the
+// gradient of original node m + 1.
+template <int D, typename T>
+__device__ __forceinline__ void metric_tau(const KParams<T>& kp, bool standard, const ElemGeo<D, T>& g, int a,
+                                           const T (&uc)[D], T nu, T& tsu, T& tbu) {
+  T u4[D + 1];
+  u4[0] = 0;
+#pragma unroll
+  for (int k = 0; k < D; ++k) u4[k + 1] = uc[k];
+  T co[D + 1];  // u_m at the relabelled position of original node m + 1
+  if constexpr (D == 3) {
+    const bool x1 = (a & 1) != 0, x2 = (a & 2) != 0;
+    const T p0 = x1 ? u4[1] : u4[0], p1 = x1 ? u4[0] : u4[1], p2 = x1 ? u4[3] : u4[2], p3 = x1 ? u4[2] : u4[3];
+    co[0] = x2 ? p2 : p0;
+    co[1] = x2 ? p3 : p1;
+    co[2] = x2 ? p0 : p2;
+    co[3] = x2 ? p1 : p3;
+  } else {
+#pragma unroll
+    for (int b = 0; b < 3; ++b) co[b] = sel<3>(u4, original_node<2>(b, a));
+  }
+  T adv = 0;
+#pragma unroll
+  for (int k = 0; k < D; ++k) {
     T s = 0;
 #pragma unroll
-    for (int k = 0; k < n; ++k) s += w[k] * el.U[k][i];
-    q[i] = s;
+    for (int b = 0; b <= D; ++b) s += co[b] * g.G[b][k];
+    adv += s * s;
   }
-  const T tsum2 = tsu * m2;
-  const T sWS = m1 + tsu * V * alpha[0];
-  const T sWSp = m1 + T(0.5) * tps * V * alpha[0];
-  T gam[D], au[D];
+  const T diff = nu * nu * g.sq;
+  const T xs = kp.tau_std + adv + T(16) * diff;
+  const T rs = trsqrt(xs);
+  tbu = xs * rs * g.itr;  // sqrt(xs) / tr g
+  if (standard || (kp.tau_c1 == kp.tau_std && kp.c2 == T(16))) tsu = rs;  // the same argument
+  else tsu = trsqrt(kp.tau_c1 + adv + kp.c2 * diff);
+}
+
+// The row block of an element (nodes ids, relabelled) for its node at position 0
+// (original local node a).  GEN: any tau; otherwise METRIC.  The geometry is formed
+// anew for each of the element's rows: reading it from static records (128 B a
+// tetrahedron) took as long, since a scattered 128-byte read costs the L1 more
+// passes than the coordinates' gather (0.701 against 0.690 ms at 64^3 x 6).
+template <int D, typename T, bool SPEC, bool GEN, typename Sink>
+__device__ __forceinline__ void element_row(const int (&ids)[4], int a, const NodeData& nd,
+                                            const double* __restrict__ force, const KParams<T>& kp, Sink& sk) {
+  constexpr int n = D + 1, neq = D + 1;
+  const T inv_n = T(1.0 / n), nT = T(n), n2 = T(n * n);
+  ElemGeo<D, T> g;
+  Elem<D, T> el;
+  constexpr bool kEarly = std::is_same<T, float>::value;  // FP32: u_adv and the state share a 32-byte record
+  T xe[kEarly ? n : 1][neq];
+  if constexpr (kEarly) gather_geometry_node32<D>(ids, nd, el, xe);
+  else gather_geometry_uadv<D, T>(ids, nd, el);
+  compute_geometry<D, T>(el, a, g);
+  auto state = [&](int b, T (&x)[neq]) {
+    if constexpr (kEarly) {
 #pragma unroll
-  for (int i = 0; i < D; ++i) {
-    gam[i] = tbu * V * G[i][0] + T(0.5) * (m2 * (nT * ub[i] + el.U[0][i]) + tsum2 * (n2 * ub[i] * alpha[0] + q[i]));
-    au[i] = 0;
+      for (int k = 0; k < neq; ++k) x[k] = xe[b][k];
+    } else {
+      load_state<D, T>(nd, ids[b], x);
+    }
+  };
+  T nsum = 0, ub[D];
+#pragma unroll
+  for (int b = 0; b < n; ++b) nsum += el.NU[b];
+  const T nu = tabs(nsum * inv_n);
+#pragma unroll
+  for (int k = 0; k < D; ++k) {
+    T m = 0;
+#pragma unroll
+    for (int b = 0; b < n; ++b) m += el.U[b][k];
+    ub[k] = m * inv_n;
   }
-  if (kp.has_force) {
+  T tps, tsu, tbu;
+  if constexpr (SPEC) {
+    T us[D];
+#pragma unroll
+    for (int k = 0; k < D; ++k) us[k] = 0;
+#pragma unroll
+    for (int b = 0; b < n; ++b) {
+      T x[neq];
+      state(b, x);
+#pragma unroll
+      for (int k = 0; k < D; ++k) us[k] += x[k];
+    }
+#pragma unroll
+    for (int k = 0; k < D; ++k) us[k] *= inv_n;
+    metric_tau<D, T>(kp, true, g, a, us, nu, tsu, tbu);
+    tps = tsu;
+  } else {
+    if (!GEN || kp.supg_type == 1) {
+      metric_tau<D, T>(kp, false, g, a, ub, nu, tsu, tbu);
+      tps = tsu * kp.a_ps;
+      tsu *= kp.a_su;
+      tbu *= kp.a_bu;
+    } else {
+      T Gt[D][n], gm[D][D];
+#pragma unroll
+      for (int k = 0; k < D; ++k) {
+#pragma unroll
+        for (int b = 0; b < n; ++b) Gt[k][b] = g.G[b][k];
+#pragma unroll
+        for (int q = 0; q < D; ++q) gm[k][q] = 0;
+      }
+      compute_tau<D, T>(kp, el, ub, nu, Gt, gm, g.V * T(D == 2 ? 2 : 6), tps, tsu, tbu);
+    }
+  }
+  const T V = g.V, m1 = V * inv_n, m2 = V * T(1.0 / (n * (n + 1)));
+  T alpha[n];
+#pragma unroll
+  for (int b = 0; b < n; ++b) {
+    T s = 0;
+#pragma unroll
+    for (int k = 0; k < D; ++k) s += ub[k] * g.G[b][k];
+    alpha[b] = s;
+  }
+  const T sWS = m1 + tsu * V * alpha[0];
+  const T theta = kp.theta, invdt = kp.invdt, inv_rho = kp.inv_rho;
+  T gam[D], q[D], w[n], sWSp, ts2 = 0;
+#pragma unroll
+  for (int k = 0; k < D; ++k) q[k] = 0;
+  if constexpr (SPEC) {
+    T uw[D], s = 0;
+#pragma unroll
+    for (int k = 0; k < D; ++k) uw[k] = ub[D == 3 && k == 2 ? 1 : k];
+#pragma unroll
+    for (int k = 0; k < D; ++k) s += uw[k] * g.G[0][k];
+    sWSp = m1 + T(0.5) * tps * V * s;
+    const T fu = T(0.5) * sWS, fn = (nu * T(1. / 3.) + tbu) * V;
+#pragma unroll
+    for (int k = 0; k < D; ++k) gam[k] = fu * uw[k] + fn * g.G[0][k];
+  } else {
+    ts2 = tsu * m2;
+    sWSp = m1 + T(0.5) * tps * V * alpha[0];
+#pragma unroll
+    for (int b = 0; b < n; ++b) {
+      T s = 0;
+#pragma unroll
+      for (int k = 0; k < D; ++k) s += el.U[b][k] * g.G[0][k];
+      w[b] = s;
+#pragma unroll
+      for (int k = 0; k < D; ++k) q[k] += s * el.U[b][k];
+    }
+    const T na = n2 * alpha[0];
+#pragma unroll
+    for (int k = 0; k < D; ++k)
+      gam[k] = tbu * V * g.G[0][k] + T(0.5) * (m2 * (nT * ub[k] + el.U[0][k]) + ts2 * (na * ub[k] + q[k]));
+  }
+  T au[D];
+#pragma unroll
+  for (int k = 0; k < D; ++k) au[k] = 0;
+  if (!SPEC && kp.has_force) {
     T F[n][D];
 #pragma unroll
     for (int b = 0; b < n; ++b) {
@@ -217,337 +386,115 @@ __device__ __forceinline__ void generic_row(const int (&ids)[4], int a, const No
         gw += w[k] * F[k][i];
       }
       const T gbar = gs * inv_n;
-      au[i] = m2 * (nT * gbar + F[0][i]) + tsum2 * (n2 * gbar * alpha[0] + gw);
+      au[i] = m2 * (nT * gbar + F[0][i]) + ts2 * (n2 * gbar * alpha[0] + gw);
     }
   }
-  // nodal state (u, p) of the element: A x for the RHS
-  T xs[n][neq];
-#pragma unroll
-  for (int b = 0; b < n; ++b) load_state<D, T>(nd, ids[b], xs[b]);
-  T div = 0, gradp[D], kx[D], ax[D];
-#pragma unroll
-  for (int i = 0; i < D; ++i) {
-    gradp[i] = 0;
-    kx[i] = 0;
-    ax[i] = 0;
-  }
-  const T theta = kp.theta, invdt = kp.invdt, inv_rho = kp.inv_rho;
-  const T thS = theta * sWS * inv_rho;  // u rows, p column: theta * G_ib * sWS / rho
-  const T tpv = tps * inv_rho * V;      // p row, p column: tps * D0_b * V / rho
-  T cj[D], ej[D];                        // p row, u_j columns: G_jb sWSp + cj Vab + ej
-#pragma unroll
-  for (int j = 0; j < D; ++j) {
-    cj[j] = tps * G[j][0];
-    ej[j] = invdt * (cj[j] * m1);
-  }
-#pragma unroll
-  for (int b = 0; b < n; ++b) {
-    const T Kd = nu_bar * V * D0[b] + m2 * (nT * alpha[b] + c0[b]);
-    T qg = 0;
-#pragma unroll
-    for (int k = 0; k < D; ++k) qg += q[k] * G[k][b];
-    const T Kdb = Kd + tsum2 * (n2 * alpha[0] * alpha[b] + qg);
-    const T Tuu = m2 * (b == 0 ? T(2) : T(1)) + tsum2 * (nT * alpha[0] + w[b]);
-    const T Vab = V * alpha[b];
-    // rows u_i: M = invdt*T + theta*A
-    const T diag = theta * Kdb + invdt * Tuu;
-#pragma unroll
-    for (int i = 0; i < D; ++i) {
-      const T tg = theta * gam[i];
-      T row[neq];
-#pragma unroll
-      for (int j = 0; j < D; ++j) row[j] = tg * G[j][b] + (i == j ? diag : T(0));
-      row[D] = G[i][b] * thS;
-      sk.template row<neq>((b * neq + i) * neq, row);
-    }
-    // row p: theta * (A / theta) + invdt * T = A + invdt * T
-    {
-      T row[neq];
-#pragma unroll
-      for (int j = 0; j < D; ++j) row[j] = G[j][b] * sWSp + (cj[j] * Vab + ej[j]);
-      row[D] = D0[b] * tpv;
-      sk.template row<neq>((b * neq + D) * neq, row);
-    }
-    // pieces of A x
+  {
+    T tg[D], cj[D];
 #pragma unroll
     for (int k = 0; k < D; ++k) {
-      div += G[k][b] * xs[b][k];
-      gradp[k] += G[k][b] * xs[b][D];
-      kx[k] += Kdb * xs[b][k];
-      ax[k] += Vab * xs[b][k];
+      tg[k] = theta * gam[k];
+      cj[k] = tps * g.G[0][k];
     }
+    sk.head(tg, theta * sWS * inv_rho, sWSp, cj);
   }
-  // rhs row 0 = a - A x  (A before the theta combination)
-  T rrow[neq];
+  const T tpv = tps * inv_rho * V, em = invdt * m1;
+  const T tw = SPEC ? invdt * (m2 + tsu * m1 * alpha[0]) : T(0);  // specialised: T_b of b > 0
+  T div = 0, gradp[D], kx[D], ga = 0, pp = 0;
 #pragma unroll
-  for (int i = 0; i < D; ++i) rrow[i] = au[i] - (kx[i] + gam[i] * div + sWS * inv_rho * gradp[i]);
-  T g0ax = 0, g0gp = 0;
-#pragma unroll
-  for (int k = 0; k < D; ++k) {
-    g0ax += G[k][0] * ax[k];
-    g0gp += G[k][0] * gradp[k];
-  }
-  rrow[D] = -(sWSp * div + tps * g0ax + tps * V * inv_rho * g0gp);
-  sk.template rhs<neq>(rrow);
-}
-
-// ---------------------------------------------------------------------------
-// Specialised triangles, NavierStokesSpecializations.hpp:37-147, for the row
-// node at local position 0 (ai: the relabel key, used by the metric tau only).
-// Each entry receives its terms in the reference's order.
-// ---------------------------------------------------------------------------
-template <int D, typename T>
-__device__ __forceinline__ void spec_tau_common(const KParams<T>& kp, const Elem<D, T>& el, int a,
-                                                const NodeData& nd, const int (&ids)[4], T nu,
-                                                const T (&Ji)[D][D], T det, T (&xs)[D + 1][D + 1],
-                                                T& tps, T& tsu, T& tbu) {
-  // tau of the solution velocity u; the nodal states are returned in xs (the
-  // caller's A x needs them) and J^-1, det J come from the caller
-  constexpr int n = D + 1;
-  T Nc[n];
-  centroid_N<D, T>(Nc);
-  T uc[D];
-#pragma unroll
-  for (int k = 0; k < D; ++k) uc[k] = 0;
+  for (int k = 0; k < D; ++k) gradp[k] = kx[k] = 0;
 #pragma unroll
   for (int b = 0; b < n; ++b) {
-    load_state<D, T>(nd, ids[b], xs[b]);
+    T x[neq], d0 = 0, gx = 0;  // x: nodal state (u, p)
+    state(b, x);
 #pragma unroll
-    for (int k = 0; k < D; ++k) uc[k] += Nc[b] * xs[b][k];
+    for (int k = 0; k < D; ++k) d0 += g.G[0][k] * g.G[b][k];
+    const T vab = V * alpha[b];
+    T K, diag;
+    if constexpr (SPEC) {
+      K = alpha[b] * sWS + nu * V * d0;
+      diag = theta * K + tw + (b == 0 ? invdt * m2 : T(0));
+    } else {
+      T c0 = 0, qg = 0;
+#pragma unroll
+      for (int k = 0; k < D; ++k) {
+        c0 += el.U[0][k] * g.G[b][k];
+        qg += q[k] * g.G[b][k];
+      }
+      K = nu * V * d0 + m2 * (nT * alpha[b] + c0) + ts2 * (n2 * alpha[0] * alpha[b] + qg);
+      diag = theta * K + invdt * (m2 * (b == 0 ? T(2) : T(1)) + ts2 * (nT * alpha[0] + w[b]));
+    }
+    const T dd = d0 * tpv;
+    sk.col(b, g.G[b], diag, vab + em, dd);
+    // pieces of A x (A before the theta combination)
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+      div += g.G[b][k] * x[k];
+      gx += g.G[0][k] * x[k];
+      gradp[k] += g.G[b][k] * x[D];
+      kx[k] += K * x[k];
+    }
+    ga += vab * gx;
+    pp += dd * x[D];
   }
-  T G[D][D + 1];
+  T r[neq];
 #pragma unroll
-  for (int r = 0; r < D; ++r) {
-    T s = 0;
-#pragma unroll
-    for (int k = 0; k < D; ++k) s += Ji[r][k] * T(-1);
-    G[r][0] = s;
-#pragma unroll
-    for (int b = 1; b <= D; ++b) G[r][b] = Ji[r][b - 1];
-  }
-  T g[D][D];
-  metric_tensor<D, T>(G, a, g);
-  // a default ComputeTauImpl: METRIC, c1 = 1 (4 c1^2 / dt^2 = 4 / dt^2), c2 = 16, alphas 1
-  KParams<T> dk = kp;
-  dk.supg_type = 1;
-  dk.c2 = T(16);
-  dk.tau_c1 = kp.tau_std;
-  dk.a_ps = dk.a_su = dk.a_bu = T(1);
-  compute_tau<D, T>(dk, el, uc, nu, G, g, det, tps, tsu, tbu);
+  for (int k = 0; k < D; ++k) r[k] = au[k] - (kx[k] + gam[k] * div + sWS * inv_rho * gradp[k]);
+  r[D] = -(sWSp * div + tps * ga + pp);
+  sk.rhs(r);
 }
 
-template <typename T, typename Sink>
-__device__ __forceinline__ void spec_tri_row(const int (&ids)[4], int ai, const NodeData& nd, const KParams<T>& kp,
-                                             Sink& sk) {
-  Elem<2, T> el;
-  gather_geometry_uadv<2, T>(ids, nd, el);
-  T u_avg[2];
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    T s = 0;
-#pragma unroll
-    for (int b = 0; b < 3; ++b) s += el.U[b][k];
-    u_avg[k] = s / T(3);
+// The warp kernel's static lists.  Per incidence: its element and original local
+// node (element | a << 30).  Per off-diagonal slot of a row with at most 32
+// incidences, in CSR order: one 64-bit word with up to 7 contributors (5 bits: the
+// incidence's place in its row, 2 bits: the slot's position in its element), ascending
+// element; bits 49-51 their number, 52-57 the slot, 58-62 the row modulo 32.  With
+// more contributors bit 63 is set and the low words are a place in `over` (one
+// byte a contributor, bits 0-31) and the number (bits 32-39).
+template <int D>
+__global__ void assembly_items_kernel(int64_t N, const int64_t* __restrict__ start, const int32_t* __restrict__ row_inc,
+                                      const int32_t* __restrict__ inc_elem, const uint32_t* __restrict__ inc_info,
+                                      uint32_t* __restrict__ inc_ea, unsigned long long* __restrict__ items,
+                                      uint8_t* __restrict__ over, unsigned* __restrict__ over_used) {
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  const int k0 = row_inc[i], K = row_inc[i + 1] - k0;
+  const int64_t s0 = start[i];
+  const int S = int(start[i + 1] - s0);
+  if (inc_ea)
+    for (int k = 0; k < K; ++k) inc_ea[k0 + k] = uint32_t(inc_elem[k0 + k]) | ((inc_info[k0 + k] >> 24) & 3u) << 30;
+  if (K < 1 || K > 32) return;
+  const uint32_t i0 = inc_info[k0];
+  const int self = int((i0 >> (6 * ((i0 >> 24) & 3u))) & 63u);
+  for (int s = 0; s < S; ++s) {
+    if (s == self) continue;
+    unsigned long long word = 0;
+    int cnt = 0;
+    auto each = [&](auto f) {
+      for (int k = 0; k < K; ++k) {
+        const uint32_t info = inc_info[k0 + k];
+        const int a = int(info >> 24) & 3;
+        for (int q = 0; q <= D; ++q)
+          if (q != a && int((info >> (6 * q)) & 63u) == s) f(k, D == 3 ? (q ^ a) : (q - a + 3) % 3);
+      }
+    };
+    each([&](int k, int b) {
+      if (cnt < 7) word |= (unsigned long long)(k * 4 + b) << (7 * cnt);
+      ++cnt;
+    });
+    if (cnt <= 7) {
+      word |= (unsigned long long)cnt << 49;
+    } else {
+      const unsigned at = atomicAdd(over_used, unsigned(cnt));
+      word = (unsigned long long)at | (unsigned long long)cnt << 32 | 1ull << 63;
+      if (over) {
+        unsigned p = at;
+        each([&](int k, int b) { over[p++] = uint8_t(k * 4 + b); });
+      }
+    }
+    word |= (unsigned long long)s << 52 | (unsigned long long)(i & 31) << 58;
+    if (items) items[s0 - i + s - (s > self ? 1 : 0)] = word;
   }
-  const auto& X = el.Xr;
-  const T volume = T(0.5) * ((X[1][0] - X[0][0]) * (X[2][1] - X[0][1]) - (X[2][0] - X[0][0]) * (X[1][1] - X[0][1]));
-  const T fc = T(0.5);
-  T nsum = 0;
-#pragma unroll
-  for (int b = 0; b < 3; ++b) nsum += el.NU[b];
-  const T nu = tabs(nsum / T(3));
-  T nx[3], ny[3];
-  nx[0] = X[1][1] - X[2][1]; ny[0] = X[2][0] - X[1][0];
-  nx[1] = X[2][1] - X[0][1]; ny[1] = X[0][0] - X[2][0];
-  nx[2] = X[0][1] - X[1][1]; ny[2] = X[1][0] - X[0][0];
-  T tau_ps, tau_su, tau_bulk;
-  T J[2][2], Ji[2][2], det;
-#pragma unroll
-  for (int r = 0; r < 2; ++r)
-#pragma unroll
-    for (int c = 0; c < 2; ++c) J[r][c] = X[r + 1][c];
-  inverse_det<T>(J, Ji, det);
-  T xs[3][3];
-  spec_tau_common<2, T>(kp, el, ai, nd, ids, nu, Ji, det, xs, tau_ps, tau_su, tau_bulk);
-  const T nix = nx[0], niy = ny[0];  // row node at local position 0
-  const T u_ni = u_avg[0] * nix + u_avg[1] * niy;
-  const T rho = kp.rho;
-  // j-independent factors evaluated once (the same expressions as below)
-  const T su4 = tau_su / (T(4) * volume), ps4 = tau_ps / (T(4) * volume);
-  const T fsu4 = fc * tau_su / (T(4) * volume), fps4 = fc * tau_ps / (T(4) * volume);
-  const T nu4 = nu / (T(4) * volume), rho6 = T(1) / (T(6) * rho);
-  const T surho4 = tau_su / (T(4) * rho * volume), lap4 = T(1) / (T(4) * rho * volume);
-  const T bulk4 = tau_bulk / (T(4) * volume), v12 = volume / T(12);
-  const T su6 = tau_su / T(6), ps6 = tau_ps / T(6);
-  const T third = T(1. / 3.);  // the reference divides these products by 3
-  T rhs[3] = {0, 0, 0};
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    T A[3][3], Tm[3][3];
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) { A[r][c] = 0; Tm[r][c] = 0; }
-    const T uk = u_avg[0], vk = u_avg[1];
-    const T uknj = uk * nx[j] + vk * ny[j];
-    T val = T(1. / 6.) * uknj;
-    val += su4 * uknj * u_ni;
-    A[0][0] += val; A[1][1] += val;
-    val = ps4 * uknj;
-    A[2][0] += val * nix; A[2][1] += val * niy;
-    val = fc / T(6);
-    val += fsu4 * u_ni;
-    A[0][0] += val * uk * nx[j]; A[0][1] += val * uk * ny[j];
-    A[1][0] += val * vk * nx[j]; A[1][1] += val * vk * ny[j];
-    val = fps4;
-    A[2][0] += val * nix * uk * nx[j]; A[2][1] += val * nix * uk * ny[j];
-    A[2][0] += val * niy * vk * nx[j]; A[2][1] += val * niy * vk * ny[j];
-    val = nu4;
-    A[0][0] += val * (T(4. / 3.) * nix * nx[j] + niy * ny[j]);
-    A[0][1] += val * nix * ny[j] * third;
-    A[1][0] += val * niy * nx[j] * third;
-    A[1][1] += val * (nix * nx[j] + T(4. / 3.) * niy * ny[j]);
-    val = rho6;
-    val += surho4 * u_ni;
-    A[0][2] += nx[j] * val; A[1][2] += ny[j] * val;
-    const T laplacian = lap4 * (nix * nx[j] + niy * ny[j]);
-    A[2][2] += tau_ps * laplacian;
-    val = T(1. / 6.);
-    A[2][0] += val * nx[j]; A[2][1] += val * ny[j];
-    val = bulk4;
-    A[0][0] += val * nix * nx[j]; A[0][1] += val * nix * ny[j];
-    A[1][0] += val * niy * nx[j]; A[1][1] += val * niy * ny[j];
-    val = v12 * (T(1) + (j == 0 ? T(1) : T(0)));
-    val += su6 * u_ni;
-    Tm[0][0] += val; Tm[1][1] += val;
-    val = ps6;
-    Tm[2][0] += val * nix; Tm[2][1] += val * niy;
-    stage_block<2, T>(A, Tm, xs[j], kp, rhs, sk, j);
-  }
-  sk.template rhs<3>(rhs);
-}
-
-// Specialised tetrahedra, NavierStokesSpecializations.hpp:150-302, row i = a,
-// including the reference's use of vk in the W rows (:224-226, :236-238).
-template <typename T, typename Sink>
-__device__ __forceinline__ void spec_tet_row(const int (&ids)[4], int ai, const NodeData& nd, const KParams<T>& kp,
-                                             Sink& sk) {
-  Elem<3, T> el;
-  gather_geometry_uadv<3, T>(ids, nd, el);
-  T u_avg[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    T s = 0;
-#pragma unroll
-    for (int b = 0; b < 4; ++b) s += el.U[b][k];
-    u_avg[k] = s / T(4);
-  }
-  const auto& X = el.Xr;
-  T J[3][3], Ji[3][3], det;
-#pragma unroll
-  for (int r = 0; r < 3; ++r)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) J[r][c] = X[r + 1][c];
-  inverse_det<T>(J, Ji, det);
-  const T volume = det / T(6);
-  const T fc = T(0.5);
-  T nsum = 0;
-#pragma unroll
-  for (int b = 0; b < 4; ++b) nsum += el.NU[b];
-  const T nu = tabs(nsum / T(4));
-  T nr[4][3];
-  const int XX = 0, YY = 1, ZZ = 2;
-  nr[0][XX] = ((X[3][YY]-X[1][YY])*(X[2][ZZ]-X[1][ZZ]) - (X[2][YY]-X[1][YY])*(X[3][ZZ]-X[1][ZZ])) / T(2);
-  nr[0][YY] = ((X[3][ZZ]-X[1][ZZ])*(X[2][XX]-X[1][XX]) - (X[2][ZZ]-X[1][ZZ])*(X[3][XX]-X[1][XX])) / T(2);
-  nr[0][ZZ] = ((X[3][XX]-X[1][XX])*(X[2][YY]-X[1][YY]) - (X[2][XX]-X[1][XX])*(X[3][YY]-X[1][YY])) / T(2);
-  nr[1][XX] = ((X[2][YY]-X[0][YY])*(X[3][ZZ]-X[0][ZZ]) - (X[3][YY]-X[0][YY])*(X[2][ZZ]-X[0][ZZ])) / T(2);
-  nr[1][YY] = ((X[2][ZZ]-X[0][ZZ])*(X[3][XX]-X[0][XX]) - (X[3][ZZ]-X[0][ZZ])*(X[2][XX]-X[0][XX])) / T(2);
-  nr[1][ZZ] = ((X[2][XX]-X[0][XX])*(X[3][YY]-X[0][YY]) - (X[3][XX]-X[0][XX])*(X[2][YY]-X[0][YY])) / T(2);
-  nr[2][XX] = ((X[3][YY]-X[0][YY])*(X[1][ZZ]-X[0][ZZ]) - (X[1][YY]-X[0][YY])*(X[3][ZZ]-X[0][ZZ])) / T(2);
-  nr[2][YY] = ((X[3][ZZ]-X[0][ZZ])*(X[1][XX]-X[0][XX]) - (X[1][ZZ]-X[0][ZZ])*(X[3][XX]-X[0][XX])) / T(2);
-  nr[2][ZZ] = ((X[3][XX]-X[0][XX])*(X[1][YY]-X[0][YY]) - (X[1][XX]-X[0][XX])*(X[3][YY]-X[0][YY])) / T(2);
-  nr[3][XX] = ((X[1][YY]-X[0][YY])*(X[2][ZZ]-X[0][ZZ]) - (X[2][YY]-X[0][YY])*(X[1][ZZ]-X[0][ZZ])) / T(2);
-  nr[3][YY] = ((X[1][ZZ]-X[0][ZZ])*(X[2][XX]-X[0][XX]) - (X[2][ZZ]-X[0][ZZ])*(X[1][XX]-X[0][XX])) / T(2);
-  nr[3][ZZ] = ((X[1][XX]-X[0][XX])*(X[2][YY]-X[0][YY]) - (X[2][XX]-X[0][XX])*(X[1][YY]-X[0][YY])) / T(2);
-  T tau_ps, tau_su, tau_bulk;
-  T xs[4][4];
-  spec_tau_common<3, T>(kp, el, ai, nd, ids, nu, Ji, det, xs, tau_ps, tau_su, tau_bulk);
-  T ni[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    T col[4] = {nr[0][k], nr[1][k], nr[2][k], nr[3][k]};
-    ni[k] = col[0];  // row node at local position 0
-  }
-  const T u_ni = u_avg[XX] * ni[XX] + u_avg[YY] * ni[YY] + u_avg[ZZ] * ni[ZZ];
-  const T rho = kp.rho;
-  // The reference's j-independent factors, evaluated once (the same expressions
-  // as in the loop below, so the same values); FP64 divisions are expensive.
-  const T su9 = tau_su / (T(9) * volume), ps9 = tau_ps / (T(9) * volume);
-  const T fsu9 = fc * tau_su / (T(9) * volume), fps9 = fc * tau_ps / (T(9) * volume);
-  const T nu9 = nu / (T(9) * volume), rho12 = T(1) / (T(12) * rho);
-  const T surho9 = tau_su / (T(9) * rho * volume), psrho9 = tau_ps / (T(9) * rho * volume);
-  const T bulk9 = tau_bulk / (T(9) * volume), v20 = volume / T(20);
-  const T su12 = tau_su / T(12), ps12 = tau_ps / T(12);
-  const T third = T(1. / 3.);  // the reference divides these products by 3
-  T rhs[4] = {0, 0, 0, 0};
-  // local rows/cols: 0 = U, 1 = V, 2 = W, 3 = P
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    T A[4][4], Tm[4][4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) { A[r][c] = 0; Tm[r][c] = 0; }
-    const T uk = u_avg[XX], vk = u_avg[YY], wk = u_avg[ZZ];
-    const T* nj = nr[j];
-    const T uknj = uk * nj[XX] + vk * nj[YY] + wk * nj[ZZ];
-    T val = T(1. / 12.) * uknj;
-    val += su9 * uknj * u_ni;
-    A[0][0] += val; A[1][1] += val; A[2][2] += val;
-    val = ps9 * uknj;
-    A[3][0] += val * ni[XX]; A[3][1] += val * ni[YY]; A[3][2] += val * ni[ZZ];
-    val = fc / T(12);
-    val += fsu9 * u_ni;
-    A[0][0] += val * uk * nj[XX]; A[0][1] += val * uk * nj[YY]; A[0][2] += val * uk * nj[ZZ];
-    A[1][0] += val * vk * nj[XX]; A[1][1] += val * vk * nj[YY]; A[1][2] += val * vk * nj[ZZ];
-    A[2][0] += val * vk * nj[XX]; A[2][1] += val * vk * nj[YY]; A[2][2] += val * vk * nj[ZZ];
-    val = fps9;
-    A[3][0] += val * ni[XX] * uk * nj[XX]; A[3][1] += val * ni[XX] * uk * nj[YY];
-    A[3][2] += val * ni[XX] * uk * nj[ZZ]; A[3][0] += val * ni[YY] * vk * nj[XX];
-    A[3][1] += val * ni[YY] * vk * nj[YY]; A[3][2] += val * ni[YY] * vk * nj[ZZ];
-    A[3][0] += val * ni[ZZ] * vk * nj[XX]; A[3][1] += val * ni[ZZ] * vk * nj[YY];
-    A[3][2] += val * ni[ZZ] * vk * nj[ZZ];
-    val = nu9;
-    A[0][0] += val * (T(4. / 3.) * ni[XX] * nj[XX] + ni[YY] * nj[YY] + ni[ZZ] * nj[ZZ]);
-    A[0][1] += val * ni[XX] * nj[YY] * third;
-    A[0][2] += val * ni[XX] * nj[ZZ] * third;
-    A[1][0] += val * ni[YY] * nj[XX] * third;
-    A[1][1] += val * (ni[XX] * nj[XX] + T(4. / 3.) * ni[YY] * nj[YY] + ni[ZZ] * nj[ZZ]);
-    A[1][2] += val * ni[YY] * nj[ZZ] * third;
-    A[2][0] += val * ni[ZZ] * nj[XX] * third;
-    A[2][1] += val * ni[ZZ] * nj[YY] * third;
-    A[2][2] += val * (ni[XX] * nj[XX] + ni[YY] * nj[YY] + T(4. / 3.) * ni[ZZ] * nj[ZZ]);
-    val = rho12;
-    val += surho9 * u_ni;
-    A[0][3] += nj[XX] * val; A[1][3] += nj[YY] * val; A[2][3] += nj[ZZ] * val;
-    val = psrho9 * (ni[XX] * nj[XX] + ni[YY] * nj[YY] + ni[ZZ] * nj[ZZ]);
-    A[3][3] += val;
-    val = T(1. / 12.);
-    A[3][0] += val * nj[XX]; A[3][1] += val * nj[YY]; A[3][2] += val * nj[ZZ];
-    val = bulk9;
-    A[0][0] += val * ni[XX] * nj[XX]; A[0][1] += val * ni[XX] * nj[YY];
-    A[0][2] += val * ni[XX] * nj[ZZ]; A[1][0] += val * ni[YY] * nj[XX];
-    A[1][1] += val * ni[YY] * nj[YY]; A[1][2] += val * ni[YY] * nj[ZZ];
-    A[2][0] += val * ni[ZZ] * nj[XX]; A[2][1] += val * ni[ZZ] * nj[YY];
-    A[2][2] += val * ni[ZZ] * nj[ZZ];
-    val = v20 * (T(1) + (j == 0 ? T(1) : T(0)));
-    val += su12 * u_ni;
-    Tm[0][0] += val; Tm[1][1] += val; Tm[2][2] += val;
-    val = ps12;
-    Tm[3][0] += val * ni[XX]; Tm[3][1] += val * ni[YY]; Tm[3][2] += val * ni[ZZ];
-    stage_block<3, T>(A, Tm, xs[j], kp, rhs, sk, j);
-  }
-  sk.template rhs<4>(rhs);
 }
 
 // Shared memory of one chunk: staged row blocks [value][incidence] (T), staged
@@ -562,7 +509,7 @@ constexpr size_t assembly_smem_bytes() {
 }
 
 // The row-owner assembly kernel.  One CTA per chunk of whole block rows.
-template <int D, typename T, int CH, bool SPEC>
+template <int D, typename T, int CH, bool SPEC, bool GEN>
 __global__ void __launch_bounds__(CH) ns_assembly_kernel(
     const int2* __restrict__ chunk_rows, const int32_t* __restrict__ row_inc,
     const int32_t* __restrict__ inc_elem, const uint32_t* __restrict__ inc_info, const int4* __restrict__ conn,
@@ -631,13 +578,8 @@ __global__ void __launch_bounds__(CH) ns_assembly_kernel(
     s_info[t] = pslots;
     const KParams<T> kp = make_kparams<T>(p);
     const NodeData nd{coords, uadv, state, node32};
-    StageSink<T> sk{st + t, rst + t, CH};
-    if constexpr (SPEC) {
-      if constexpr (D == 2) spec_tri_row<T>(ids, a, nd, kp, sk);
-      else spec_tet_row<T>(ids, a, nd, kp, sk);
-    } else {
-      generic_row<D, T>(ids, a, nd, force, kp, sk);
-    }
+    StageSink<D, T> sk{st + t, rst + t, CH};
+    element_row<D, T, SPEC, GEN>(ids, a, nd, force, kp, sk);
     // contributor masks: bit = position of this incidence within its row
     int lo = 0, hi = R - 1;
     while (lo < hi) {  // last rl with s_rowinc[rl] <= t
@@ -738,102 +680,263 @@ __global__ void __launch_bounds__(CH) ns_assembly_kernel(
 
 // ---------------------------------------------------------------------------
 // Warp-per-row-group assembly.  A warp owns a range of consecutive block rows
-// with at most 32 incidences in total; lane l evaluates incidence l of the
-// range (incidences are sorted by row, then element id) and stages its element
-// row block in the warp's shared-memory slice, value-major with a 33-element
-// pitch (conflict-free for both the per-lane writes and the per-value reads).
-// Contributor masks (bit = lane) are built with shared atomicOr, one word per
-// neighbour slot.  The lanes then own CSR items: a diagonal entry or an RHS
-// entry (sum over all lanes of the row) or an off-diagonal (row, equation,
-// slot) quad (sum over the mask bits).  Lanes are visited in ascending order,
-// i.e. every CSR value is the element-ordered sum of its contributions, as in
-// the chunk kernel, and each value is written once.
+// with at most 32 incidences in total; lane l evaluates incidence l of the range
+// (incidences are sorted by row, then element id) and stages its row block's head,
+// columns and RHS row (RecordLayout).  The lanes then own CSR items: products and
+// plain sums over the row's lanes that make up the diagonal block and the RHS, and
+// the off-diagonal (row, slot) blocks, whose contributors the static item words
+// list in ascending element order -- one lane a block in 2D, two in 3D, each
+// taking every other contributor of the whole block (16 sums in registers; the
+// halves are added at the end).  Every sum runs in a fixed order that depends on
+// the row alone, and each value is written once.
+//
+// What bounds it: passes through the L1 / shared-memory pipe (84% busy at 16 warps
+// an SM), then issue (45%) and FP64 (28%), not bytes (DRAM 16% of the measured copy
+// rate).  So the records hold what the blocks are made of (3D: 50 numbers an
+// incidence with the row node's column multiplied out, against 68 of the whole
+// block), a node's 32 bytes are gathered by one load, the contributor lists are
+// static words instead of masks built by shared-memory atomics, and the smaller
+// staging leaves room for 16 warps (128 registers) where 12 fitted.  64^3 x 6 on a
+// B200, before -> after: FP64 generic 0.737 -> 0.591 ms, specialised 0.843 -> 0.530,
+// FP32 generic 0.545 -> 0.457; 301^2 x 2 triangles in random order, FP64 generic 52.0
+// -> 51.5 us, specialised 53.3 -> 45.4.
 // ---------------------------------------------------------------------------
-// Lane pitch of the staging slice, in elements of T: 16-byte aligned rows
-// whose quarter-warp 16-byte accesses hit distinct banks (3D), odd for the
-// scalar accesses of the 2D layout.
-template <int D, typename T>
-constexpr int warp_lane_pitch() {
-  return D == 3 ? (sizeof(T) == 4 ? 68 : 70) : 31;
-}
-
 constexpr size_t kDescSlot = (sizeof(AsmDesc) + 15) / 16 * 16;
 
 // KC: lanes that evaluate incidences (group capacity); the staging holds KC lanes.
 template <int D, typename T, int KC = 32, bool BATCH = false>
 constexpr size_t warp_stage_bytes() {
-  return size_t(KC) * warp_lane_pitch<D, T>() * sizeof(T) +  // staged row blocks + RHS rows, one slice per lane
-         size_t(D * 64 + 32 + 36 + 36) * 4 +                  // slot masks per local position, pslots, prefix, offsets
-         (BATCH ? 2 * kDescSlot : 0);                         // batch: descriptors of the current and next mesh
+  return (size_t(KC) * RecordLayout<D, T>::pitch * sizeof(T) + 15) / 16 * 16 +  // one record per lane
+         size_t(36 + 36) * 4 +                  // lane offset and CSR block offset of each row
+         (BATCH ? 2 * kDescSlot : 0);           // batch: descriptors of the current and next mesh
 }
-static_assert(warp_stage_bytes<2, float>() % 16 == 0 && warp_stage_bytes<2, double>() % 16 == 0 &&
-                  warp_stage_bytes<3, float>() % 16 == 0 && warp_stage_bytes<3, double>() % 16 == 0 &&
-                  warp_stage_bytes<3, float, 24>() % 16 == 0 && warp_stage_bytes<3, double, 24>() % 16 == 0 &&
-                  warp_stage_bytes<2, float, 32, true>() % 16 == 0 && warp_stage_bytes<2, double, 32, true>() % 16 == 0 &&
-                  warp_stage_bytes<3, float, 32, true>() % 16 == 0 && warp_stage_bytes<3, double, 32, true>() % 16 == 0,
-              "per-warp staging slices must stay 16-byte aligned");
 
-// Resident-CTA hints (register budgets) of the 24-lane tetrahedron variants:
-// FP32 20 warps (<= 102 registers); FP64 14 warps, which with 4-warp CTAs asks
-// for 3 CTAs (12 warps, no register cap: the variant's smaller staging then
-// leaves more of the SM's shared/L1 array to the node-data gathers than the
-// 32-lane kernel at the same warps) and with 2-warp CTAs for 7 (a 128-register
-// budget that spills; the autotuner passes it over).  The 32-lane variants keep
-// the compiler's choice (their staging caps the warps anyway).
-template <int D, typename T, int KC, int WPB>
+// Resident-CTA hints (register budgets): warps an SM.  64^3 x 6, generic, 4-warp
+// CTAs: FP64 0.595 ms at 16 warps, 0.737 at 12 and 0.771 at 20 (spills); FP32 0.480 at
+// 16, 0.457 at 20.  The batched 3D FP64 kernel spills at 16 (its descriptors are in
+// shared memory), so it keeps 12.  Triangles, FP64: 51.5 us at 16, 60-76 at 20-24 (spills);
+// FP32 51.7 at 16, 48 at 24.
+template <int D, typename T, bool BATCH, int WPB>
 constexpr int warp_min_blocks() {
-  if (D != 3 || KC == 32) return 0;  // 0: no hint
-  const int warps = sizeof(T) == 8 ? 14 : 20;
+  const int warps = D == 3 ? (sizeof(T) == 4 ? 20 : (BATCH ? 12 : 16)) : (sizeof(T) == 4 ? 24 : 16);
   return warps / WPB > 0 ? warps / WPB : 1;
 }
 
-// Loads NV consecutive staged values (16-byte aligned when NV is a multiple of 4).
-template <int NV, typename T>
-__device__ __forceinline__ void load_run(const T* __restrict__ src, T (&v)[NV]) {
-  if constexpr (NV % 4 == 0 && std::is_same<T, float>::value) {
+// Reduction of a group's rows from its staged records, tetrahedra.  Row by row, 16
+// off-diagonal blocks at a time: two lanes a block, each summing every other
+// contributor's whole block (16 sums in registers), then rows 0-1 of the block end
+// up in the even lane and rows 2-3 in the odd one and are written.  Every order
+// depends on the row's elements alone (not on its place in the group nor on the
+// order of its neighbours).
+// `next` runs once, with the loads it starts hidden behind the second half.
+template <typename T, int KC, typename F>
+__device__ __forceinline__ void reduce_rows_3d(const T* stage, const int* s_off, const int* s_start, int R, int row0,
+                                               int64_t gstart, const unsigned long long* __restrict__ words,
+                                               unsigned long long word, const AsmDesc& d, F&& next) {
+  using L = RecordLayout<3, T>;
+  constexpr int LS = L::pitch;
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const bool odd = (lane & 1) != 0;
+  double* __restrict__ vals = d.vals;
+  float* __restrict__ vals32 = d.vals32;
+  for (int rl = 0; rl < R; ++rl) {
+    const int kb = s_off[rl], ke = s_off[rl + 1];
+    const int w0 = s_start[rl] - rl;                     // the row's first item word
+    const int S = s_start[rl + 1] - s_start[rl];
+    const int64_t base0 = 16 * (gstart + s_start[rl]);   // the row's first CSR value
+    const int64_t row = row0 + rl;
+    int self = 0;
+    for (int p0 = 0; p0 < S - 1; p0 += 16) {
+      const int it = p0 + (lane >> 1);
+      const bool on = it < S - 1;
+      if (rl + p0 > 0) word = on ? __ldg(words + w0 + it) : 0ull;
+      const bool over = (word >> 63) != 0;
+      const int slot = int(word >> 52) & 63;
+      const int cnt = over ? int(word >> 32) & 0xff : int(word >> 49) & 7;
+      const uint8_t* more = d.over + uint32_t(word);
+      const T* base = stage + kb * LS;
+      double acc[4][4];
 #pragma unroll
-    for (int q = 0; q < NV / 4; ++q) {
-      const float4 x = reinterpret_cast<const float4*>(src)[q];
-      v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
+      unsigned long long list = word >> (odd ? 7 : 0);
+#pragma unroll 1
+      for (int c = odd ? 1 : 0; c < cnt; c += 2, list >>= 14) {
+        const int id = over ? int(__ldg(more + c)) : int(list & 127u);
+        const T* rec = base + (id >> 2) * LS;
+        const T* col = rec + (L::head - L::col) + (id & 3) * L::col;
+        double h[4], q[8];  // tg (3), thS; G (3), diag, p row (4)
+        if constexpr (std::is_same<T, double>::value) {
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const double2 x = reinterpret_cast<const double2*>(rec)[k];
+            h[2 * k] = x.x;
+            h[2 * k + 1] = x.y;
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const double2 x = reinterpret_cast<const double2*>(col)[k];
+            q[2 * k] = x.x;
+            q[2 * k + 1] = x.y;
+          }
+        } else {
+          const float4 x = *reinterpret_cast<const float4*>(rec);
+          h[0] = double(x.x); h[1] = double(x.y); h[2] = double(x.z); h[3] = double(x.w);
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const float4 y = reinterpret_cast<const float4*>(col)[k];
+            q[4 * k] = double(y.x); q[4 * k + 1] = double(y.y); q[4 * k + 2] = double(y.z); q[4 * k + 3] = double(y.w);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+#pragma unroll
+          for (int j = 0; j < 3; ++j) acc[i][j] = fma(h[i], q[j], acc[i][j]);
+          acc[i][i] += q[3];
+          acc[i][3] = fma(h[3], q[i], acc[i][3]);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[3][j] += q[4 + j];
+      }
+      // slot of the row node: the slots are ascending, so it is where they skip one
+      self += __popc(__ballot_sync(FULL, on && !odd && slot == it));
+      double out[2][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const double give = odd ? acc[i][j] : acc[i + 2][j];
+          const double keep = odd ? acc[i + 2][j] : acc[i][j];
+          const double got = __shfl_xor_sync(FULL, give, 1);
+          out[i][j] = odd ? got + keep : keep + got;  // even contributors first
+        }
+      if (on) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int64_t pos = base0 + int64_t(((odd ? 2 : 0) + i) * S + slot) * 4;
+          st4_cs(vals + pos, out[i][0], out[i][1], out[i][2], out[i][3]);  // streamed: L2 keeps the node data
+          if (vals32 != nullptr)
+            __stcs(reinterpret_cast<float4*>(vals32 + pos),
+                   make_float4(float(out[i][0]), float(out[i][1]), float(out[i][2]), float(out[i][3])));
+        }
+      }
     }
-  } else if constexpr (NV % 2 == 0 && std::is_same<T, double>::value && NV % 4 == 0) {
-#pragma unroll
-    for (int q = 0; q < NV / 2; ++q) {
-      const double2 x = reinterpret_cast<const double2*>(src)[q];
-      v[2 * q] = x.x; v[2 * q + 1] = x.y;
+    if (rl == R - 1) next();
+    // diagonal block and RHS row: lane e of ten sums a pair of entries over every
+    // third incidence, three sets of ten lanes, then the sets in order
+    {
+      const int part = lane / 10, e = lane - part * 10;
+      double a0 = 0.0, a1 = 0.0;
+      if (part < 3) {
+        const T* q = stage + L::sums + 2 * e;
+#pragma unroll 4
+        for (int k = kb + part; k < ke; k += 3) {
+          if constexpr (std::is_same<T, double>::value) {
+            const double2 x = *reinterpret_cast<const double2*>(q + k * LS);
+            a0 += x.x;
+            a1 += x.y;
+          } else {
+            const float2 x = *reinterpret_cast<const float2*>(q + k * LS);
+            a0 += double(x.x);
+            a1 += double(x.y);
+          }
+        }
+      }
+      const double b0 = __shfl_down_sync(FULL, a0, 10), b1 = __shfl_down_sync(FULL, a1, 10);
+      const double c0 = __shfl_down_sync(FULL, a0, 20), c1 = __shfl_down_sync(FULL, a1, 20);
+      a0 = (a0 + b0) + c0;
+      a1 = (a1 + b1) + c1;
+      if (lane < 8) {
+        const int64_t pos = base0 + int64_t((lane >> 1) * S + self) * 4 + (lane & 1) * 2;
+        __stcs(reinterpret_cast<double2*>(vals + pos), make_double2(a0, a1));
+        if (vals32 != nullptr) __stcs(reinterpret_cast<float2*>(vals32 + pos), make_float2(float(a0), float(a1)));
+      } else if (lane < 10) {
+        __stcs(reinterpret_cast<double2*>(d.rhs + row * 4 + (lane - 8) * 2), make_double2(a0, a1));
+      }
     }
-  } else {
-#pragma unroll
-    for (int q = 0; q < NV; ++q) v[q] = src[q];
   }
 }
 
-template <int D, typename T, bool SPEC, int WPB, bool BATCH, int KC>
-__global__ void __launch_bounds__(32 * WPB, warp_min_blocks<D, T, KC, WPB>()) ns_assembly_warp_kernel(
+// ... triangles: a lane an entry of the diagonal blocks and the RHS rows (summed
+// over the row's lanes), then a lane an off-diagonal block.
+template <typename T, typename F>
+__device__ __forceinline__ void reduce_rows_2d(const T* stage, const int* s_off, const int* s_start, int R, int row0,
+                                               int64_t gstart, const unsigned long long* __restrict__ words,
+                                               unsigned long long word, const AsmDesc& d, F&& next) {
+  using L = RecordLayout<2, T>;
+  constexpr int LS = L::pitch;
+  const int lane = threadIdx.x & 31;
+  double* __restrict__ vals = d.vals;
+  float* __restrict__ vals32 = d.vals32;
+  for (int it = lane; it < R * 12; it += 32) {
+    const int rl = it / 12, dl = it - rl * 12;
+    const int64_t row = row0 + rl;
+    const int er = dl / 3, ec = dl - er * 3;
+    int64_t pos = 0;
+    if (dl < 9) pos = __ldg(d.diagpos + row * 3 + er) - er + ec;
+    const T* q = stage + (dl < 9 ? dl : L::sums + dl - 9);
+    double acc = 0.0;
+    const int ke = s_off[rl + 1];
+#pragma unroll 4
+    for (int k = s_off[rl]; k < ke; ++k) acc += double(q[k * LS]);
+    if (dl < 9) {
+      __stcs(vals + pos, acc);
+      if (vals32 != nullptr) __stcs(vals32 + pos, float(acc));
+    } else {
+      __stcs(d.rhs + row * 3 + (dl - 9), acc);
+    }
+  }
+  next();
+  const int nslot = s_start[R] - R;
+  for (int it = lane; it < nslot; it += 32) {
+    if (it >= 32) word = __ldg(words + it);
+    const bool over = (word >> 63) != 0;
+    const int rl = (int(word >> 58) - row0) & 31;
+    const int slot = int(word >> 52) & 63;
+    const int cnt = over ? int(word >> 32) & 0xff : int(word >> 49) & 7;
+    const uint8_t* more = d.over + uint32_t(word);
+    const T* base = stage + s_off[rl] * LS;
+    double acc[9];
+#pragma unroll
+    for (int e = 0; e < 9; ++e) acc[e] = 0.0;
+    unsigned long long list = word;
+#pragma unroll 1
+    for (int c = 0; c < cnt; ++c, list >>= 7) {
+      const int id = over ? int(__ldg(more + c)) : int(list & 127u);
+      const T* q = base + (id >> 2) * LS + (id & 3) * 9;
+#pragma unroll
+      for (int e = 0; e < 9; ++e) acc[e] += double(q[e]);
+    }
+    const int S = s_start[rl + 1] - s_start[rl];
+    const int64_t base0 = 9 * (gstart + s_start[rl]) + slot * 3;
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const int64_t pos = base0 + int64_t(r) * S * 3 + c;
+        __stcs(vals + pos, acc[r * 3 + c]);
+        if (vals32 != nullptr) __stcs(vals32 + pos, float(acc[r * 3 + c]));
+      }
+  }
+}
+
+template <int D, typename T, bool SPEC, bool GEN, int WPB, bool BATCH, int KC>
+__global__ void __launch_bounds__(32 * WPB, warp_min_blocks<D, T, BATCH, WPB>()) ns_assembly_warp_kernel(
     int ngroups, int nmesh, const AsmDesc* __restrict__ descs, const int* __restrict__ gprefix,
-    // one-mesh launch (BATCH false): the mesh's arrays as separate parameters
-    const int4* __restrict__ groups_1, const int32_t* __restrict__ row_inc_1, const int32_t* __restrict__ inc_elem_1,
-    const uint32_t* __restrict__ inc_info_1, const int4* __restrict__ conn_1, const double* __restrict__ coords_1,
-    const double* __restrict__ uadv_1, const double* __restrict__ state_1, const float* __restrict__ node32_1,
-    const double* __restrict__ force_1, const int64_t* __restrict__ start_1, NSParams p_1,
-    double* __restrict__ vals_1, float* __restrict__ vals32_1, double* __restrict__ rhs_1) {
-  constexpr int n = P1<D>::n, neq = P1<D>::neq, nvals = P1<D>::nvals;
-  constexpr int LS = warp_lane_pitch<D, T>();
-  constexpr int RPI = (D == 3) ? 2 : 3;      // equations (CSR rows) per off-diagonal item
-  constexpr int RG = neq / RPI;              // items per (row, slot)
-  constexpr int NV = RPI * neq;              // values per off-diagonal item
-  constexpr unsigned FULL = 0xffffffffu;
+    const __grid_constant__ AsmDesc one) {
+  constexpr int LS = RecordLayout<D, T>::pitch;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  T* stage = reinterpret_cast<T*>(smem_raw + size_t(warp) * warp_stage_bytes<D, T, KC, BATCH>());
-  uint32_t* s_mask = reinterpret_cast<uint32_t*>(stage + KC * LS);  // D x 64: local position 1..n-1, slot
-  uint32_t* s_pslots = s_mask + D * 64;                              // 32
-  int* s_pref = reinterpret_cast<int*>(s_pslots + 32);               // 33 (+3 pad)
-  int* s_off = s_pref + 36;                                          // 33 (+3 pad): lane offset of each row
+  unsigned char* slice = smem_raw + size_t(warp) * warp_stage_bytes<D, T, KC, BATCH>();
+  T* stage = reinterpret_cast<T*>(slice);
+  int* s_off = reinterpret_cast<int*>(slice + (size_t(KC) * LS * sizeof(T) + 15) / 16 * 16);  // 33 (+3 pad)
+  int* s_start = s_off + 36;                                                                  // 33 (+3 pad)
   // Mesh descriptors: a one-mesh launch reads its descriptor from the kernel
   // parameters; a batch keeps the descriptors of the current and the next
   // group's mesh in the warp's slice (copied when the mesh changes).
-  AsmDesc* s_desc = reinterpret_cast<AsmDesc*>(reinterpret_cast<unsigned char*>(s_off + 36));
+  AsmDesc* s_desc = reinterpret_cast<AsmDesc*>(reinterpret_cast<unsigned char*>(s_start + 36));
   int mesh0 = -1, mesh1 = -1;  // mesh held by descriptor slot 0 / 1
   auto load_desc = [&](int m, int slot) {
     if constexpr (BATCH) {
@@ -848,15 +951,13 @@ __global__ void __launch_bounds__(32 * WPB, warp_min_blocks<D, T, KC, WPB>()) ns
       }
     }
   };
-  // Field f of the mesh in descriptor slot `slot`: a batch reads its shared
-  // descriptor copy, a one-mesh launch its own parameters.
-#define UFEM_F(slot, f) (BATCH ? s_desc[(slot)].f : f##_1)
-
+  // The descriptor of the mesh in slot `slot`: a batch's shared copy, or the
+  // launch's parameter.
+#define UFEM_DESC(slot) (BATCH ? s_desc[(slot)] : one)
   // Persistent warps: a warp walks the global groups g, g + stride, ... of all
   // meshes of the launch (mesh m owns groups [gprefix[m], gprefix[m + 1])).
-  // While it reduces one group it already loads the incidence records
-  // (element id, slot word) and the connectivity of the next, so the next
-  // element phase starts with only the node gathers outstanding.
+  // While it reduces one group it already loads the incidence records, the
+  // connectivity and the item words of the next.
   int g = blockIdx.x * WPB + warp;
   if (g >= ngroups) return;  // whole warp; no CTA-wide barrier below
   const int gstride = gridDim.x * WPB;
@@ -872,23 +973,21 @@ __global__ void __launch_bounds__(32 * WPB, warp_min_blocks<D, T, KC, WPB>()) ns
   int cs = 0;  // descriptor slot of the current mesh
   load_desc(cm, cs);
   // first row, end row, first incidence, incidences
-  int4 G = BATCH ? __ldg(UFEM_F(cs, groups) + (g - __ldg(gprefix + cm))) : groups_1[g];
-  int pe = 0, poff = 0, pitems = 0;
-  uint32_t pinfo = 0;
+  int4 G = BATCH ? __ldg(UFEM_DESC(cs).groups + (g - __ldg(gprefix + cm))) : __ldg(one.groups + g);
+  uint32_t pea = 0;                 // the lane's incidence
+  int poff = 0, pstart = 0;         // the lane's row: lane offset, CSR block offset from the group's first
+  int pend = 0;                     // CSR blocks of the group
+  int64_t gs = 0;                   // CSR block offset of the group's first row
   int4 pcn = make_int4(0, 0, 0, 0);
-  auto fetch_records = [&](const int4& q, const int32_t* inc_elem, const uint32_t* inc_info,
-                           const int32_t* row_inc, const int64_t* start) {
-    if (lane < q.w) {
-      pe = __ldg(inc_elem + q.z + lane);
-      pinfo = __ldg(inc_info + q.z + lane);
-    }
-    if (lane < q.y - q.x) {
-      poff = __ldg(row_inc + q.x + lane) - q.z;
-      pitems = int(__ldg(start + q.x + lane + 1) - __ldg(start + q.x + lane) - 1) * RG;
-    }
+  auto fetch_records = [&](const int4& q, const AsmDesc& d) {
+    if (lane < q.w) pea = __ldg(d.inc_ea + q.z + lane);
+    gs = __ldg(d.start + q.x);
+    if (lane < q.y - q.x) poff = __ldg(d.row_inc + q.x + lane) - q.z;
+    if (lane < q.y - q.x) pstart = int(__ldg(d.start + q.x + lane) - gs);
+    pend = int(__ldg(d.start + q.y) - gs);
   };
-  fetch_records(G, UFEM_F(cs, inc_elem), UFEM_F(cs, inc_info), UFEM_F(cs, row_inc), UFEM_F(cs, start));
-  if (lane < G.w) pcn = __ldg(UFEM_F(cs, conn) + pe);
+  fetch_records(G, UFEM_DESC(cs));
+  if (lane < G.w) pcn = __ldg(UFEM_DESC(cs).conn + (pea & 0x3fffffffu));
   for (;;) {
     const int row0 = G.x, R = G.y - G.x, K = G.w;  // 1 <= R <= K <= KC
     const int gn = g + gstride;
@@ -896,153 +995,65 @@ __global__ void __launch_bounds__(32 * WPB, warp_min_blocks<D, T, KC, WPB>()) ns
     const int ns = (mn == cm) ? cs : 1 - cs;  // descriptor slot of the next group's mesh
     int4 Gn = make_int4(0, 0, 0, 0);
     if constexpr (!BATCH) {
-      if (gn < ngroups) Gn = groups_1[gn];
+      if (gn < ngroups) Gn = __ldg(one.groups + gn);
     }
     __syncwarp();  // the previous group's reads of the shared slice are complete
     if constexpr (BATCH) {
       load_desc(mn, ns);
       if (gn < ngroups) Gn = __ldg(s_desc[ns].groups + (gn - __ldg(gprefix + mn)));
     }
-    const int64_t* __restrict__ start = UFEM_F(cs, start);
-    int pref = lane < R ? pitems : 0;  // inclusive scan of the off-diagonal item counts
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(FULL, pref, o);
-      if (lane >= o) pref += v;
-    }
-    const int nitems = __shfl_sync(FULL, pref, R - 1);
     if (lane < R) {
-      s_pref[lane + 1] = pref;
       s_off[lane] = poff;
+      s_start[lane] = pstart;
     }
     if (lane == 0) {
-      s_pref[0] = 0;
       s_off[R] = K;
+      s_start[R] = pend;
     }
-#pragma unroll
-    for (int q = 0; q < D * 2; ++q) s_mask[q * 32 + lane] = 0u;
-    __syncwarp();
+    const int64_t gstart = gs;
+    const unsigned long long* __restrict__ words = UFEM_DESC(cs).items + (gstart - row0);
 
-    // Phase 1: one lane per incidence; the row node is relabelled to local
-    // position 0 exactly as in the chunk kernel.  Lane k stages its block
-    // (local column node b, equation r, component c) at k*LS + (b*neq + r)*neq + c
-    // and its RHS row at k*LS + nvals + r.
-    uint32_t pslots = 0xFFFFFFFFu;
-    if (lane < K) {
-      const uint32_t info = pinfo;
-      const int a = int(info >> 24) & 3;
+    // Phase 1: one lane per incidence, the element's nodes relabelled so that the
+    // row node is local node 0.
+    // A batch's launch leaves the meshes of the other kind (GEN) to their own.
+    const bool skip = BATCH && (UFEM_DESC(cs).gen != 0) != GEN;  // warp-uniform
+    if (lane < K && !skip) {
+      const int a = int(pea >> 30);
       const int ids0[4] = {pcn.x, pcn.y, pcn.z, pcn.w};
-      int ids[4];
-      pslots = 0;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int src = (D == 3) ? (q ^ a) : (q < 3 ? (q + a) % 3 : 3);
-        ids[q] = ids0[src];
-        const uint32_t sl = (q < n) ? ((info >> (6 * src)) & 63u) : 0xFFu;
-        pslots |= sl << (8 * q);
-      }
-      T* st = stage + lane * LS;
-      const KParams<T> kp = make_kparams<T>(UFEM_F(cs, p));
-      const NodeData nd{UFEM_F(cs, coords), UFEM_F(cs, uadv), UFEM_F(cs, state), UFEM_F(cs, node32)};
-      StageSink<T> sk{st, st + nvals, 1};
-      if constexpr (SPEC) {
-        if constexpr (D == 2) spec_tri_row<T>(ids, a, nd, kp, sk);
-        else spec_tet_row<T>(ids, a, nd, kp, sk);
+      int ids[4] = {0, 0, 0, 0};
+      if constexpr (D == 3) {
+        const bool x1 = (a & 1) != 0, x2 = (a & 2) != 0;
+        const int p0 = x1 ? ids0[1] : ids0[0], p1 = x1 ? ids0[0] : ids0[1], p2 = x1 ? ids0[3] : ids0[2],
+                  p3 = x1 ? ids0[2] : ids0[3];
+        ids[0] = x2 ? p2 : p0;
+        ids[1] = x2 ? p3 : p1;
+        ids[2] = x2 ? p0 : p2;
+        ids[3] = x2 ? p1 : p3;
       } else {
-        generic_row<D, T>(ids, a, nd, UFEM_F(cs, force), kp, sk);
+        ids[0] = a == 0 ? ids0[0] : (a == 1 ? ids0[1] : ids0[2]);
+        ids[1] = a == 0 ? ids0[1] : (a == 1 ? ids0[2] : ids0[0]);
+        ids[2] = a == 0 ? ids0[2] : (a == 1 ? ids0[0] : ids0[1]);
       }
-#pragma unroll
-      for (int q = 1; q < n; ++q) atomicOr(s_mask + (q - 1) * 64 + ((pslots >> (8 * q)) & 0xFFu), 1u << lane);
+      const AsmDesc& d = UFEM_DESC(cs);
+      const KParams<T> kp = make_kparams<T>(d.p);
+      const NodeData nd{d.coords, d.uadv, d.state, d.node32};
+      RecordSink<D, T> sk{stage + lane * LS};
+      element_row<D, T, SPEC, GEN>(ids, a, nd, d.force, kp, sk);
     }
-    s_pslots[lane] = pslots;
     __syncwarp();
-    fetch_records(Gn, UFEM_F(ns, inc_elem), UFEM_F(ns, inc_info), UFEM_F(ns, row_inc),
-                  UFEM_F(ns, start));  // next group's records load while this group is reduced
-    double* __restrict__ vals = UFEM_F(cs, vals);
-    float* __restrict__ vals32 = UFEM_F(cs, vals32);
-    double* __restrict__ rhs = UFEM_F(cs, rhs);
-
-    // Phase 2a: diagonal entries and RHS entries, neq * (neq + 1) items per row,
-    // each the sum over the row's lanes in element order.
-    constexpr int ND = neq * (neq + 1);
-    for (int it = lane; it < R * ND; it += 32) {
-      const int rl = it / ND, j = it - rl * ND;
-      const int kb = s_off[rl], ke = s_off[rl + 1];  // lanes of row rl
-      const int row = row0 + rl;
-      const T* src = stage + (j < neq * neq ? j : nvals + (j - neq * neq));  // b = 0 block, or the RHS row
-      double acc = 0.0;
-#pragma unroll 8
-      for (int k = kb; k < ke; ++k) acc += double(src[k * LS]);
-      if (j < neq * neq) {
-        const int r = j / neq, c = j - r * neq;
-        const int64_t s0 = __ldg(start + row);
-        const int S = int(__ldg(start + row + 1) - s0);
-        const int self = int(s_pslots[kb] & 0xFFu);
-        const int64_t pos = int64_t(neq) * neq * s0 + int64_t(r * S + self) * neq + c;
-        __stcs(vals + pos, acc);  // streamed: keep L2 for the node data the element phase gathers
-        if (vals32 != nullptr) __stcs(vals32 + pos, float(acc));
-      } else {
-        __stcs(rhs + int64_t(row) * neq + (j - neq * neq), acc);
-      }
-    }
-
-    if (lane < Gn.w) pcn = __ldg(UFEM_F(ns, conn) + pe);
-
-    // Phase 2b: off-diagonal items (row, slot != self, group of RPI equations):
-    // the contributors of slot s are the row's lanes holding s at local position
-    // b = 1..n-1, visited in ascending lane (= element) order.
-    for (int it = lane; it < nitems; it += 32) {
-      int lo = 0, hi = R - 1;
-      while (lo < hi) {  // last rl with s_pref[rl] <= it
-        const int mid = (lo + hi + 1) >> 1;
-        if (s_pref[mid] <= it) lo = mid; else hi = mid - 1;
-      }
-      const int rl = lo;
-      const int row = row0 + rl;
-      const int64_t s0 = __ldg(start + row);
-      const int S = int(__ldg(start + row + 1) - s0);
-      const int local = it - s_pref[rl];
-      const int s1 = local / RG;
-      const int rg = local - s1 * RG;
-      const int kb = s_off[rl], ke = s_off[rl + 1];
-      const int self = int(s_pslots[kb] & 0xFFu);
-      const int s = s1 + (s1 >= self ? 1 : 0);
-      const unsigned rowmask = unsigned((1ull << ke) - (1ull << kb));
-      const unsigned m1 = s_mask[s] & rowmask;
-      const unsigned m2 = s_mask[64 + s] & rowmask;
-      const unsigned m3 = (D == 3) ? (s_mask[128 + s] & rowmask) : 0u;
-      unsigned m = m1 | m2 | m3;
-      double acc[NV];
-#pragma unroll
-      for (int q = 0; q < NV; ++q) acc[q] = 0.0;
-      while (m) {
-        const int k = __ffs(m) - 1;
-        m &= m - 1;
-        const int b = 1 + int((m2 >> k) & 1u) + 2 * int((m3 >> k) & 1u);
-        T v[NV];
-        load_run<NV, T>(stage + k * LS + (b * neq + rg * RPI) * neq, v);
-#pragma unroll
-        for (int q = 0; q < NV; ++q) acc[q] += double(v[q]);
-      }
-#pragma unroll
-      for (int rr = 0; rr < RPI; ++rr) {
-        const int r = rg * RPI + rr;
-        const int64_t pos = int64_t(neq) * neq * s0 + int64_t(r * S + s) * neq;
-        if constexpr (neq == 4) {
-          __stcs(reinterpret_cast<double2*>(vals + pos), make_double2(acc[4 * rr], acc[4 * rr + 1]));
-          __stcs(reinterpret_cast<double2*>(vals + pos) + 1, make_double2(acc[4 * rr + 2], acc[4 * rr + 3]));
-          if (vals32 != nullptr)
-            __stcs(reinterpret_cast<float4*>(vals32 + pos),
-                   make_float4(float(acc[4 * rr]), float(acc[4 * rr + 1]), float(acc[4 * rr + 2]), float(acc[4 * rr + 3])));
-        } else {
-#pragma unroll
-          for (int c = 0; c < neq; ++c) __stcs(vals + pos + c, acc[rr * neq + c]);
-          if (vals32 != nullptr) {
-#pragma unroll
-            for (int c = 0; c < neq; ++c) __stcs(vals32 + pos + c, float(acc[rr * neq + c]));
-          }
-        }
-      }
+    constexpr int PAR = D == 3 ? 2 : 1;  // lanes per off-diagonal block
+    // item words of the group's first pass (3D: the first row's, 2D: the group's)
+    const int nfirst = D == 3 ? s_start[1] - 1 : s_start[R] - R;
+    unsigned long long word = lane < nfirst * PAR ? __ldg(words + lane / PAR) : 0ull;
+    fetch_records(Gn, UFEM_DESC(ns));  // next group's records load while this group is reduced
+    if (skip) {
+      if (lane < Gn.w) pcn = __ldg(UFEM_DESC(ns).conn + (pea & 0x3fffffffu));
+    } else if constexpr (D == 3) {
+      reduce_rows_3d<T, KC>(stage, s_off, s_start, R, row0, gstart, words, word, UFEM_DESC(cs),
+                            [&] { if (lane < Gn.w) pcn = __ldg(UFEM_DESC(ns).conn + (pea & 0x3fffffffu)); });
+    } else {
+      reduce_rows_2d<T>(stage, s_off, s_start, R, row0, gstart, words, word, UFEM_DESC(cs),
+                        [&] { if (lane < Gn.w) pcn = __ldg(UFEM_DESC(ns).conn + (pea & 0x3fffffffu)); });
     }
     if (gn >= ngroups) break;
     g = gn;
@@ -1050,7 +1061,7 @@ __global__ void __launch_bounds__(32 * WPB, warp_min_blocks<D, T, KC, WPB>()) ns
     cm = mn;
     cs = ns;
   }
-#undef UFEM_F
+#undef UFEM_DESC
 }
 
 // LinearizeU (NavierStokes.cpp:105), evaluated left to right without FMA
@@ -1226,6 +1237,9 @@ void fill_params(const ufem_ns_handle* h, NSParams& p) {
   p.has_force = h->d_force != nullptr;
 }
 
+// Whether the handle's element routine is the general one (another tau than METRIC).
+bool assembly_general(const ufem_ns_handle* h) { return h->opt.use_specializations == 0 && h->opt.supg_type != 1; }
+
 void fill_desc(const ufem_ns_handle* h, bool write32, AsmDesc& d, const WarpPlan* plan) {
   d.coords = h->d_coords;
   d.uadv = h->d_uadv;
@@ -1234,8 +1248,11 @@ void fill_desc(const ufem_ns_handle* h, bool write32, AsmDesc& d, const WarpPlan
   d.force = h->d_force;
   d.start = h->d_start;
   d.row_inc = h->d_row_inc;
-  d.inc_elem = h->d_inc_elem;
-  d.inc_info = h->d_inc_info;
+  d.inc_ea = h->d_inc_ea;
+  d.items = h->d_items;
+  d.over = h->d_over;
+  d.diagpos = h->d_diagpos;
+  d.gen = assembly_general(h) ? 1 : 0;
   d.conn = reinterpret_cast<const int4*>(h->d_conn);
   d.groups = (plan ? plan : &h->wplan)->groups;
   d.vals = h->d_vals;
@@ -1246,19 +1263,25 @@ void fill_desc(const ufem_ns_handle* h, bool write32, AsmDesc& d, const WarpPlan
 
 namespace {
 
+template <int D, typename T, int CH, bool SPEC, bool GEN>
+int launch_chunk_g(const ufem_ns_handle* h, const AssemblyPlan& plan, const NSParams& p, cudaStream_t s,
+                   bool write32) {
+  constexpr size_t smem = assembly_smem_bytes<D, T, CH>();
+  ns_assembly_kernel<D, T, CH, SPEC, GEN><<<plan.nchunks, CH, smem, s>>>(
+      plan.chunks, h->d_row_inc, h->d_inc_elem, h->d_inc_info, reinterpret_cast<const int4*>(h->d_conn),
+      h->d_coords, h->d_uadv, h->d_state, h->d_node32, h->d_force, h->d_start, p, h->d_vals,
+      write32 ? h->d_vals32 : nullptr, h->d_rhs);
+  UFEM_CUDA_TRY(cudaGetLastError());
+  return UFEM_OK;
+}
+
 template <int D, typename T, int CH, bool SPEC>
 int launch_chunk_t(const ufem_ns_handle* h, const AssemblyPlan& plan, const NSParams& p, cudaStream_t s,
                    bool write32) {
   if (plan.nchunks == 0) return UFEM_OK;
-  constexpr size_t smem = assembly_smem_bytes<D, T, CH>();
   if (plan.cap != CH) return set_error(UFEM_ERR_STATE, "assembly plan does not match the kernel width");
-  ns_assembly_kernel<D, T, CH, SPEC><<<plan.nchunks, CH, smem, s>>>(
-      plan.chunks, h->d_row_inc, h->d_inc_elem, h->d_inc_info, reinterpret_cast<const int4*>(h->d_conn),
-      h->d_coords, h->d_uadv, h->d_state, h->d_node32, h->d_force, h->d_start, p, h->d_vals,
-      write32 ? h->d_vals32 : nullptr,
-      h->d_rhs);
-  UFEM_CUDA_TRY(cudaGetLastError());
-  return UFEM_OK;
+  return assembly_general(h) ? launch_chunk_g<D, T, CH, SPEC, true>(h, plan, p, s, write32)
+                             : launch_chunk_g<D, T, CH, SPEC, false>(h, plan, p, s, write32);
 }
 
 // Resident CTAs of a kernel on the current device (persistent-warp grids).
@@ -1272,28 +1295,28 @@ int resident_ctas(K kernel, int threads, size_t smem) {
   return sms * per_sm;
 }
 
-template <int D, typename T, bool SPEC, int WPB, bool BATCH, int KC>
+template <int D, typename T, bool SPEC, bool GEN, int WPB, bool BATCH, int KC>
 int launch_warp_t(int ngroups, int nmesh, const AsmDesc* descs, const int* gprefix, const AsmDesc& one,
                   cudaStream_t s) {
   if (ngroups == 0) return UFEM_OK;
   constexpr size_t smem = warp_stage_bytes<D, T, KC, BATCH>() * WPB;
-  static const int resident = resident_ctas(ns_assembly_warp_kernel<D, T, SPEC, WPB, BATCH, KC>, 32 * WPB, smem);
+  static const int resident =
+      resident_ctas(ns_assembly_warp_kernel<D, T, SPEC, GEN, WPB, BATCH, KC>, 32 * WPB, smem);
   if (resident <= 0) return set_error(UFEM_ERR_CUDA, "occupancy query of the warp assembly kernel failed");
   const unsigned grid = unsigned(std::min<int64_t>((ngroups + WPB - 1) / WPB, resident));
-  ns_assembly_warp_kernel<D, T, SPEC, WPB, BATCH, KC><<<grid, 32 * WPB, smem, s>>>(
-      ngroups, nmesh, descs, gprefix, one.groups, one.row_inc, one.inc_elem, one.inc_info, one.conn, one.coords,
-      one.uadv, one.state, one.node32, one.force, one.start, one.p, one.vals, one.vals32, one.rhs);
+  ns_assembly_warp_kernel<D, T, SPEC, GEN, WPB, BATCH, KC><<<grid, 32 * WPB, smem, s>>>(ngroups, nmesh, descs, gprefix,
+                                                                                        one);
   UFEM_CUDA_TRY(cudaGetLastError());
   return UFEM_OK;
 }
 
-template <int D, typename T, bool SPEC, bool BATCH, int KC = 32>
+template <int D, typename T, bool SPEC, bool GEN, bool BATCH, int KC = 32>
 int launch_warp_w(int warps, int ngroups, int nmesh, const AsmDesc* descs, const int* gprefix, const AsmDesc& one,
                   cudaStream_t s) {
   switch (warps) {
-    case 2: return launch_warp_t<D, T, SPEC, 2, BATCH, KC>(ngroups, nmesh, descs, gprefix, one, s);
-    case 8: return launch_warp_t<D, T, SPEC, 8, BATCH, KC>(ngroups, nmesh, descs, gprefix, one, s);
-    default: return launch_warp_t<D, T, SPEC, 4, BATCH, KC>(ngroups, nmesh, descs, gprefix, one, s);
+    case 2: return launch_warp_t<D, T, SPEC, GEN, 2, BATCH, KC>(ngroups, nmesh, descs, gprefix, one, s);
+    case 8: return launch_warp_t<D, T, SPEC, GEN, 8, BATCH, KC>(ngroups, nmesh, descs, gprefix, one, s);
+    default: return launch_warp_t<D, T, SPEC, GEN, 4, BATCH, KC>(ngroups, nmesh, descs, gprefix, one, s);
   }
 }
 
@@ -1304,46 +1327,57 @@ int launch_assembly_t(ufem_ns_handle* h, cudaStream_t s, bool write32) {
   constexpr bool f32 = std::is_same<T, float>::value;
   if (h->asm_variant == kAsmChunk) return launch_chunk_t<D, T, CH, SPEC>(h, f32 ? h->plan32 : h->plan64, p, s, write32);
   int rc;
-  const bool w24 = D == 3 && h->asm_variant == kAsmWarp24;
+  // Without rows of more than 24 incidences the 24-lane plan serves the "warp"
+  // variant too: less staging a warp leaves the L1 more of the SM's array (the rows'
+  // values are the same bits under both plans).
+  const bool w24 = D == 3 && (h->asm_variant == kAsmWarp24 || (h->wplan24.big64.nchunks == 0 && h->wplan24.ngroups > 0));
   const WarpPlan& wp = w24 ? h->wplan24 : h->wplan;
   AsmDesc one;  // this handle's descriptor, passed as a kernel parameter
   fill_desc(h, write32, one, &wp);
-  if constexpr (D == 3) {
-    if (w24) rc = launch_warp_w<D, T, SPEC, false, 24>(h->asm_warps, wp.ngroups, 1, nullptr, nullptr, one, s);
-    else rc = launch_warp_w<D, T, SPEC, false, 32>(h->asm_warps, wp.ngroups, 1, nullptr, nullptr, one, s);
-  } else {
-    rc = launch_warp_w<D, T, SPEC, false, 32>(h->asm_warps, wp.ngroups, 1, nullptr, nullptr, one, s);
-  }
+  auto run = [&](auto gen) {
+    constexpr bool G = decltype(gen)::value;
+    if constexpr (D == 3) {
+      if (w24) return launch_warp_w<D, T, SPEC, G, false, 24>(h->asm_warps, wp.ngroups, 1, nullptr, nullptr, one, s);
+    }
+    return launch_warp_w<D, T, SPEC, G, false, 32>(h->asm_warps, wp.ngroups, 1, nullptr, nullptr, one, s);
+  };
+  rc = one.gen ? run(std::true_type{}) : run(std::false_type{});
   if (rc) return rc;
   return launch_chunk_t<D, T, CH, SPEC>(h, f32 ? wp.big32 : wp.big64, p, s, write32);
 }
 
-template <int D, typename T, bool SPEC, bool BATCH, int KC>
+template <int D, typename T, bool SPEC, bool GEN, bool BATCH, int KC>
 int set_warp_smem_attr() {
-  UFEM_CUDA_TRY(cudaFuncSetAttribute(ns_assembly_warp_kernel<D, T, SPEC, 2, BATCH, KC>,
+  UFEM_CUDA_TRY(cudaFuncSetAttribute(ns_assembly_warp_kernel<D, T, SPEC, GEN, 2, BATCH, KC>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      int(2 * warp_stage_bytes<D, T, KC, BATCH>())));
-  UFEM_CUDA_TRY(cudaFuncSetAttribute(ns_assembly_warp_kernel<D, T, SPEC, 4, BATCH, KC>,
+  UFEM_CUDA_TRY(cudaFuncSetAttribute(ns_assembly_warp_kernel<D, T, SPEC, GEN, 4, BATCH, KC>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      int(4 * warp_stage_bytes<D, T, KC, BATCH>())));
-  UFEM_CUDA_TRY(cudaFuncSetAttribute(ns_assembly_warp_kernel<D, T, SPEC, 8, BATCH, KC>,
+  UFEM_CUDA_TRY(cudaFuncSetAttribute(ns_assembly_warp_kernel<D, T, SPEC, GEN, 8, BATCH, KC>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      int(8 * warp_stage_bytes<D, T, KC, BATCH>())));
   return UFEM_OK;
 }
 
-template <int D, typename T, int CH, bool SPEC>
-int set_smem_attr() {
+template <int D, typename T, int CH, bool SPEC, bool GEN>
+int set_smem_attr_g() {
   constexpr size_t smem = assembly_smem_bytes<D, T, CH>();
-  UFEM_CUDA_TRY(cudaFuncSetAttribute(ns_assembly_kernel<D, T, CH, SPEC>,
+  UFEM_CUDA_TRY(cudaFuncSetAttribute(ns_assembly_kernel<D, T, CH, SPEC, GEN>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   int rc;
-  if ((rc = set_warp_smem_attr<D, T, SPEC, false, 32>()) || (rc = set_warp_smem_attr<D, T, SPEC, true, 32>()))
+  if ((rc = set_warp_smem_attr<D, T, SPEC, GEN, false, 32>()) || (rc = set_warp_smem_attr<D, T, SPEC, GEN, true, 32>()))
     return rc;
   if constexpr (D == 3) {
-    if ((rc = set_warp_smem_attr<D, T, SPEC, false, 24>())) return rc;
+    if ((rc = set_warp_smem_attr<D, T, SPEC, GEN, false, 24>())) return rc;
   }
   return UFEM_OK;
+}
+
+template <int D, typename T, int CH, bool SPEC>
+int set_smem_attr() {
+  const int rc = set_smem_attr_g<D, T, CH, SPEC, false>();
+  return rc ? rc : set_smem_attr_g<D, T, CH, SPEC, true>();
 }
 
 // ---------------------------------------------------------------------------
@@ -1352,7 +1386,7 @@ int set_smem_attr() {
 // increment dx, r = b - M dx of the FP64 system that the FP64 assembly and the
 // symmetric Dirichlet conditions would have built, evaluated element by element
 // without forming M.  Per incidence (row node, element) the FP64 element
-// routines run with a sink that applies each row of M = invdt T + theta A
+// routine runs with a sink that applies the row block of M = invdt T + theta A
 // (NavierStokesAssembly.hpp:69-71) to the element's increment instead of staging
 // it, and keeps the RHS row a - A x (the reference's system_rhs += -_A _x + _a,
 // :69); the rows' contributions are then summed in element order.
@@ -1365,24 +1399,37 @@ struct ResidSink {
   double dl[D + 1][D + 1];  // increment of the relabelled element nodes (u, v, [w], p)
   double acc[D + 1];        // (M dx) of the row
   double rr[D + 1];         // a - A x of the row
-  template <int NEQ>
-  __device__ __forceinline__ void row(int idx, const double (&v)[NEQ]) {
-    const int b = idx / (NEQ * NEQ), r = (idx / NEQ) % NEQ;
-    double s = 0.0;
+  double tg[D], thS, sWSp, c[D];
+  __device__ __forceinline__ void head(const double (&tg_)[D], double thS_, double sWSp_, const double (&c_)[D]) {
 #pragma unroll
-    for (int c = 0; c < NEQ; ++c) s += v[c] * dl[b][c];
-    acc[r] += s;
+    for (int k = 0; k < D; ++k) {
+      tg[k] = tg_[k];
+      c[k] = c_[k];
+    }
+    thS = thS_;
+    sWSp = sWSp_;
   }
-  template <int NEQ>
-  __device__ __forceinline__ void rhs(const double (&v)[NEQ]) {
+  __device__ __forceinline__ void col(int b, const double (&g)[D], double diag, double vem, double dd) {
+    double div = 0.0, cd = 0.0;
 #pragma unroll
-    for (int r = 0; r < NEQ; ++r) rr[r] = v[r];
+    for (int k = 0; k < D; ++k) {
+      div += g[k] * dl[b][k];
+      cd += c[k] * dl[b][k];
+    }
+#pragma unroll
+    for (int i = 0; i < D; ++i) acc[i] += tg[i] * div + (diag * dl[b][i] + thS * (g[i] * dl[b][D]));
+    acc[D] += sWSp * div + (vem * cd + dd * dl[b][D]);
+  }
+  __device__ __forceinline__ void rhs(const double (&v)[D + 1]) {
+#pragma unroll
+    for (int r = 0; r <= D; ++r) rr[r] = v[r];
   }
 };
 
 // One CTA per chunk of whole rows (the chunk plan), one thread per incidence.
-template <int D, int CH, bool SPEC>
-__global__ void __launch_bounds__(CH) ns_residual_kernel(
+// 128 registers a thread (16 warps an SM): the gathers' latency is what it waits for.
+template <int D, int CH, bool SPEC, bool GEN>
+__global__ void __launch_bounds__(CH, 512 / CH) ns_residual_kernel(
     const int2* __restrict__ chunk_rows, const int32_t* __restrict__ row_inc, const int32_t* __restrict__ inc_elem,
     const uint32_t* __restrict__ inc_info, const int4* __restrict__ conn, const double* __restrict__ coords,
     const double* __restrict__ uadv, const double* __restrict__ state, const double* __restrict__ force, NSParams p,
@@ -1414,12 +1461,7 @@ __global__ void __launch_bounds__(CH) ns_residual_kernel(
     for (int r = 0; r < neq; ++r) sk.acc[r] = 0.0;
     const KParams<double> kp = make_kparams<double>(p);
     const NodeData nd{coords, uadv, state, nullptr};
-    if constexpr (SPEC) {
-      if constexpr (D == 2) spec_tri_row<double>(ids, a, nd, kp, sk);
-      else spec_tet_row<double>(ids, a, nd, kp, sk);
-    } else {
-      generic_row<D, double>(ids, a, nd, force, kp, sk);
-    }
+    element_row<D, double, SPEC, GEN>(ids, a, nd, force, kp, sk);
 #pragma unroll
     for (int r = 0; r < neq; ++r) s_res[r * CH + t] = sk.rr[r] - sk.acc[r];
   }
@@ -1450,9 +1492,11 @@ int launch_residual_t(ufem_ns_handle* h, const double* dxp, double* res, cudaStr
   NSParams p;
   fill_params(h, p);
   if (h->plan64.cap != CH) return set_error(UFEM_ERR_STATE, "chunk plan does not match the residual kernel width");
-  ns_residual_kernel<D, CH, SPEC><<<h->plan64.nchunks, CH, 0, s>>>(
-      h->plan64.chunks, h->d_row_inc, h->d_inc_elem, h->d_inc_info, reinterpret_cast<const int4*>(h->d_conn),
-      h->d_coords, h->d_uadv, h->d_state, h->d_force, p, dxp, res);
+  const bool gen = !SPEC && h->opt.supg_type != 1;
+  auto kernel = gen ? ns_residual_kernel<D, CH, SPEC, true> : ns_residual_kernel<D, CH, SPEC, false>;
+  kernel<<<h->plan64.nchunks, CH, 0, s>>>(h->plan64.chunks, h->d_row_inc, h->d_inc_elem, h->d_inc_info,
+                                          reinterpret_cast<const int4*>(h->d_conn), h->d_coords, h->d_uadv,
+                                          h->d_state, h->d_force, p, dxp, res);
   UFEM_CUDA_TRY(cudaGetLastError());
   return UFEM_OK;
 }
@@ -1499,19 +1543,32 @@ int launch_assembly(ufem_ns_handle* h, cudaStream_t s, bool write32) {
               : launch_assembly_t<3, double, kChunk3D64, false>(h, s, write32);
 }
 
-int launch_assembly_batch(int dim, int precision, bool spec, int warps, int ngroups, int nmesh,
+namespace {
+template <int D, typename T, bool SPEC>
+int launch_batch_t(int warps, int kinds, int ngroups, int nmesh, const AsmDesc* d_descs, const int* d_gprefix,
+                   cudaStream_t s) {
+  int rc;
+  if ((kinds & 1) && (rc = launch_warp_w<D, T, SPEC, false, true>(warps, ngroups, nmesh, d_descs, d_gprefix, AsmDesc{}, s)))
+    return rc;
+  if ((kinds & 2) && (rc = launch_warp_w<D, T, SPEC, true, true>(warps, ngroups, nmesh, d_descs, d_gprefix, AsmDesc{}, s)))
+    return rc;
+  return UFEM_OK;
+}
+}  // namespace
+
+int launch_assembly_batch(int dim, int precision, bool spec, int warps, int kinds, int ngroups, int nmesh,
                           const AsmDesc* d_descs, const int* d_gprefix, cudaStream_t s) {
   const bool f32 = precision == 1;
   if (dim == 2) {
-    if (f32) return spec ? launch_warp_w<2, float, true, true>(warps, ngroups, nmesh, d_descs, d_gprefix, AsmDesc{}, s)
-                         : launch_warp_w<2, float, false, true>(warps, ngroups, nmesh, d_descs, d_gprefix, AsmDesc{}, s);
-    return spec ? launch_warp_w<2, double, true, true>(warps, ngroups, nmesh, d_descs, d_gprefix, AsmDesc{}, s)
-                : launch_warp_w<2, double, false, true>(warps, ngroups, nmesh, d_descs, d_gprefix, AsmDesc{}, s);
+    if (f32) return spec ? launch_batch_t<2, float, true>(warps, kinds, ngroups, nmesh, d_descs, d_gprefix, s)
+                         : launch_batch_t<2, float, false>(warps, kinds, ngroups, nmesh, d_descs, d_gprefix, s);
+    return spec ? launch_batch_t<2, double, true>(warps, kinds, ngroups, nmesh, d_descs, d_gprefix, s)
+                : launch_batch_t<2, double, false>(warps, kinds, ngroups, nmesh, d_descs, d_gprefix, s);
   }
-  if (f32) return spec ? launch_warp_w<3, float, true, true>(warps, ngroups, nmesh, d_descs, d_gprefix, AsmDesc{}, s)
-                       : launch_warp_w<3, float, false, true>(warps, ngroups, nmesh, d_descs, d_gprefix, AsmDesc{}, s);
-  return spec ? launch_warp_w<3, double, true, true>(warps, ngroups, nmesh, d_descs, d_gprefix, AsmDesc{}, s)
-              : launch_warp_w<3, double, false, true>(warps, ngroups, nmesh, d_descs, d_gprefix, AsmDesc{}, s);
+  if (f32) return spec ? launch_batch_t<3, float, true>(warps, kinds, ngroups, nmesh, d_descs, d_gprefix, s)
+                       : launch_batch_t<3, float, false>(warps, kinds, ngroups, nmesh, d_descs, d_gprefix, s);
+  return spec ? launch_batch_t<3, double, true>(warps, kinds, ngroups, nmesh, d_descs, d_gprefix, s)
+              : launch_batch_t<3, double, false>(warps, kinds, ngroups, nmesh, d_descs, d_gprefix, s);
 }
 
 int launch_assembly_big_rows(ufem_ns_handle* h, cudaStream_t s, bool write32) {
@@ -1530,6 +1587,16 @@ int launch_assembly_big_rows(ufem_ns_handle* h, cudaStream_t s, bool write32) {
                        : launch_chunk_t<3, float, kChunk3D32, false>(h, w.big32, p, s, write32);
   return spec ? launch_chunk_t<3, double, kChunk3D64, true>(h, w.big64, p, s, write32)
               : launch_chunk_t<3, double, kChunk3D64, false>(h, w.big64, p, s, write32);
+}
+
+int launch_assembly_items(ufem_ns_handle* h, unsigned* over_used, cudaStream_t s) {
+  const unsigned blocks = unsigned((h->N + 127) / 128);
+  unsigned long long* items = h->d_items;
+  auto kernel = h->dim == 2 ? assembly_items_kernel<2> : assembly_items_kernel<3>;
+  kernel<<<blocks, 128, 0, s>>>(h->N, h->d_start, h->d_row_inc, h->d_inc_elem, h->d_inc_info, h->d_inc_ea, items,
+                                h->d_over, over_used);
+  UFEM_CUDA_TRY(cudaGetLastError());
+  return UFEM_OK;
 }
 
 int launch_linearize(ufem_ns_handle* h, cudaStream_t s) {

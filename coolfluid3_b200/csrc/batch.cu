@@ -864,6 +864,7 @@ struct ufem_batch {
   int nmesh = 0;
   int64_t total_nodes = 0, total_rows = 0, total_bc = 0, total_fix = 0;
   int ngroups = 0, nchunks = 0;
+  int kinds = 1;  // element routines of the members (launch_assembly_batch)
   bool graphs = true;
   // device
   AsmDesc* d_asm = nullptr;
@@ -916,10 +917,12 @@ int batch_refresh(ufem_batch* b) {
   std::vector<AsmDesc> ad(b->nmesh);
   std::vector<BatchMesh> bm(b->nmesh);
   std::vector<int64_t> bcp(b->nmesh + 1, 0), fxp(b->nmesh + 1, 0);
+  b->kinds = 0;
   for (int m = 0; m < b->nmesh; ++m) {
     ufem_ns_handle* h = b->members[m];
     if (h->bcp.dirty && (rc = build_bc_plan(h))) return rc;
     fill_desc(h, h->d_vals32 != nullptr, ad[m]);
+    b->kinds |= ad[m].gen ? 2 : 1;
     BatchMesh& M = bm[m];
     M.N = h->N;
     M.nrows = h->nrows;
@@ -1425,7 +1428,7 @@ int ufem_batch_tune_assembly(ufem_batch* b, void* stream, int32_t reps, int32_t*
   rc = UFEM_OK;
   for (int w : {2, 4, 8}) {
     auto launch = [&] {
-      return launch_assembly_batch(b->dim, b->precision, b->spec != 0, w, b->ngroups, b->nmesh, b->d_asm,
+      return launch_assembly_batch(b->dim, b->precision, b->spec != 0, w, b->kinds, b->ngroups, b->nmesh, b->d_asm,
                                    b->d_gprefix, st);
     };
     if ((rc = launch())) break;  // warm-up
@@ -1466,7 +1469,7 @@ int ufem_batch_assemble(ufem_batch* b, void* stream) {
   linearize_batch_kernel<<<blocks_for(b->total_nodes, 256), 256, 0, st>>>(b->total_nodes, b->nmesh,
                                                                           b->d_node_prefix, b->d_mesh);
   UFEM_CUDA_TRY(cudaGetLastError());
-  if ((rc = launch_assembly_batch(b->dim, b->precision, b->spec != 0, b->warps, b->ngroups, b->nmesh, b->d_asm,
+  if ((rc = launch_assembly_batch(b->dim, b->precision, b->spec != 0, b->warps, b->kinds, b->ngroups, b->nmesh, b->d_asm,
                                   b->d_gprefix, st)))
     return rc;
   for (ufem_ns_handle* h : b->members) {  // rows with more than 32 elements (none on most meshes)

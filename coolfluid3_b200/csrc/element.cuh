@@ -60,10 +60,20 @@ __device__ __forceinline__ T sel(const T (&arr)[M], int i) {
   return r;
 }
 
+// One 32-byte record (32-byte aligned) in one 256-bit load: a gather's cost is the
+// lines its lanes touch, once per instruction, and two 16-byte loads touch them
+// twice.
 __device__ __forceinline__ void ld4(const double* __restrict__ p, double& a, double& b, double& c, double& d) {
-  const double2 x = __ldg(reinterpret_cast<const double2*>(p));
-  const double2 y = __ldg(reinterpret_cast<const double2*>(p) + 1);
-  a = x.x; b = x.y; c = y.x; d = y.y;
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(a), "=d"(b), "=d"(c), "=d"(d) : "l"(p));
+}
+__device__ __forceinline__ void ld8(const float* __restrict__ p, float (&v)[8]) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+      : "l"(p));
+}
+// 32 bytes (32-byte aligned), streamed.
+__device__ __forceinline__ void st4_cs(double* __restrict__ p, double a, double b, double c, double d) {
+  asm volatile("st.global.cs.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
 }
 
 // Inverse and determinant in the cofactor form (Proto/ElementData.hpp:308-314).
@@ -116,8 +126,8 @@ struct NodeData {
   const float* node32;   // N x 8 (u_adv, nu_eff, u, p), FP32 path only
 };
 
-template <int D, typename T>
-__device__ __forceinline__ void gather_geometry_uadv(const int (&ids)[4], const NodeData& nd, Elem<D, T>& el) {
+template <int D>
+__device__ __forceinline__ void relative_coords(const int (&ids)[4], const NodeData& nd, double (&X)[D + 1][D]) {
   double X0[4];
   ld4(nd.coords + 4ll * ids[0], X0[0], X0[1], X0[2], X0[3]);
 #pragma unroll
@@ -125,20 +135,43 @@ __device__ __forceinline__ void gather_geometry_uadv(const int (&ids)[4], const 
     double x[4];
     ld4(nd.coords + 4ll * ids[b], x[0], x[1], x[2], x[3]);
 #pragma unroll
-    for (int k = 0; k < D; ++k) el.Xr[b][k] = T(x[k] - X0[k]);
-    if constexpr (std::is_same<T, float>::value) {
-      const float4 u = __ldg(reinterpret_cast<const float4*>(nd.node32) + 2ll * ids[b]);
-      const float uu[4] = {u.x, u.y, u.z, u.w};
+    for (int k = 0; k < D; ++k) X[b][k] = x[k] - X0[k];
+  }
+}
+
+// FP32: relative coordinates, and u_adv, nu_eff and the state x from one 32-byte
+// record a node ((u, v, [w], p): p is the record's last number).
+template <int D>
+__device__ __forceinline__ void gather_geometry_node32(const int (&ids)[4], const NodeData& nd, Elem<D, float>& el,
+                                                       float (&x)[D + 1][D + 1]) {
+  double X[D + 1][D];
+  relative_coords<D>(ids, nd, X);
 #pragma unroll
-      for (int k = 0; k < D; ++k) el.U[b][k] = uu[k];
-      el.NU[b] = u.w;
-    } else {
-      double u[4];
-      ld4(nd.uadv + 4ll * ids[b], u[0], u[1], u[2], u[3]);
+  for (int b = 0; b <= D; ++b) {
+    float v[8];
+    ld8(nd.node32 + 8ll * ids[b], v);
 #pragma unroll
-      for (int k = 0; k < D; ++k) el.U[b][k] = T(u[k]);
-      el.NU[b] = T(u[3]);
+    for (int k = 0; k < D; ++k) {
+      el.Xr[b][k] = float(X[b][k]);
+      el.U[b][k] = v[k];
+      x[b][k] = v[4 + k];
     }
+    el.NU[b] = v[3];
+    x[b][D] = v[7];
+  }
+}
+
+// FP64: relative coordinates, u_adv and nu_eff.
+template <int D, typename T>
+__device__ __forceinline__ void gather_geometry_uadv(const int (&ids)[4], const NodeData& nd, Elem<D, T>& el) {
+  relative_coords<D>(ids, nd, el.Xr);
+#pragma unroll
+  for (int b = 0; b <= D; ++b) {
+    double u[4];
+    ld4(nd.uadv + 4ll * ids[b], u[0], u[1], u[2], u[3]);
+#pragma unroll
+    for (int k = 0; k < D; ++k) el.U[b][k] = u[k];
+    el.NU[b] = u[3];
   }
 }
 

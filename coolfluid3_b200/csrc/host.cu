@@ -105,6 +105,29 @@ void dfree(T*& p) {
   p = nullptr;
 }
 
+// The warp kernel's static lists; a second pass writes the contributor lists of
+// items with more than 7 contributors, where there are any.
+int build_assembly_lists(ufem_ns_handle* h, cudaStream_t s) {
+  unsigned* used = nullptr;
+  int rc;
+  if ((rc = dmalloc(&used, 1, "list counter"))) return rc;
+  unsigned n = 0;
+  cudaError_t ce = cudaMemsetAsync(used, 0, sizeof(unsigned), s);
+  if (ce == cudaSuccess && (rc = launch_assembly_items(h, used, s)) == UFEM_OK) {
+    ce = cudaMemcpyAsync(&n, used, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
+    if (ce == cudaSuccess && n > 0 && (rc = dmalloc(&h->d_over, n, "long item lists")) == UFEM_OK) {
+      h->over_bytes = n;
+      ce = cudaMemsetAsync(used, 0, sizeof(unsigned), s);
+      if (ce == cudaSuccess && (rc = launch_assembly_items(h, used, s)) == UFEM_OK) ce = cudaStreamSynchronize(s);
+    }
+  }
+  dfree(used);
+  if (rc) return rc;
+  if (ce != cudaSuccess) return set_error(UFEM_ERR_CUDA, std::string("assembly lists: ") + cudaGetErrorString(ce));
+  return UFEM_OK;
+}
+
 int validate_options(const ufem_ns_options* o) {
   if (!o) return set_error(UFEM_ERR_ARG, "options pointer is NULL");
   if (!(o->theta > 0.0 && o->theta <= 1.0))
@@ -351,6 +374,7 @@ void destroy_impl(ufem_ns_handle* h) {
   dfree(h->d_nu); dfree(h->d_force); dfree(h->d_node32); dfree(h->d_start); dfree(h->d_adj); dfree(h->d_rowptr);
   dfree(h->d_colidx); dfree(h->d_vals); dfree(h->d_vals32); dfree(h->d_rhs); dfree(h->d_sol);
   dfree(h->d_diagpos); dfree(h->d_row_inc); dfree(h->d_inc_elem); dfree(h->d_inc_info);
+  dfree(h->d_inc_ea); dfree(h->d_items); dfree(h->d_over);
   dfree(h->plan64.chunks); dfree(h->plan32.chunks); dfree(h->d_tie);
   for (WarpPlan* wp : {&h->wplan, &h->wplan24}) {
     dfree(wp->groups);
@@ -650,6 +674,9 @@ int create_impl(const ufem_mesh* mesh, const ufem_ns_options* opts, const uint32
       (rc = dmalloc(&h->plan32.chunks, chunks32.size(), "chunks32")) ||
       (rc = dmalloc(&h->d_stage, size_t(N) * 4 * dim, "stage")))
     return fail(rc);
+  if (coupled && ((rc = dmalloc(&h->d_inc_ea, inc_elem.size(), "inc_ea")) ||
+                  (rc = dmalloc(&h->d_items, std::max<size_t>(size_t(h->bnnz - N), 1), "assembly items"))))
+    return fail(rc);
   if (coupled && opts->precision == 1 && ((rc = dmalloc(&h->d_vals32, size_t(h->nnz), "vals32")) ||
                                (rc = dmalloc(&h->d_node32, size_t(h->N) * 8, "node32"))))
     return fail(rc);
@@ -699,7 +726,10 @@ int create_impl(const ufem_mesh* mesh, const ufem_ns_options* opts, const uint32
       (ce = cudaMemsetAsync(h->d_hist, 0, size_t(N) * 96, cs)) ||
       (ce = cudaMemsetAsync(h->d_uadv, 0, size_t(N) * 32, cs)) || (ce = cudaMemsetAsync(h->d_nu, 0, size_t(N) * 8, cs)))
     return fail(set_error(UFEM_ERR_CUDA, std::string("memset: ") + cudaGetErrorString(ce)));
-  if (coupled && (rc = launch_build_csr(h, cs))) return fail(rc);
+  if (coupled) {
+    if ((rc = launch_build_csr(h, cs)) || (rc = build_assembly_lists(h, cs)))
+      return fail(rc);
+  }
   if ((ce = cudaStreamSynchronize(cs)) != cudaSuccess)
     return fail(set_error(UFEM_ERR_CUDA, std::string("CSR build: ") + cudaGetErrorString(ce)));
   for (auto& e : h->ev)
@@ -899,6 +929,8 @@ int ufem_ns_device_bytes(const ufem_ns_handle* h, int64_t* bytes) {
   if (h->d_force) b += N * 32;
   if (h->d_vals32) b += Z * 4;
   if (h->d_node32) b += N * 32;
+  if (h->d_inc_ea) b += E * h->nn * 4;
+  if (h->d_items) b += (h->bnnz - N) * 8 + h->over_bytes;
   b += krylov_device_bytes(h);  // solver workspace allocated so far (none for a batch member's vectors)
   if (h->pipe.buf[0]) b += 2 * (N * (h->neq + 4 * h->dim + 1) + R) * 8;  // overlapped-transfer buffers, once used
   if (h->d_tie) b += h->ntie * 8;

@@ -74,14 +74,17 @@ struct AsmDesc {
   const double* force;
   const int64_t* start;
   const int32_t* row_inc;
-  const int32_t* inc_elem;
-  const uint32_t* inc_info;
+  const uint32_t* inc_ea;         // per incidence: element | local node << 30
+  const unsigned long long* items;  // off-diagonal item words
+  const uint8_t* over;            // contributors of items with more than 7
+  const int64_t* diagpos;
   const int4* conn;
   const int4* groups;
   double* vals;
   float* vals32;  // null: no FP32 copy of the values
   double* rhs;
   NSParams p;
+  int gen;                        // the general element routine (assembly_general)
 };
 
 // Assembly kernel variants (selected per handle, see ufem_ns_set_assembly_kernel).
@@ -183,6 +186,12 @@ struct ufem_ns_handle {
   int32_t* d_row_inc = nullptr;   // N+1
   int32_t* d_inc_elem = nullptr;  // E*nn
   uint32_t* d_inc_info = nullptr; // E*nn : 6-bit slots + local index << 24
+  // static lists of the warp assembly kernel (assembly.cu): the incidences'
+  // elements and local nodes, the off-diagonal items and their overflow lists
+  uint32_t* d_inc_ea = nullptr;   // E*nn
+  unsigned long long* d_items = nullptr;  // bnnz - N
+  uint8_t* d_over = nullptr;
+  int64_t over_bytes = 0;
 
   ufem::AssemblyPlan plan64;       // chunks sized for the FP64-element chunk kernel (all rows)
   ufem::AssemblyPlan plan32;       // chunks sized for the FP32-element chunk kernel (all rows)
@@ -215,9 +224,14 @@ int launch_linearize(ufem_ns_handle* h, cudaStream_t s);
 int launch_assembly(ufem_ns_handle* h, cudaStream_t s, bool write32);
 void fill_params(const ufem_ns_handle* h, NSParams& p);
 void fill_desc(const ufem_ns_handle* h, bool write32, AsmDesc& d, const WarpPlan* plan = nullptr);
-// Warp assembly of many meshes in one persistent launch (same dim and precision;
+// The warp kernel's static lists; over_used: device counter of the overflow bytes
+// (the lists are written where d_over is allocated).
+int launch_assembly_items(ufem_ns_handle* h, unsigned* over_used, cudaStream_t s);
+bool assembly_general(const ufem_ns_handle* h);
+// Warp assembly of many meshes in one persistent launch per kind of element routine
+// (kinds: bit 0 METRIC, bit 1 general; same dim and precision;
 // rows with more than 32 incidences go through each mesh's chunk plan).
-int launch_assembly_batch(int dim, int precision, bool spec, int warps, int ngroups, int nmesh,
+int launch_assembly_batch(int dim, int precision, bool spec, int warps, int kinds, int ngroups, int nmesh,
                           const AsmDesc* d_descs, const int* d_gprefix, cudaStream_t s);
 int launch_dirichlet(ufem_ns_handle* h, cudaStream_t s);
 // Adds the constant Neumann contributions to the RHS (before the Dirichlet passes).
