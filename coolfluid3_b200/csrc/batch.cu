@@ -11,7 +11,9 @@
 //    is split into fixed chunks of kChunkNodes nodes, vector kernels produce
 //    one partial per chunk, and the last CTA of each mesh to finish (an atomic
 //    counter per mesh) folds that mesh's partials in a fixed order and updates
-//    its scalars, so an iteration is seven launches.  A member's arithmetic therefore depends only on its own
+//    its scalars, so an iteration is seven launches.  Members whose system fits one
+//    thread-block cluster are solved there instead, whole solves in one launch per
+//    cluster size (persist.cu).  A member's arithmetic depends only on its own
 //    data: its results are bitwise the same alone (a batch of one) and in any
 //    mix.  Converged members drop out (their kernels return at once) while the
 //    others continue.  The mixed-precision solve iterates with an FP32 copy of
@@ -28,6 +30,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "persist.h"
 #include "spmv_node.cuh"
 
 namespace ufem {
@@ -887,6 +890,18 @@ struct ufem_batch {
   cudaGraphExec_t block_exec[3] = {nullptr, nullptr, nullptr};
   cudaStream_t capture_stream = nullptr;
   int block_pkind[3] = {-1, -1, -1};
+  // One-cluster solves of the members that fit one (persist.cu): their plans per
+  // operator type, with the coarse sizes they were made for, the device list of
+  // solves, and the solves' scalars and flags (16 and 8 a member).
+  std::vector<PersistPlan> plan[2];
+  std::vector<int> plan_nc[2];
+  PersistSolve* d_solves = nullptr;
+  double* p_dctl = nullptr;
+  int* p_ictl = nullptr;
+  std::vector<int> p_flags;
+  // launches of different cluster sizes run beside each other
+  cudaStream_t side[4] = {};
+  cudaEvent_t fork = nullptr, join[4] = {};
   // matrix-free refinement (mixed = 2): the members' FP64 residuals, the inner
   // solve's right-hand sides (residual / its norm) and corrections
   double *mfr = nullptr, *mfb = nullptr, *mfz = nullptr;
@@ -899,12 +914,18 @@ void batch_free(ufem_batch* b) {
   for (auto& g : b->block_exec)
     if (g) cudaGraphExecDestroy(g);
   if (b->capture_stream) cudaStreamDestroy(b->capture_stream);
+  for (auto& q : b->side)
+    if (q) cudaStreamDestroy(q);
+  for (auto& e : b->join)
+    if (e) cudaEventDestroy(e);
+  if (b->fork) cudaEventDestroy(b->fork);
   dfr(b->d_asm); dfr(b->d_gprefix); dfr(b->d_mesh); dfr(b->d_node_prefix); dfr(b->d_bc_prefix);
   dfr(b->d_fix_prefix); dfr(b->d_chunks); dfr(b->d_cprefix);
   dfr(b->r); dfr(b->rh); dfr(b->p); dfr(b->v); dfr(b->s); dfr(b->t); dfr(b->ph); dfr(b->sh); dfr(b->dinv);
   dfr(b->w); dfr(b->part); dfr(b->counters); dfr(b->dctl); dfr(b->ictl);
   dfr(b->d_coarse_prefix); dfr(b->cvec); dfr(b->yvec);
   dfr(b->mfr); dfr(b->mfb); dfr(b->mfz);
+  dfr(b->d_solves); dfr(b->p_dctl); dfr(b->p_ictl);
   if (b->h_dctl) cudaFreeHost(b->h_dctl);
   if (b->h_ictl) cudaFreeHost(b->h_ictl);
   delete b;
@@ -1068,11 +1089,121 @@ int residual_b(ufem_batch* b, double* x, double* bw, bool init_rh, bool skip_don
   return UFEM_OK;
 }
 
+// Solves the members in `todo` that fit one cluster, one cluster each, all at once
+// (launches by cluster size); the others are left in `todo`.  The choice and the
+// arithmetic depend on the member alone.  The chunk kernels are bound by launches
+// (55 us an iteration for 8 members of 40^2 cells, 27 blocks busy); in a cluster an
+// iteration costs its four barriers and the member's product, about 9 us, and
+// clusters need no one else: 10.2 -> 1.9 ms a time step of those 8 members.  solved[m] is set, and p_flags holds their
+// flags (8 ints a member: done, -, status, iterations).
+template <typename MT>
+int solve_in_clusters(ufem_batch* b, int pkind, double tol, int maxit, double* xw, double* bw, std::vector<int>& todo,
+                      std::vector<int>& solved, cudaStream_t st) {
+  constexpr bool f32 = std::is_same<MT, float>::value;
+  const int n = b->nmesh;
+  std::vector<PersistPlan>& plan = b->plan[f32];
+  std::vector<int>& plan_nc = b->plan_nc[f32];
+  plan.resize(size_t(n));
+  plan_nc.resize(size_t(n), -1);
+  std::vector<PersistSolve> list;
+  std::vector<int64_t> off(size_t(n) + 1, 0);
+  for (int m = 0; m < n; ++m) off[size_t(m) + 1] = off[size_t(m)] + b->members[m]->nrows;
+  int rc;
+  if (!b->d_solves && ((rc = dmal(&b->d_solves, size_t(n))) || (rc = dmal(&b->p_dctl, size_t(16) * n)) ||
+                       (rc = dmal(&b->p_ictl, size_t(8) * n))))
+    return rc;
+  struct Group {
+    int blocks, first, count;
+    size_t smem;
+  };
+  std::vector<Group> groups;
+  for (int blocks = 1; blocks <= 16; blocks *= 2) {
+    Group g{blocks, int(list.size()), 0, 0};
+    for (int m = 0; m < n; ++m) {
+      if (!todo[m]) continue;
+      const ufem_ns_handle* h = b->members[m];
+      const CoarseView cv = pkind == 4 && m < int(b->coarse.size()) ? b->coarse[m] : CoarseView{};
+      if (plan_nc[m] != cv.nc) {
+        plan[m] = persist_plan(h->start_h.data(), h->adj_h.data(), h->N, h->neq, f32, cv.nc);
+        plan_nc[m] = cv.nc;
+      }
+      if (plan[m].form != kPersistCluster || plan[m].blocks != blocks) continue;
+      PersistSolve a;
+      a.N = h->N;
+      a.neq = h->neq;
+      a.start = h->d_start;
+      a.adj = h->d_adj;
+      a.vals = f32 ? static_cast<const void*>(h->d_vals32) : h->d_vals;
+      a.f32 = f32;
+      a.diagpos = h->d_diagpos;
+      a.b = bw ? bw + off[size_t(m)] : h->d_rhs;
+      a.x = xw ? xw + off[size_t(m)] : h->d_sol;
+      a.r = b->r + off[size_t(m)];
+      a.rh = b->rh + off[size_t(m)];
+      a.q = b->p + off[size_t(m)];
+      a.v = b->v + off[size_t(m)];
+      a.jacobi = pkind != 0;
+      a.nc = cv.nc;
+      a.agg = cv.agg;
+      a.agg_ptr = cv.agg_ptr;
+      a.agg_rows = cv.agg_rows;
+      a.ainv = cv.ainv;
+      a.dctl = b->p_dctl + 16 * m;
+      a.ictl = b->p_ictl + 8 * m;
+      a.tol = tol;
+      a.alpha_max = 1e150;
+      a.maxit = maxit;
+      list.push_back(a);
+      ++g.count;
+      g.smem = std::max(g.smem, plan[m].smem);
+      solved[m] = 1;
+    }
+    if (g.count > 0) groups.push_back(g);
+  }
+  if (list.empty()) return UFEM_OK;
+  UFEM_CUDA_TRY(cudaMemcpyAsync(b->d_solves, list.data(), list.size() * sizeof(PersistSolve), cudaMemcpyHostToDevice, st));
+  UFEM_CUDA_TRY(cudaMemsetAsync(b->p_ictl, 0, sizeof(int) * 8 * n, st));
+  // the largest clusters on `st`, the other sizes on side streams that start after
+  // what `st` holds and that `st` waits for
+  if (groups.size() > 1) {
+    DeviceLock lk(device_mutex());
+    int prio = 0;
+    UFEM_CUDA_TRY(cudaStreamGetPriority(st, &prio));
+    if (!b->fork) UFEM_CUDA_TRY(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
+    for (size_t k = 0; k + 1 < groups.size(); ++k) {
+      if (!b->side[k]) UFEM_CUDA_TRY(cudaStreamCreateWithPriority(&b->side[k], cudaStreamNonBlocking, prio));
+      if (!b->join[k]) UFEM_CUDA_TRY(cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming));
+    }
+    UFEM_CUDA_TRY(cudaEventRecord(b->fork, st));
+  }
+  rc = UFEM_OK;
+  for (size_t k = groups.size(); k-- > 0;) {
+    const Group& g = groups[k];
+    const bool aside = k + 1 < groups.size();
+    const cudaStream_t q = aside ? b->side[k] : st;
+    if (aside) UFEM_CUDA_TRY(cudaStreamWaitEvent(q, b->fork, 0));
+    const int lrc = persist_bicgstab_members(b->d_solves + g.first, g.count, b->neq, f32, g.blocks, g.smem,
+                                             std::max(1, maxit), q);
+    if (lrc) rc = lrc;
+    if (aside) {
+      UFEM_CUDA_TRY(cudaEventRecord(b->join[k], q));
+      UFEM_CUDA_TRY(cudaStreamWaitEvent(st, b->join[k], 0));
+    }
+  }
+  if (rc) return rc;
+  b->p_flags.resize(size_t(8) * n);
+  UFEM_CUDA_TRY(cudaMemcpyAsync(b->p_flags.data(), b->p_ictl, sizeof(int) * 8 * n, cudaMemcpyDeviceToHost, st));
+  UFEM_CUDA_TRY(cudaStreamSynchronize(st));
+  for (int m = 0; m < n; ++m)
+    if (solved[m]) todo[m] = 0;
+  return UFEM_OK;
+}
+
 // BiCGStab over the batch.  MT: operator values; XL/BL: solution and RHS
 // locations; `use_outer`: skip meshes already converged in refinement.
 template <typename MT, int XL, int BL>
-int bicgstab_b(ufem_batch* b, int pkind, double tol, int maxit, bool use_outer, int slot, cudaStream_t st,
-               bool reliable = false, double* xw = nullptr, double* bw = nullptr) {
+int bicgstab_chunks(ufem_batch* b, int pkind, double tol, int maxit, bool use_outer, int slot, cudaStream_t st,
+                    bool reliable, double* xw, double* bw) {
   // xw / bw: the solution and RHS when they are batch work vectors (kWork);
   // for kSol / kRhs they are the members' own arrays and these stay null
   const unsigned nc = unsigned(b->nchunks);
@@ -1164,6 +1295,53 @@ int bicgstab_b(ufem_batch* b, int pkind, double tol, int maxit, bool use_outer, 
       if (fin) break;
     }
   }
+  return UFEM_OK;
+}
+
+// The same with the members that fit one cluster solved there, and the others, if
+// any, by the chunk kernels.  Leaves every member's flags in b->ictl.  The mixed form
+// with residual replacement (`reliable`) runs in the chunk kernels alone.
+template <typename MT, int XL, int BL>
+int bicgstab_b(ufem_batch* b, int pkind, double tol, int maxit, bool use_outer, int slot, cudaStream_t st,
+               bool reliable = false, double* xw = nullptr, double* bw = nullptr) {
+  if (reliable) return bicgstab_chunks<MT, XL, BL>(b, pkind, tol, maxit, use_outer, slot, st, reliable, xw, bw);
+  const int n = b->nmesh;
+  std::vector<int> todo(size_t(n), 1), solved(size_t(n), 0), outer(size_t(n), 0);
+  if (use_outer)
+    for (int m = 0; m < n; ++m) {
+      outer[m] = b->h_ictl[m * kIc + fOuter];
+      todo[m] = outer[m] ? 0 : 1;
+    }
+  int rc;
+  if ((rc = solve_in_clusters<MT>(b, pkind, tol, maxit, xw, bw, todo, solved, st))) return rc;
+  bool any_solved = false, rest = false;
+  for (int m = 0; m < n; ++m) {
+    any_solved = any_solved || solved[m];
+    rest = rest || todo[m];
+  }
+  if (!any_solved) return bicgstab_chunks<MT, XL, BL>(b, pkind, tol, maxit, use_outer, slot, st, false, xw, bw);
+  if (rest) {
+    for (int m = 0; m < n; ++m) {
+      for (int q = 0; q < kIc; ++q) b->h_ictl[m * kIc + q] = 0;
+      b->h_ictl[m * kIc + fOuter] = todo[m] ? 0 : 1;
+    }
+    if ((rc = bicgstab_chunks<MT, XL, BL>(b, pkind, tol, maxit, true, slot, st, false, xw, bw))) return rc;
+    UFEM_CUDA_TRY(cudaMemcpyAsync(b->h_ictl, b->ictl, sizeof(int) * kIc * n, cudaMemcpyDeviceToHost, st));
+    UFEM_CUDA_TRY(cudaStreamSynchronize(st));
+  } else {
+    for (int m = 0; m < n; ++m)
+      for (int q = 0; q < kIc; ++q) b->h_ictl[m * kIc + q] = 0;
+  }
+  for (int m = 0; m < n; ++m) {
+    int* f = b->h_ictl + m * kIc;
+    if (solved[m]) {
+      f[fStatus] = b->p_flags[size_t(8) * m + 2];
+      f[fIters] = b->p_flags[size_t(8) * m + 3];
+    }
+    if (solved[m] || !todo[m]) f[fDone] = f[fFinal] = 1;
+    f[fOuter] = outer[m];
+  }
+  UFEM_CUDA_TRY(cudaMemcpyAsync(b->ictl, b->h_ictl, sizeof(int) * kIc * n, cudaMemcpyHostToDevice, st));
   return UFEM_OK;
 }
 

@@ -1482,8 +1482,7 @@ int solve_persist(KrylovWork& kw, const PersistSolve& a, const PersistPlan& plan
   res.status = kw.h_ictl[2];
   expect = res.iters;
   const double bnorm = kw.h_dctl[kBnorm];
-  if (bnorm == 0.0) {  // a zero RHS has the zero solution
-    UFEM_CUDA_TRY(cudaMemsetAsync(a.x, 0, size_t(a.N) * a.neq * sizeof(double), st));
+  if (bnorm == 0.0) {  // a zero RHS has the zero solution (stored by the kernel)
     res.converged = true;
     res.status = 0;
     return UFEM_OK;

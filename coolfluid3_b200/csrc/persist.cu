@@ -730,6 +730,8 @@ __device__ __forceinline__ void bicgstab_body(const PersistSolve& a, Shared& sh,
       status = 3;
     }
     fresh = done != 0;  // x is the initial guess: its true residual is r
+    if (bnorm == 0.0)   // a zero right-hand side has the zero solution
+      for (int i = threadIdx.x; i < nr; i += kThreads) c.x(i) = 0.0;
     if (rank == 0 && threadIdx.x == 0) {
       a.dctl[kBnorm] = bnorm;
       a.dctl[kBeta] = sqrt(rr);
@@ -910,6 +912,8 @@ __device__ __forceinline__ void cg_body(const PersistSolve& a, Shared& sh, int s
       status = 3;
     }
     fresh = done != 0;
+    if (bnorm == 0.0)
+      for (int i = threadIdx.x; i < nr; i += kThreads) c.x(i) = 0.0;
     if (rank == 0 && threadIdx.x == 0) {
       a.dctl[kBnorm] = bnorm;
       a.dctl[kBeta] = sqrt(rr);
@@ -1024,6 +1028,21 @@ __global__ void __launch_bounds__(kThreads, 1)
     bicgstab_body<NEQ, MT, CL>(a, sh, smem_bytes, int(blockIdx.x), int(gridDim.x), first != 0, iters);
 }
 
+// One cluster per solve of a list (the members of a batch): cluster k runs solve k,
+// with its arguments copied to shared memory (kernel arguments would be indexed by k).
+template <int NEQ, typename MT>
+__global__ void __launch_bounds__(kThreads, 1)
+    persist_members_kernel(const PersistSolve* __restrict__ list, int blocks, int smem_bytes, int iters) {
+  __shared__ Shared sh;
+  __shared__ PersistSolve a;
+  static_assert(sizeof(PersistSolve) % 8 == 0, "copied in 8-byte words");
+  const int k = int(blockIdx.x) / blocks;
+  for (int q = threadIdx.x; q < int(sizeof(PersistSolve) / 8); q += kThreads)
+    reinterpret_cast<unsigned long long*>(&a)[q] = __ldg(reinterpret_cast<const unsigned long long*>(list + k) + q);
+  __syncthreads();
+  bicgstab_body<NEQ, MT, true>(a, sh, smem_bytes, int(blockIdx.x) - k * blocks, blocks, true, iters);
+}
+
 constexpr size_t kSmemMax = 224 * 1024;  // dynamic shared memory of a block (227 KB less the static part)
 
 template <bool CG, int NEQ, typename MT, bool CL>
@@ -1053,6 +1072,26 @@ int launch(const PersistSolve& a, const PersistPlan& plan, bool first, int iters
   cfg.attrs = at;
   cfg.numAttrs = 1;
   UFEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, a, int(plan.smem), first ? 1 : 0, iters));
+  return UFEM_OK;
+}
+
+template <int NEQ, typename MT>
+int launch_members(const PersistSolve* list, int count, int blocks, size_t smem, int iters, cudaStream_t s) {
+  auto kernel = persist_members_kernel<NEQ, MT>;
+  UFEM_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemMax)));
+  UFEM_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(count) * unsigned(blocks));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = unsigned(blocks);
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  UFEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, list, blocks, int(smem), iters));
   return UFEM_OK;
 }
 
@@ -1141,6 +1180,15 @@ PersistPlan persist_plan(const int64_t* start_h, const int32_t* adj_h, int64_t N
     p.smem = kSmemMax;  // what the lists and vectors leave holds values
   }
   return p;
+}
+
+int persist_bicgstab_members(const PersistSolve* d_list, int count, int neq, bool f32, int blocks, size_t smem,
+                             int iters, cudaStream_t s) {
+  if (neq == 3)
+    return f32 ? launch_members<3, float>(d_list, count, blocks, smem, iters, s)
+               : launch_members<3, double>(d_list, count, blocks, smem, iters, s);
+  return f32 ? launch_members<4, float>(d_list, count, blocks, smem, iters, s)
+             : launch_members<4, double>(d_list, count, blocks, smem, iters, s);
 }
 
 int persist_bicgstab(const PersistSolve& a, const PersistPlan& plan, bool first, int iters, cudaStream_t s) {

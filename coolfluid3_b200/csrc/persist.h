@@ -72,4 +72,10 @@ PersistPlan persist_plan(const int64_t* start_h, const int32_t* adj_h, int64_t N
 int persist_bicgstab(const PersistSolve& a, const PersistPlan& plan, bool first, int iters, cudaStream_t s);
 int persist_cg(const PersistSolve& a, const PersistPlan& plan, bool first, int iters, cudaStream_t s);
 
+// BiCGStab of `count` systems of the cluster form (device list; the same `blocks` for
+// all), one cluster each, from their initial residuals to their end or `iters`
+// iterations.  The arithmetic of a solve is persist_bicgstab's.
+int persist_bicgstab_members(const PersistSolve* d_list, int count, int neq, bool f32, int blocks, size_t smem,
+                             int iters, cudaStream_t s);
+
 }  // namespace ufem

@@ -119,3 +119,39 @@ def test_zero_right_hand_side():
     st = ns.solve(precond="jacobi", tol=1e-10)
     assert st["converged"] == 1 and np.all(ns.solution() == 0.0)
     ns.close()
+
+
+@pytest.mark.parametrize("mixed,precond", [(False, "jacobi"), ("matrix_free", "two_level_coupled")])
+def test_batch_members_of_both_forms(mixed, precond):
+    """Members solved in one cluster (of several sizes) and a member too large for one
+    (131 x 131 cells) in one batch: each the bits it has in a batch of its own, its
+    true residual within the tolerance."""
+    from coolfluid3_b200 import Batch
+
+    def member(n):
+        pb = P.make_problem(2, n)
+        ns = NavierStokes(pb.coords, pb.conn, dt=pb.dt, use_specializations=False,
+                          precision="fp32" if mixed else "fp64")
+        ns.set_state(pb.up, pb.lin, pb.nu)
+        ns.add_dirichlet(pb.bc_nodes, pb.bc_comps, pb.bc_values)
+        return ns
+
+    sizes = [4, 131, 12, 40, 25]
+    kr = dict(precond=precond, tol=1e-9, max_iters=6000, mixed=mixed)
+    ms = [member(n) for n in sizes]
+    b = Batch(ms)
+    b.assemble()
+    st = b.solve(**kr)
+    for n, m, s in zip(sizes, ms, st):
+        assert s["converged"] == 1 and s["rel_residual"] <= 1e-9, (n, s)
+        one = member(n)
+        alone = Batch([one])
+        alone.assemble()
+        s1 = alone.solve(**kr)[0]
+        assert s1["iterations"] == s["iterations"]
+        assert np.array_equal(one.solution(), m.solution()), n
+        alone.close()
+        if not mixed:
+            r, bound = residual_and_bound(m, 1e-9)
+            assert r <= bound
+    b.close()
