@@ -1704,13 +1704,11 @@ int ufem_batch_solve(ufem_batch* b, const ufem_krylov_opts* kopts, ufem_krylov_s
   if (o.precond == 4) {
     // every member's coarse space and coarse matrix (of its current system);
     // aggregates capped at kBatchCoarseSide2D^2 (2D) and kBatchCoarseSide3D^3
-    // (3D) boxes, so that the host inversions of all members stay short
+    // (3D) boxes, so that the inversions of all members stay short
     if (b->coarse.size() != size_t(b->nmesh)) b->coarse.assign(size_t(b->nmesh), CoarseView{});
     bool any_new = false;
     std::vector<CoarseView> cv(size_t(b->nmesh));
     std::unique_ptr<bool[]> rebuilt(new bool[size_t(b->nmesh)]);
-    // not lagged: each member's inverse is of its current matrix (with the
-    // previous step's, the hardest cfg4-like members converged less often)
     if ((rc = krylov_coupled_coarse_members(b->members.data(), b->active.data(), b->nmesh, st, kBatchCoarseSide2D,
                                             kBatchCoarseSide3D, rebuilt.get(), cv.data())))
       return rc;

@@ -203,7 +203,6 @@ struct ufem_ns_handle {
   ufem::StagePipe pipe;
   ufem::KrylovWork* kw = nullptr;
   bool vals32_valid = false;            // d_vals32 holds the current system (written by the assembly)
-  bool conditioned = false;             // the Dirichlet conditions ran after the latest assembly
 
   // transfer staging (reference field layouts <-> padded node records)
   double* d_stage = nullptr;      // N x 4*dim doubles
@@ -271,12 +270,8 @@ void destroy_handle(ufem_ns_handle* h);
 int krylov_solve(ufem_ns_handle* h, const ufem_krylov_opts* ko, ufem_krylov_status* st, cudaStream_t s);
 int krylov_apply(ufem_ns_handle* h, const double* d_x, double* d_y, cudaStream_t s);
 int krylov_fp64_residual(ufem_ns_handle* h, double* r_host, cudaStream_t s);
-// Coarse space of the coupled two-level preconditioner of one handle, rebuilt
-// when its Dirichlet plan or the aggregate caps change (rebuilt = true) and its
-// coarse matrix refreshed from the current system (krylov.cu).  lag: from the
-// handle's second refresh on, the inverse is the previous refresh's matrix's,
-// and this refresh's matrix is inverted on a host thread for the next one.
-// nc = 0: no usable coarse space (point Jacobi).
+// Coarse space of the coupled two-level preconditioner of one handle.
+// nc = 0: no coarse space (point Jacobi).
 struct CoarseView {
   int nc = 0;
   const int32_t* agg = nullptr;
@@ -284,17 +279,13 @@ struct CoarseView {
   const int32_t* agg_rows = nullptr;
   const double* ainv = nullptr;
 };
-int krylov_coupled_coarse(ufem_ns_handle* h, cudaStream_t s, int max_side_2d, int max_side_3d, bool* rebuilt,
-                          CoarseView* view, bool lag);
-// The same for the active members of a batch, not lagged: every member's
-// coarse matrix summed and copied on `s`, one synchronisation, the inversions
-// on host threads in parallel (each the one-handle inversion, bitwise), the
-// inverses uploaded on `s`.
+// The coarse spaces of the active members of a batch, rebuilt when a member's
+// Dirichlet plan or the aggregate caps change (rebuilt[m]), and the inverses of
+// their coarse matrices of the current systems, all on `s` (krylov.cu, coarse.cu).
 int krylov_coupled_coarse_members(ufem_ns_handle* const* hs, const int32_t* active, int n, cudaStream_t s,
                                   int max_side_2d, int max_side_3d, bool* rebuilt, CoarseView* views);
 // Aggregate caps (boxes a side) of the coupled two-level preconditioner: one
-// handle (its coarse inverse is computed on a host thread while the previous
-// one is used), and batch members (every member's inverse before the batch solve).
+// handle, and batch members (every member's inverse before the batch solve).
 constexpr int kCoarseSide2D = 20, kCoarseSide3D = 8;
 constexpr int kBatchCoarseSide2D = 16, kBatchCoarseSide3D = 5;
 // Allocations and static preconditioner structure of the solves `ko` describes,

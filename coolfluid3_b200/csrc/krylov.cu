@@ -13,14 +13,13 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
-#include <thread>
 #include <type_traits>
 #include <vector>
 
+#include "coarse.h"
 #include "internal.h"
 #include "persist.h"
 #include "spmv_node.cuh"
@@ -91,20 +90,9 @@ struct KrylovWork {
   int32_t* cp_seg = nullptr;   // cp_nseg + 1 segment starts
   int32_t* cp_dst = nullptr;   // dense index I * nc + J of each segment
   int cp_nseg = 0;
-  double* acd = nullptr;       // nc x nc coarse matrix on the device
-  double* h_ac = nullptr;      // pinned host copy (nc x nc)
+  double* acd = nullptr;       // nc x nc: the other buffer of the inversion (coarse.h)
   int64_t cp_bc_version = -1;  // condition lists the structure was built for (bc_list_version)
   int cp_caps = -1;            // aggregate caps it was built with (2D side * 1000 + 3D side)
-  bool cp_spd = false;         // the coarse inverse on the device is valid
-  // Lagged refresh: the coarse matrix of solve k is inverted on a host thread
-  // while solve k runs with the inverse from solve k-1 (the first solve after a
-  // (re)build inverts its own matrix before it starts).
-  std::thread cp_thread;
-  bool cp_pending = false;     // cp_thread holds the next inverse in h_ac2
-  bool cp_lag_ready = false;   // the device inverse is the latest solve's: the next lagged solve keeps it
-  bool cp_next_spd = false;
-  double* h_ac2 = nullptr;     // pinned: the inverse the thread produces
-  cudaEvent_t cp_event = nullptr;
 };
 
 namespace {
@@ -140,137 +128,6 @@ __device__ __forceinline__ double block_sum(double v, double* sm) {
     for (int k = 0; k < int(blockDim.x >> 5); ++k) s += sm[k];
   __syncthreads();
   return s;
-}
-
-// Runs fn(lo, hi) on nt threads over [n0, n) cut into ranges of equal work
-// (cost(u): the work of unit u); each unit's arithmetic is the same whatever
-// the cut.
-template <typename F, typename C>
-void parallel_ranges(int nt, int n0, int n, C&& cost, F&& fn) {
-  const int extra = (nt <= 1 || n - n0 < 2) ? 0 : acquire_spare_threads(nt - 1);
-  nt = 1 + extra;
-  if (nt <= 1) {
-    fn(n0, n);
-    return;
-  }
-  double total = 0.0;
-  for (int u = n0; u < n; ++u) total += cost(u);
-  std::vector<std::thread> th;
-  int lo = n0;
-  double acc = 0.0;
-  for (int t = 0; t < nt && lo < n; ++t) {
-    int hi = lo;
-    const double goal = total * (t + 1) / nt;
-    while (hi < n && (t + 1 == nt || acc + 0.5 * cost(hi) < goal)) acc += cost(hi++);
-    if (hi == lo) continue;
-    if (hi == n) fn(lo, hi);  // the last range on the calling thread
-    else th.emplace_back(fn, lo, hi);
-    lo = hi;
-  }
-  for (auto& x : th) x.join();
-  release_spare_threads(extra);
-}
-
-// In-place inverse of an SPD matrix (row-major, n x n): A = L L^T, X = L^-1,
-// A^-1 = X^T X (the LAPACK potrf / trtri / lauum sequence, n^3 / 2
-// multiply-adds), every inner loop a contiguous multiply-add over rows that
-// stay in cache (the Cholesky in panels of 32 columns, L^-1 in groups of 8
-// columns, the product in groups of 8 rows).  From n = 256 the last two
-// phases are split over `threads` host threads (default: up to 4, since several
-// handles may refresh their coarse spaces at once), in ranges of equal work;
-// every element's arithmetic is the same whatever the split.  False if a pivot
-// is not positive (a coarse matrix of a system without conditions that fix its
-// constant mode is singular).
-bool spd_invert(double* A, int n, int threads = 0) {
-  const int nt = n < 256 ? 1
-                         : (threads > 0 ? threads
-                                        : int(std::max(1u, std::min(4u, std::thread::hardware_concurrency()))));
-  // Cholesky A = L L^T, right-looking in panels of kPanel columns: every
-  // element receives its updates L[i][k] L[j][k] in ascending k (the order of
-  // the column-by-column algorithm).  The panel is factored in a contiguous
-  // copy P (row i: its kPanel columns); Lt row k holds column k of L.
-  constexpr int kPanel = 32;
-  std::vector<double> W(A, A + size_t(n) * n), Lt(size_t(n) * n, 0.0), P(size_t(n) * kPanel);
-  for (int p0 = 0; p0 < n; p0 += kPanel) {
-    const int p1 = std::min(n, p0 + kPanel), b = p1 - p0;
-    for (int i = p0; i < n; ++i)
-      for (int q = 0; q < b; ++q) P[size_t(i) * kPanel + q] = W[size_t(i) * n + p0 + q];
-    for (int k = p0; k < p1; ++k) {
-      const int kq = k - p0;
-      const double d = P[size_t(k) * kPanel + kq];
-      if (!(d > 0.0) || !std::isfinite(d)) return false;
-      const double lkk = std::sqrt(d);
-      P[size_t(k) * kPanel + kq] = lkk;
-      for (int i = k + 1; i < n; ++i) P[size_t(i) * kPanel + kq] /= lkk;
-      for (int i = k + 1; i < n; ++i) {  // the panel's remaining columns
-        double* __restrict__ pi = &P[size_t(i) * kPanel];
-        const double lik = pi[kq];
-        const int je = std::min(i, p1 - 1) - p0;
-        for (int j = kq + 1; j <= je; ++j) pi[j] -= lik * P[size_t(p0 + j) * kPanel + kq];
-      }
-    }
-    for (int q = 0; q < b; ++q)
-      for (int i = p0 + q; i < n; ++i) Lt[size_t(p0 + q) * n + i] = P[size_t(i) * kPanel + q];
-    if (p1 < n)  // the trailing rows and columns: the panel's rank-b update, on this thread (a
-                 // fork per panel costs more than it saves beside a serving loop's threads)
-      parallel_ranges(1, p1, n, [p1](int i) { return double(i - p1 + 1); }, [&, p0, p1](int r0, int r1) {
-        for (int i = r0; i < r1; ++i) {
-          double* __restrict__ wi = &W[size_t(i) * n];
-          for (int k = p0; k < p1; ++k) {
-            const double* __restrict__ lk = &Lt[size_t(k) * n];
-            const double lik = lk[i];
-            for (int j = p1; j <= i; ++j) wi[j] -= lik * lk[j];
-          }
-        }
-      });
-  }
-  // X = L^-1 by forward substitution, kCols columns at a time (X^T rows of
-  // kCols values: every L column is read once per group of columns).
-  constexpr int kCols = 8;
-  std::vector<double> X(size_t(n) * n, 0.0);  // X[i][c]
-  parallel_ranges(nt, 0, (n + kCols - 1) / kCols,
-                  [n](int g) { const double r = n - g * kCols; return r * r; },
-                  [&](int g0, int g1) {
-    std::vector<double> x(size_t(n) * kCols);
-    for (int g = g0; g < g1; ++g) {
-      const int c0 = g * kCols, w = std::min(kCols, n - c0);
-      std::fill(x.begin(), x.end(), 0.0);
-      for (int q = 0; q < w; ++q) x[size_t(c0 + q) * kCols + q] = 1.0;
-      for (int k = c0; k < n; ++k) {  // row k of x is final once columns < k of L are applied
-        const double* __restrict__ lk = &Lt[size_t(k) * n];
-        double v[kCols];
-        for (int q = 0; q < kCols; ++q) v[q] = x[size_t(k) * kCols + q] / lk[k];
-        for (int q = 0; q < kCols; ++q) x[size_t(k) * kCols + q] = v[q];
-        for (int i = k + 1; i < n; ++i) {
-          const double lik = lk[i];
-          double* __restrict__ xi = &x[size_t(i) * kCols];
-          for (int q = 0; q < kCols; ++q) xi[q] -= lik * v[q];
-        }
-      }
-      for (int i = c0; i < n; ++i)
-        for (int q = 0; q < w; ++q) X[size_t(i) * n + c0 + q] = x[size_t(i) * kCols + q];
-    }
-  });
-  // A^-1 = X^T X: row i = sum over k >= i of X[k][i] X[k][0..k], kRows rows at
-  // a time (each X row is read once per group of rows).
-  constexpr int kRows = 8;
-  parallel_ranges(nt, 0, (n + kRows - 1) / kRows,
-                  [n](int g) { const double r0 = g * kRows; return double(n) * n - r0 * r0; },
-                  [&](int g0, int g1) {
-    for (int g = g0; g < g1; ++g) {
-      const int i0 = g * kRows, h = std::min(kRows, n - i0);
-      for (int r = 0; r < h; ++r) std::fill(A + size_t(i0 + r) * n, A + size_t(i0 + r + 1) * n, 0.0);
-      for (int k = i0; k < n; ++k) {
-        const double* __restrict__ xk = &X[size_t(k) * n];
-        for (int r = 0; r < h && i0 + r <= k; ++r) {
-          const double xki = xk[i0 + r];
-          double* __restrict__ ai = A + size_t(i0 + r) * n;
-          for (int j = 0; j <= k; ++j) ai[j] += xki * xk[j];
-        }
-      }
-    }
-  });
-  return true;
 }
 
 #define GRID_STRIDE(i, n) \
@@ -1849,29 +1706,16 @@ namespace {
 // Aggregates of the coupled two-level form: k^dim boxes of the mesh's bounding
 // box (k chosen for at least 64 nodes a box, at most max_side_3d boxes a side
 // in 3D and max_side_2d in 2D, so the coarse matrix stays small enough to invert
-// on the host at every solve); the coarse space holds the pressure rows of the
+// at every solve); the coarse space holds the pressure rows of the
 // nodes whose pressure is neither a Dirichlet dof nor a periodic slave.  Built
 // once per condition list: the aggregate of each row, the rows of each aggregate, and
 // the pressure-pressure CSR positions sorted by (row aggregate, column
 // aggregate, position) with their segments.
 int coupled_coarse_build(ufem_ns_handle* h, int max_side_2d, int max_side_3d) {
   KrylovWork& kw = *h->kw;
-  if (kw.cp_thread.joinable()) kw.cp_thread.join();
-  kw.cp_pending = false;
-  kw.cp_lag_ready = false;
-  if (kw.h_ac2) {
-    DeviceLock lk(device_mutex());
-    cudaFreeHost(kw.h_ac2);
-    kw.h_ac2 = nullptr;
-  }
   kw.cp_caps = max_side_2d * 1000 + max_side_3d;
   dfree(kw.agg); dfree(kw.agg_ptr); dfree(kw.agg_rows); dfree(kw.ainv); dfree(kw.cvec); dfree(kw.yvec);
   dfree(kw.cp_pos); dfree(kw.cp_seg); dfree(kw.cp_dst); dfree(kw.acd);
-  if (kw.h_ac) {
-    DeviceLock lk(device_mutex());
-    cudaFreeHost(kw.h_ac);
-    kw.h_ac = nullptr;
-  }
   kw.nc = 0;
   kw.cp_nseg = 0;
   kw.cp_bc_version = h->bc_list_version;
@@ -1961,10 +1805,6 @@ int coupled_coarse_build(ufem_ns_handle* h, int max_side_2d, int max_side_3d) {
       (rc = dalloc(&kw.cp_pos, std::max<size_t>(pos.size(), 1))) || (rc = dalloc(&kw.cp_seg, seg.size())) ||
       (rc = dalloc(&kw.cp_dst, std::max<size_t>(dst.size(), 1))) || (rc = dalloc(&kw.acd, size_t(nc) * nc)))
     return rc;
-  {
-    DeviceLock lk(device_mutex());
-    UFEM_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&kw.h_ac), size_t(nc) * nc * sizeof(double)));
-  }
   UFEM_CUDA_TRY(cudaMemcpy(kw.agg, agg.data(), agg.size() * 4, cudaMemcpyHostToDevice));
   UFEM_CUDA_TRY(cudaMemcpy(kw.agg_ptr, ptr.data(), ptr.size() * 4, cudaMemcpyHostToDevice));
   if (!rows.empty()) UFEM_CUDA_TRY(cudaMemcpy(kw.agg_rows, rows.data(), rows.size() * 4, cudaMemcpyHostToDevice));
@@ -1976,64 +1816,21 @@ int coupled_coarse_build(ufem_ns_handle* h, int max_side_2d, int max_side_3d) {
   return UFEM_OK;
 }
 
-// The coarse matrix of the current system (FP64 values, after the Dirichlet
-// pass), its inverse on the host, uploaded for the solve; cp_spd false (point
-// Jacobi for this solve) when it is not positive definite.
-int coupled_coarse_refresh(ufem_ns_handle* h, cudaStream_t s, int max_side_2d = kCoarseSide2D,
-                           int max_side_3d = kCoarseSide3D,
-                           bool* rebuilt = nullptr, bool lag = false) {
+// The coarse space of the handle, rebuilt when its conditions or the caps changed
+// (*rebuilt), and its coarse matrix of the current system (FP64 values, after the
+// Dirichlet pass) summed on `s` into the buffer its inversion starts from.
+int coupled_coarse_matrix(ufem_ns_handle* h, cudaStream_t s, int max_side_2d, int max_side_3d, bool* rebuilt) {
   KrylovWork& kw = *h->kw;
   int rc;
-  const bool stale = kw.cp_bc_version != h->bc_list_version || kw.cp_caps != max_side_2d * 1000 + max_side_3d;
-  if (rebuilt) *rebuilt = stale;
-  if (stale && (rc = coupled_coarse_build(h, max_side_2d, max_side_3d))) return rc;  // (joins the thread)
-  const int nc = kw.nc;
-  if (nc == 0) {
-    kw.cp_spd = false;
-    return UFEM_OK;
-  }
-  const size_t bytes = size_t(nc) * nc * sizeof(double);
-  // lagged: an inverse of the previous solve's coarse matrix exists (on the
-  // device, or on its way from the host thread); this solve uses it
-  const bool lagged = lag && !stale && (kw.cp_pending || kw.cp_lag_ready);
-  if (lagged && kw.cp_pending) {
-    kw.cp_thread.join();
-    kw.cp_pending = false;
-    kw.cp_spd = kw.cp_next_spd;
-    if (kw.cp_spd) UFEM_CUDA_TRY(cudaMemcpyAsync(kw.ainv, kw.h_ac2, bytes, cudaMemcpyHostToDevice, s));
-  }
-  UFEM_CUDA_TRY(cudaMemsetAsync(kw.acd, 0, bytes, s));
+  *rebuilt = kw.cp_bc_version != h->bc_list_version || kw.cp_caps != max_side_2d * 1000 + max_side_3d;
+  if (*rebuilt && (rc = coupled_coarse_build(h, max_side_2d, max_side_3d))) return rc;
+  if (kw.nc == 0) return UFEM_OK;
+  double* ac = coarse_source(CoarseInverse{kw.acd, kw.ainv, kw.nc});
+  UFEM_CUDA_TRY(cudaMemsetAsync(ac, 0, size_t(kw.nc) * kw.nc * sizeof(double), s));
   if (kw.cp_nseg > 0)
     coarse_matrix_kernel<<<unsigned((int64_t(kw.cp_nseg) * 32 + 255) / 256), 256, 0, s>>>(
-        kw.cp_nseg, kw.cp_seg, kw.cp_dst, kw.cp_pos, h->d_vals, kw.acd);
+        kw.cp_nseg, kw.cp_seg, kw.cp_dst, kw.cp_pos, h->d_vals, ac);
   UFEM_CUDA_TRY(cudaGetLastError());
-  UFEM_CUDA_TRY(cudaMemcpyAsync(kw.h_ac, kw.acd, bytes, cudaMemcpyDeviceToHost, s));
-  if (!lagged) {  // invert this solve's own matrix before the solve starts
-    UFEM_CUDA_TRY(cudaStreamSynchronize(s));
-    kw.cp_spd = spd_invert(kw.h_ac, nc);
-    if (kw.cp_spd) UFEM_CUDA_TRY(cudaMemcpyAsync(kw.ainv, kw.h_ac, bytes, cudaMemcpyHostToDevice, s));
-    kw.cp_lag_ready = lag;  // the next lagged solve keeps this inverse
-    return UFEM_OK;
-  }
-  // the next solve's inverse: this solve's matrix, inverted on a host thread
-  // once its copy has landed, while this solve runs
-  if (!kw.h_ac2) {
-    DeviceLock lk(device_mutex());
-    UFEM_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&kw.h_ac2), bytes));
-  }
-  if (!kw.cp_event) UFEM_CUDA_TRY(cudaEventCreateWithFlags(&kw.cp_event, cudaEventDisableTiming));
-  UFEM_CUDA_TRY(cudaEventRecord(kw.cp_event, s));
-  double* src = kw.h_ac;
-  double* dst = kw.h_ac2;
-  cudaEvent_t ev = kw.cp_event;
-  KrylovWork* kwp = &kw;
-  kw.cp_thread = std::thread([src, dst, bytes, nc, ev, kwp]() {
-    const bool ok = cudaEventSynchronize(ev) == cudaSuccess;
-    if (ok) std::memcpy(dst, src, bytes);
-    kwp->cp_next_spd = ok && spd_invert(dst, nc);
-  });
-  kw.cp_pending = true;
-  kw.cp_lag_ready = false;
   return UFEM_OK;
 }
 
@@ -2055,108 +1852,26 @@ int krylov_prepare(ufem_ns_handle* h, const ufem_krylov_opts* ko, int batched) {
     if ((kw.cp_bc_version != h->bc_list_version || kw.cp_caps != s2 * 1000 + s3) &&
         (rc = coupled_coarse_build(h, s2, s3)))
       return rc;
-    if (!batched && h->conditioned) {
-      // the coarse inverse of the system as it stands, which the next solve
-      // takes as its lagged inverse: the first solve after this does not wait
-      // for a host inversion (on a private stream; nothing else is touched)
-      cudaStream_t ps = nullptr;
-      UFEM_CUDA_TRY(cudaStreamCreateWithFlags(&ps, cudaStreamNonBlocking));
-      rc = coupled_coarse_refresh(h, ps, s2, s3, nullptr, true);
-      const cudaError_t ce = cudaStreamSynchronize(ps);
-      cudaStreamDestroy(ps);
-      if (rc) return rc;
-      if (ce != cudaSuccess) return set_error(UFEM_ERR_CUDA, std::string("prepare: ") + cudaGetErrorString(ce));
-    }
   }
   return UFEM_OK;
 }
 
 int krylov_coupled_coarse_members(ufem_ns_handle* const* hs, const int32_t* active, int n, cudaStream_t s,
                                   int max_side_2d, int max_side_3d, bool* rebuilt, CoarseView* views) {
-  // (1) every active member's coarse matrix, summed on the device and copied
-  // to its pinned host buffer, all on `s`
   int rc;
+  std::vector<CoarseInverse> list;
   for (int m = 0; m < n; ++m) {
     rebuilt[m] = false;
+    views[m] = CoarseView{};
     if (!active[m]) continue;
     ufem_ns_handle* h = hs[m];
     if (!h->kw) h->kw = new KrylovWork();  // coarse data only: batch members keep their vectors in the batch
     KrylovWork& kw = *h->kw;
-    if (kw.cp_pending) {  // a lagged inversion from solves of the handle on its own
-      kw.cp_thread.join();
-      kw.cp_pending = false;
-    }
-    const bool stale = kw.cp_bc_version != h->bc_list_version || kw.cp_caps != max_side_2d * 1000 + max_side_3d;
-    rebuilt[m] = stale;
-    if (stale && (rc = coupled_coarse_build(h, max_side_2d, max_side_3d))) return rc;
-    if (kw.nc == 0) continue;
-    const size_t bytes = size_t(kw.nc) * kw.nc * sizeof(double);
-    UFEM_CUDA_TRY(cudaMemsetAsync(kw.acd, 0, bytes, s));
-    if (kw.cp_nseg > 0)
-      coarse_matrix_kernel<<<unsigned((int64_t(kw.cp_nseg) * 32 + 255) / 256), 256, 0, s>>>(
-          kw.cp_nseg, kw.cp_seg, kw.cp_dst, kw.cp_pos, h->d_vals, kw.acd);
-    UFEM_CUDA_TRY(cudaGetLastError());
-    UFEM_CUDA_TRY(cudaMemcpyAsync(kw.h_ac, kw.acd, bytes, cudaMemcpyDeviceToHost, s));
+    if ((rc = coupled_coarse_matrix(h, s, max_side_2d, max_side_3d, &rebuilt[m]))) return rc;
+    if (kw.nc > 0) list.push_back({kw.acd, kw.ainv, kw.nc});
+    views[m] = CoarseView{kw.nc, kw.agg, kw.agg_ptr, kw.agg_rows, kw.ainv};
   }
-  // (2) one synchronisation, (3) the inversions on host threads, one member
-  // per thread at a time (each inversion's arithmetic is the one-handle
-  // refresh's: the same inverse, bitwise), (4) the inverses uploaded
-  UFEM_CUDA_TRY(cudaStreamSynchronize(s));
-  std::vector<int> todo;
-  for (int m = 0; m < n; ++m)
-    if (active[m] && hs[m]->kw->nc > 0) todo.push_back(m);
-  std::vector<char> spd(size_t(n), 0);
-  const int extra = todo.size() > 1 ? acquire_spare_threads(int(todo.size()) - 1) : 0;
-  const int nt = 1 + extra;
-  std::atomic<size_t> next{0};
-  auto work = [&]() {
-    for (size_t q = next++; q < todo.size(); q = next++) {
-      const int m = todo[q];
-      KrylovWork& kw = *hs[m]->kw;
-      spd[size_t(m)] = spd_invert(kw.h_ac, kw.nc, 1) ? 1 : 0;
-    }
-  };
-  {
-    std::vector<std::thread> th;
-    for (int t = 1; t < nt; ++t) th.emplace_back(work);
-    work();  // the calling thread takes members too
-    for (auto& x : th) x.join();
-  }
-  release_spare_threads(extra);
-  for (int m = 0; m < n; ++m) {
-    views[m] = CoarseView{};
-    if (!active[m]) continue;
-    KrylovWork& kw = *hs[m]->kw;
-    if (kw.nc == 0) {
-      kw.cp_spd = false;
-    } else {
-      kw.cp_spd = spd[size_t(m)] != 0;
-      if (kw.cp_spd)
-        UFEM_CUDA_TRY(cudaMemcpyAsync(kw.ainv, kw.h_ac, size_t(kw.nc) * kw.nc * sizeof(double),
-                                      cudaMemcpyHostToDevice, s));
-      kw.cp_lag_ready = false;
-    }
-    views[m].nc = kw.cp_spd ? kw.nc : 0;
-    views[m].agg = kw.agg;
-    views[m].agg_ptr = kw.agg_ptr;
-    views[m].agg_rows = kw.agg_rows;
-    views[m].ainv = kw.ainv;
-  }
-  return UFEM_OK;
-}
-
-int krylov_coupled_coarse(ufem_ns_handle* h, cudaStream_t s, int max_side_2d, int max_side_3d, bool* rebuilt,
-                          CoarseView* view, bool lag) {
-  if (!h->kw) h->kw = new KrylovWork();  // coarse data only: batch members keep their vectors in the batch
-  int rc;
-  if ((rc = coupled_coarse_refresh(h, s, max_side_2d, max_side_3d, rebuilt, lag))) return rc;
-  const KrylovWork& kw = *h->kw;
-  view->nc = kw.cp_spd ? kw.nc : 0;
-  view->agg = kw.agg;
-  view->agg_ptr = kw.agg_ptr;
-  view->agg_rows = kw.agg_rows;
-  view->ainv = kw.ainv;
-  return UFEM_OK;
+  return coarse_invert(list.data(), int(list.size()), s);
 }
 
 int krylov_solve(ufem_ns_handle* h, const ufem_krylov_opts* ko, ufem_krylov_status* st, cudaStream_t s) {
@@ -2179,11 +1894,14 @@ int krylov_solve(ufem_ns_handle* h, const ufem_krylov_opts* ko, ufem_krylov_stat
   const bool bicg = o.method == 1 || use_cg;  // CG uses the BiCGStab work vectors
   int rc;
   if ((rc = ensure_work(h, o.restart, mixed, bicg))) return rc;
-  if (o.precond == 4) {  // coarse matrix of this system; point Jacobi when it is not positive definite
-    // lagged: from the second solve on, each solve uses the previous solve's coarse
-    // inverse while its own matrix is inverted on a host thread for the next one
-    if ((rc = coupled_coarse_refresh(h, s, kCoarseSide2D, kCoarseSide3D, nullptr, true))) return rc;
-    if (!h->kw->cp_spd) o.precond = 1;
+  if (o.precond == 4) {
+    // the inverse of this system's coarse matrix; zero (which is point Jacobi)
+    // when the matrix is not positive definite
+    bool rebuilt;
+    if ((rc = coupled_coarse_matrix(h, s, kCoarseSide2D, kCoarseSide3D, &rebuilt))) return rc;
+    const CoarseInverse ci{h->kw->acd, h->kw->ainv, h->kw->nc};
+    if (ci.n == 0) o.precond = 1;
+    else if ((rc = coarse_invert(&ci, 1, s))) return rc;
   }
   KrylovWork& kw = *h->kw;
   const int64_t n = h->nrows;
@@ -2328,15 +2046,6 @@ int ensure_vals32(ufem_ns_handle* h, cudaStream_t s) {
   return UFEM_OK;
 }
 
-namespace {
-
-// In-place inverse of an SPD matrix through its Cholesky factor; false if a
-// pivot is not positive (the coarse matrix of a system without conditions
-// that fix its constant mode is singular).
-bool spd_inverse(std::vector<double>& A, int n) { return spd_invert(A.data(), n); }
-
-}  // namespace
-
 int krylov_set_coarse(ufem_ns_handle* h, const std::vector<int32_t>& agg, int nc, cudaStream_t s) {
   if (h->neq != 1) return set_error(UFEM_ERR_ARG, "aggregates are defined for one-equation systems");
   if (int64_t(agg.size()) != h->nrows) return set_error(UFEM_ERR_ARG, "one aggregate id per row expected");
@@ -2373,15 +2082,26 @@ int krylov_set_coarse(ufem_ns_handle* h, const std::vector<int32_t>& agg, int nc
       if (J >= 0) A[size_t(I) * nc + J] += vals[size_t(q)];
     }
   }
-  if (!spd_inverse(A, nc)) return UFEM_OK;  // nc stays 0: the caller falls back to point Jacobi
+  // an inverse of zeros: nc stays 0 and the caller falls back to point Jacobi
+  if ((rc = dalloc(&kw.ainv, A.size())) || (rc = dalloc(&kw.acd, A.size()))) return rc;
+  const CoarseInverse ci{kw.acd, kw.ainv, nc};
+  UFEM_CUDA_TRY(cudaMemcpyAsync(coarse_source(ci), A.data(), A.size() * 8, cudaMemcpyHostToDevice, s));
+  if ((rc = coarse_invert(&ci, 1, s))) return rc;
+  double first = 0.0;  // positive in the inverse of an SPD matrix
+  UFEM_CUDA_TRY(cudaMemcpyAsync(&first, kw.ainv, sizeof(double), cudaMemcpyDeviceToHost, s));
+  UFEM_CUDA_TRY(cudaStreamSynchronize(s));
+  dfree(kw.acd);
+  if (!(first > 0.0)) {
+    dfree(kw.ainv);
+    return UFEM_OK;
+  }
   if ((rc = dalloc(&kw.agg, size_t(h->nrows))) || (rc = dalloc(&kw.agg_ptr, ptr.size())) ||
-      (rc = dalloc(&kw.agg_rows, std::max<size_t>(rows.size(), 1))) || (rc = dalloc(&kw.ainv, A.size())) ||
+      (rc = dalloc(&kw.agg_rows, std::max<size_t>(rows.size(), 1))) ||
       (rc = dalloc(&kw.cvec, size_t(nc))) || (rc = dalloc(&kw.yvec, size_t(2) * nc)))
     return rc;
   UFEM_CUDA_TRY(cudaMemcpy(kw.agg, agg.data(), agg.size() * 4, cudaMemcpyHostToDevice));
   UFEM_CUDA_TRY(cudaMemcpy(kw.agg_ptr, ptr.data(), ptr.size() * 4, cudaMemcpyHostToDevice));
   if (!rows.empty()) UFEM_CUDA_TRY(cudaMemcpy(kw.agg_rows, rows.data(), rows.size() * 4, cudaMemcpyHostToDevice));
-  UFEM_CUDA_TRY(cudaMemcpy(kw.ainv, A.data(), A.size() * 8, cudaMemcpyHostToDevice));
   kw.nc = nc;
   return UFEM_OK;
 }
@@ -2428,12 +2148,8 @@ void krylov_free(ufem_ns_handle* h) {
   dfree(k.part); dfree(k.hbuf); dfree(k.H); dfree(k.cs); dfree(k.sn); dfree(k.g); dfree(k.y);
   dfree(k.dctl); dfree(k.ictl); dfree(k.cg_counter);
   dfree(k.agg); dfree(k.agg_ptr); dfree(k.agg_rows); dfree(k.ainv); dfree(k.cvec); dfree(k.yvec);
-  if (k.cp_thread.joinable()) k.cp_thread.join();
   dfree(k.cp_pos); dfree(k.cp_seg); dfree(k.cp_dst); dfree(k.acd);
   DeviceLock lk(device_mutex());
-  if (k.h_ac) cudaFreeHost(k.h_ac);
-  if (k.h_ac2) cudaFreeHost(k.h_ac2);
-  if (k.cp_event) cudaEventDestroy(k.cp_event);
   for (auto& g : k.cg_graph)
     if (g.exec) cudaGraphExecDestroy(g.exec);
   for (auto& g : k.bicg_graph)

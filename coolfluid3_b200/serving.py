@@ -453,9 +453,8 @@ class Server:
                 # the one-time work of the first step on this host thread, not on
                 # the worker that steps the request: the Dirichlet plan (built by
                 # the first conditioning of an assembled system), the solver
-                # workspace, the preconditioner structure and, for one handle,
-                # the coarse inverse of the first system (which its first solve
-                # would otherwise compute first); the state is unchanged
+                # workspace and the preconditioner structure; the state is
+                # unchanged
                 s = torch.cuda.Stream()
                 ns.assemble(s)
                 ns.apply_dirichlet(s)
