@@ -78,7 +78,7 @@ struct KrylovWork {
   int32_t* agg_ptr = nullptr;  // nc + 1
   int32_t* agg_rows = nullptr; // the members of each aggregate, ascending
   double* ainv = nullptr;      // nc x nc, row-major
-  double* cvec = nullptr;      // nc: R^T r
+  double* cvec = nullptr;      // 2 nc: R^T r (the persistent BiCGStab keeps two)
   double* yvec = nullptr;      // 2 nc: Ac^-1 R^T r (the persistent BiCGStab keeps two)
   // Two-level preconditioner of the coupled system (precond 4): point Jacobi
   // plus the same piecewise-constant correction on aggregates of pressure rows
@@ -1402,6 +1402,10 @@ int bicgstab(ufem_ns_handle* h, KrylovWork& kw, const MT* vals, const BT* b, VT*
       a.rh = rh;
       a.q = p;
       a.v = v;
+      const bool two = a.nc > 0;
+      a.r2 = two ? sv : r;
+      a.q2 = two ? ph : p;
+      a.t = tv;
       a.alpha_max = alpha_max;
       return solve_persist(kw, a, plan, false, kw.bicg_expect[f32], st, res);
     }
@@ -1600,8 +1604,10 @@ int cg(ufem_ns_handle* h, KrylovWork& kw, const MT* vals, const BT* b, VT* x, VT
     if (plan.form != kPersistNone) {
       PersistSolve a = persist_args<MT>(h, kw, vals, b, x, pkind, tol, maxit);
       a.r = r;
-      a.q = p;
+      a.q = a.q2 = p;
       a.v = z;
+      a.r2 = a.nc > 0 ? dinv : r;
+      a.t = q;
       return solve_persist(kw, a, plan, true, kw.cg_expect[f32], st, res);
     }
   }
@@ -1801,7 +1807,7 @@ int coupled_coarse_build(ufem_ns_handle* h, int max_side_2d, int max_side_3d) {
   int rc;
   if ((rc = dalloc(&kw.agg, agg.size())) || (rc = dalloc(&kw.agg_ptr, ptr.size())) ||
       (rc = dalloc(&kw.agg_rows, std::max<size_t>(rows.size(), 1))) || (rc = dalloc(&kw.ainv, size_t(nc) * nc)) ||
-      (rc = dalloc(&kw.cvec, size_t(nc))) || (rc = dalloc(&kw.yvec, size_t(2) * nc)) ||
+      (rc = dalloc(&kw.cvec, size_t(2) * nc)) || (rc = dalloc(&kw.yvec, size_t(2) * nc)) ||
       (rc = dalloc(&kw.cp_pos, std::max<size_t>(pos.size(), 1))) || (rc = dalloc(&kw.cp_seg, seg.size())) ||
       (rc = dalloc(&kw.cp_dst, std::max<size_t>(dst.size(), 1))) || (rc = dalloc(&kw.acd, size_t(nc) * nc)))
     return rc;
@@ -2097,7 +2103,7 @@ int krylov_set_coarse(ufem_ns_handle* h, const std::vector<int32_t>& agg, int nc
   }
   if ((rc = dalloc(&kw.agg, size_t(h->nrows))) || (rc = dalloc(&kw.agg_ptr, ptr.size())) ||
       (rc = dalloc(&kw.agg_rows, std::max<size_t>(rows.size(), 1))) ||
-      (rc = dalloc(&kw.cvec, size_t(nc))) || (rc = dalloc(&kw.yvec, size_t(2) * nc)))
+      (rc = dalloc(&kw.cvec, size_t(2) * nc)) || (rc = dalloc(&kw.yvec, size_t(2) * nc)))
     return rc;
   UFEM_CUDA_TRY(cudaMemcpy(kw.agg, agg.data(), agg.size() * 4, cudaMemcpyHostToDevice));
   UFEM_CUDA_TRY(cudaMemcpy(kw.agg_ptr, ptr.data(), ptr.size() * 4, cudaMemcpyHostToDevice));

@@ -13,7 +13,9 @@
 // which saves the barrier between forming a direction and applying the matrix
 // to it; p, s and their preconditioned forms are never stored.  The two-level
 // forms add a barrier after the restriction and one after the coarse product
-// before each product; the correction enters with that copy.
+// before each product; the correction enters with that copy.  (In the grid form a
+// restriction of the updated residual is summed beside the update, from its
+// published terms, and needs no barrier of its own.)
 //
 // Two forms (persist_plan chooses):
 //  - cluster: up to 16 blocks of one thread-block cluster; vectors and matrix live
@@ -30,8 +32,10 @@
 // What bounds it: barriers and the latency of each phase, not bytes.  An
 // iteration, launches against this: 64 x 64 x 2 triangles, BiCGStab with point
 // Jacobi, 27 -> 9.3 us (cluster of 16); 24^3 x 6 tetrahedra, two-level BiCGStab,
-// 46 -> 29 us; 32^3 x 6, two-level CG of the pressure 29 -> 13.5 us, CG of the
-// velocity 24 -> 15 us (grid).
+// 46 -> 22 us; 32^3 x 6, two-level CG of the pressure 29 -> 12 us, CG of the
+// velocity 24 -> 15 us (grid).  (With the restriction after the update and its own
+// barrier, and the coarse sums' last rows one at a time, the two-level forms took 27
+// and 13.5 us.)
 //
 // All sums run in fixed orders, so a solve is deterministic; FP64 throughout,
 // FP32 only in the stored values of the mixed forms.  Grid barriers wait a
@@ -124,6 +128,7 @@ struct Ctx {
   int nslice;       // slices of NPW nodes whose values are in shared memory (the first of the range)
   int64_t base;     // the range's first block entry
   int epoch = 0;
+  int par = 0;      // which of the two global copies of r and q is the current one (grid form)
   int wide;         // entries of one vector's place in shared memory
   // byte places in shared memory (Layout)
   int o_off, o_soff, o_adj, o_touched, o_tagg, o_dinv, o_u, o_vals, o_coarse;
@@ -138,7 +143,9 @@ struct Ctx {
   __device__ __forceinline__ double& v(int i) const { return vec(4)[i]; }
   __device__ __forceinline__ double& t(int i) const { return vec(5)[i]; }
   // The global copy of vectors 1, 3 and 4 (grid form: what other blocks read).
-  __device__ __forceinline__ double* global(int k) const { return k == 1 ? a.r : k == 3 ? a.q : a.v; }
+  __device__ __forceinline__ double* global(int k) const {
+    return k == 1 ? (par ? a.r2 : a.r) : k == 3 ? (par ? a.q2 : a.q) : a.v;
+  }
   // Stores entry i of vector k where its readers look for it.
   __device__ __forceinline__ void publish(int k, int i, double s) const {
     vec(k)[i] = s;
@@ -262,7 +269,7 @@ struct Ctx {
   __device__ __forceinline__ void fill(int kw, double k, int ky, bool plain = false) const {
     constexpr int Q = 4;
     const uint32_t dw = uint32_t((kw - 1) * wide) * 8u;
-    const double* gr = a.r;
+    const double* gr = global(1);
     const double* gw = global(kw);
     const double* y = ky ? coarse_vec(ky) : nullptr;
     const int* list = touched();
@@ -439,37 +446,84 @@ struct Ctx {
       if (lane == 0) w[I] = s;
     }
   }
-  // y = Ac^-1 R^T value (coarse vector ky): one warp per aggregate and per coarse
-  // row, a barrier after the restriction (the caller's next one covers y).  cy: the
-  // thread's share of c . y.
-  template <typename F>
-  __device__ __forceinline__ bool correct(int ky, F&& at, double* cy) {
+  // K coarse vectors (the first of them coarse_vec(0), the others after it: grid form)
+  // from the rows of each aggregate, one warp an aggregate, the block's last warps
+  // first: at(row, shares) gives a row's shares.  Four rows a lane in flight, the last
+  // ones too (a remainder loop would wait for the L2 once a row).
+  template <int K, typename F>
+  __device__ __forceinline__ void restrict_rows(F&& at) const {
+    const int lane = threadIdx.x & 31, warp = int(threadIdx.x >> 5);
     double* cs = coarse_vec(0);
+#pragma unroll 1
+    for (int k = kWarps - 1 - warp; rank + k * blocks < a.nc; k += kWarps) {
+      const int* list = agg_rows_of(k);
+      const int p0 = list[0], len = list[1];
+      double s[K];
+#pragma unroll
+      for (int q = 0; q < K; ++q) s[q] = 0.0;
+      constexpr int Q = 4;
+      const int near = min(len, kAggRows - 2);
+#pragma unroll 1
+      for (int j0 = lane; j0 < len; j0 += Q * 32) {
+        double v[Q][K];
+#pragma unroll
+        for (int b = 0; b < Q; ++b) {
+          const int j = min(j0 + b * 32, len - 1);
+          at(j < near ? list[2 + j] : __ldg(a.agg_rows + p0 + j), v[b]);
+        }
+#pragma unroll
+        for (int b = 0; b < Q; ++b)
+#pragma unroll
+          for (int q = 0; q < K; ++q)
+            if (j0 + b * 32 < len) s[q] += v[b][q];
+      }
+#pragma unroll
+      for (int q = 0; q < K; ++q) put(cs + q * a.nc, rank + k * blocks, wsum(s[q]));
+    }
+  }
+  // y = Ac^-1 c (coarse vector ky), c = coarse_vec(0), PAIR: plus k2 times the one
+  // after it; one warp a coarse row.  cy: the thread's share of c . y.
+  template <bool PAIR>
+  __device__ __forceinline__ void coarse_product(int ky, double k2, double* cy) const {
+    const double* cs = coarse_vec(0);
     double* y = coarse_vec(ky);
     const int lane = threadIdx.x & 31, warp = int(threadIdx.x >> 5);
-#pragma unroll 1
-    for (int k = warp; rank + k * blocks < a.nc; k += kWarps) {
-      const int I = rank + k * blocks;
-      const int* list = agg_rows_of(k);
-      const int p0 = __ldg(a.agg_ptr + I), len = __ldg(a.agg_ptr + I + 1) - p0, near = min(len, kAggRows);
-      double s = 0.0;
-#pragma unroll 4
-      for (int j = lane; j < near; j += 32) s += at(list[j]);
-      for (int j = kAggRows + lane; j < len; j += 32) s += at(__ldg(a.agg_rows + p0 + j));
-      put(cs, I, wsum(s));
-    }
-    if (!barrier()) return false;
+    auto entry = [&](int J) {
+      double v = CL ? cs[J] : __ldcg(cs + J);
+      if constexpr (PAIR) v += k2 * __ldcg(cs + a.nc + J);
+      return v;
+    };
 #pragma unroll 1
     for (int k = warp; rank + k * blocks < a.nc; k += kWarps) {
       const int I = rank + k * blocks;
       const double* inv = a.ainv + int64_t(I) * a.nc;
       double s = 0.0;
-#pragma unroll 8
-      for (int J = lane; J < a.nc; J += 32) s += __ldg(inv + J) * (CL ? cs[J] : __ldcg(cs + J));
+      constexpr int Q = 8;  // in flight, the last ones too
+#pragma unroll 1
+      for (int J0 = lane; J0 < a.nc; J0 += Q * 32) {
+        double m[Q], v[Q];
+#pragma unroll
+        for (int b = 0; b < Q; ++b) {
+          const int J = min(J0 + b * 32, a.nc - 1);
+          m[b] = __ldg(inv + J);
+          v[b] = entry(J);
+        }
+#pragma unroll
+        for (int b = 0; b < Q; ++b)
+          if (J0 + b * 32 < a.nc) s += m[b] * v[b];
+      }
       s = wsum(s);
       put(y, I, s);
-      if (cy != nullptr && lane == 0) *cy += (CL ? cs[I] : __ldcg(cs + I)) * s;
+      if (cy != nullptr && lane == 0) *cy += entry(I) * s;
     }
+  }
+  // y = Ac^-1 R^T value(row), a barrier between the two (the caller's next one
+  // covers y).
+  template <typename F>
+  __device__ __forceinline__ bool correct(int ky, F&& value, double* cy) {
+    restrict_rows<1>([&](int i, double (&s)[1]) { s[0] = value(i); });
+    if (!barrier()) return false;
+    coarse_product<false>(ky, 0.0, cy);
     return true;
   }
 };
@@ -655,7 +709,10 @@ __device__ __forceinline__ void setup(Ctx<NEQ, MT, CL>& c, int smem_bytes) {
   for (int i = threadIdx.x; i < nr; i += kThreads) c.x(i) = a.x[r0 + i];
   for (int k = threadIdx.x >> 5; c.rank + k * c.blocks < a.nc; k += kWarps) {
     const int p0 = __ldg(a.agg_ptr + c.rank + k * c.blocks), p1 = __ldg(a.agg_ptr + c.rank + k * c.blocks + 1);
-    for (int j = lane; j < min(p1 - p0, kAggRows); j += 32) c.agg_rows_of(k)[j] = __ldg(a.agg_rows + p0 + j);
+    int* list = c.agg_rows_of(k);  // where its rows start, how many, and the first of them
+    if (lane == 0) list[0] = p0;
+    if (lane == 0) list[1] = p1 - p0;
+    for (int j = lane; j < min(p1 - p0, kAggRows - 2); j += 32) list[2 + j] = __ldg(a.agg_rows + p0 + j);
   }
   __syncthreads();
   if constexpr (CL) cluster_sync();  // every block of the cluster runs and its partials are cleared
@@ -678,7 +735,7 @@ __device__ __forceinline__ bool begin(Ctx<NEQ, MT, CL>& c, double (&rr)[3], bool
     rr[1] += bi * bi;
     rr[2] += ri * (c.dinv(i) * ri);
   });
-  return c.template sum<3>(0, rr);
+  return c.template sum<3>(5, rr);  // (the loop's first sum follows at once: other slots)
 }
 
 // ||b - A x||^2 of the stored x; every block has passed a barrier since the last
@@ -753,7 +810,18 @@ __device__ __forceinline__ void bicgstab_body(const PersistSolve& a, Shared& sh,
 #pragma unroll 1
   for (int it = 0; it < iters && !done && !late; ++it) {
     if (two) {
-      late = !c.correct(1, [&](int i) { return c.row_of(1, a.r, i) + beta * c.row_of(3, a.q, i); }, nullptr);
+      if constexpr (CL) {
+        late = !c.correct(1, [&](int i) { return c.row_of(1, a.r, i) + beta * c.row_of(3, a.q, i); }, nullptr);
+      } else {
+        if (it == 0) {  // later ones: beside the update below
+          c.template restrict_rows<2>([&](int i, double (&s)[2]) {
+            s[0] = c.row_of(1, a.r, i);
+            s[1] = c.row_of(3, a.q, i);
+          });
+          late = !c.barrier();
+        }
+        if (!late) c.template coarse_product<true>(1, beta, nullptr);
+      }
       if (late || !c.barrier()) {
         late = true;
         break;
@@ -783,7 +851,8 @@ __device__ __forceinline__ void bicgstab_body(const PersistSolve& a, Shared& sh,
     }
     alpha = al;
     if (two) {
-      late = !c.correct(2, [&](int i) { return c.row_of(1, a.r, i) - alpha * c.row_of(4, a.v, i); }, nullptr);
+      const double* gr = c.global(1);
+      late = !c.correct(2, [&](int i) { return c.row_of(1, gr, i) - alpha * c.row_of(4, a.v, i); }, nullptr);
       if (late || !c.barrier()) {
         late = true;
         break;
@@ -794,6 +863,8 @@ __device__ __forceinline__ void bicgstab_body(const PersistSolve& a, Shared& sh,
     c.fill(4, -alpha, two ? 2 : 0);
     c.product([&](int i, double ti) {
       c.t(i) = ti;
+      if constexpr (!CL)
+        if (two) a.t[r0 + i] = ti;
       d2[0] += ti * (c.r(i) - alpha * c.v(i));
       d2[1] += ti * ti;
     });
@@ -810,8 +881,22 @@ __device__ __forceinline__ void bicgstab_body(const PersistSolve& a, Shared& sh,
     // t.s = 0 with t != 0: the next beta would divide by omega (breakdown);
     // x still advances by alpha ph before stopping
     if (omega == 0.0 && d2[1] != 0.0) status = 2;
-    // x, r and the next q; r . r and rh . r
+    // x, r and the next q; r . r and rh . r.  Grid form, two-level: the aggregates'
+    // sums of r and q from what was published before the last barrier (so r and q
+    // alternate between two copies), which saves a barrier after this update
     double d3[2] = {0.0, 0.0};
+    if constexpr (!CL) {
+      if (two) {
+        const double *gr = c.global(1), *gq = c.global(3);
+        c.template restrict_rows<2>([&](int i, double (&s)[2]) {
+          const double ri = __ldcg(gr + i), qi = __ldcg(gq + i), vi = __ldcg(a.v + i), ti = __ldcg(a.t + i);
+          const double pi = ri + beta * qi, si = ri - alpha * vi;
+          s[0] = si - omega * ti;
+          s[1] = pi - omega * vi;
+        });
+      }
+      c.par ^= 1;
+    }
 #pragma unroll 1
     for (int i = threadIdx.x; i < nr; i += kThreads) {
       const double ri = c.r(i), qi = c.q(i), vi = c.v(i), di = c.dinv(i);
@@ -858,10 +943,8 @@ __device__ __forceinline__ void bicgstab_body(const PersistSolve& a, Shared& sh,
     a.x[r0 + i] = c.x(i);
     if (!done) {
       a.rh[r0 + i] = c.rh(i);
-      if constexpr (CL) {
-        a.r[r0 + i] = c.r(i);
-        a.q[r0 + i] = c.q(i);
-      }
+      a.r[r0 + i] = c.r(i);
+      a.q[r0 + i] = c.q(i);
     }
   }
   double tr = rr;
@@ -892,9 +975,11 @@ __device__ __forceinline__ void cg_body(const PersistSolve& a, Shared& sh, int s
   bool late = false, fresh = false;
   // y = Ac^-1 R^T r (z = D^-1 r + y[aggregate] is formed where it is read);
   // r . z = r . D^-1 r + c . y
-  auto coarse = [&](double rz) {
+  // (c: the restriction is there already)
+  auto coarse = [&](double rz, bool c_ready) {
     double d[1] = {0.0};
-    if (!c.correct(1, [&](int i) { return c.row_of(1, a.r, i); }, d)) late = true;
+    if (!c_ready) late = !c.correct(1, [&](int i) { return c.row_of(1, c.global(1), i); }, d);
+    else c.template coarse_product<false>(1, 0.0, d);
     if (late || !c.template sum<1>(6, d)) late = true;
     return rz + d[0];
   };
@@ -905,7 +990,7 @@ __device__ __forceinline__ void cg_body(const PersistSolve& a, Shared& sh, int s
     rho = w[2];
     const double bnorm = sqrt(w[1]);
     limit = a.tol * bnorm;
-    if (two && !late) rho = coarse(rho);
+    if (two && !late) rho = coarse(rho, false);
     done = (sqrt(rr) <= limit || bnorm == 0.0) ? 1 : 0;
     if (!isfinite(rr)) {
       done = 1;
@@ -931,7 +1016,7 @@ __device__ __forceinline__ void cg_body(const PersistSolve& a, Shared& sh, int s
       c.v(i) = a.v[r0 + i];
     }
     if (!late) late = !c.barrier();
-    if (two && !late) coarse(0.0);  // y of the interrupted iteration
+    if (two && !late) coarse(0.0, false);  // y of the interrupted iteration
   }
 #pragma unroll 1
   for (int it = 0; it < iters && !done && !late; ++it) {
@@ -944,6 +1029,8 @@ __device__ __forceinline__ void cg_body(const PersistSolve& a, Shared& sh, int s
       const double pi = p[i];
       c.publish(kn, i, pi);
       c.t(i) = ti;
+      if constexpr (!CL)
+        if (two) a.t[r0 + i] = ti;
       d1[0] += pi * ti;
     });
     if (!c.template sum<1>(0, d1)) {
@@ -958,6 +1045,13 @@ __device__ __forceinline__ void cg_body(const PersistSolve& a, Shared& sh, int s
     const double alpha = rho / d1[0];
     double d2[2] = {0.0, 0.0};
     const double* pn = c.vec(kn);
+    if constexpr (!CL) {  // the aggregates' sums of the new r, as in BiCGStab
+      if (two) {
+        const double* gr = c.global(1);
+        c.template restrict_rows<1>([&](int i, double (&s)[1]) { s[0] = __ldcg(gr + i) - alpha * __ldcg(a.t + i); });
+      }
+      c.par ^= 1;
+    }
 #pragma unroll 1
     for (int i = threadIdx.x; i < nr; i += kThreads) {
       c.x(i) += alpha * pn[i];
@@ -975,7 +1069,7 @@ __device__ __forceinline__ void cg_body(const PersistSolve& a, Shared& sh, int s
     const bool conv = within(rr, limit);
     double rho_new = d2[1];
     if (two && isfinite(rr) && !conv) {
-      rho_new = coarse(rho_new);
+      rho_new = coarse(rho_new, !CL);
       if (late) break;
     }
     beta = rho_new / rho;
@@ -995,9 +1089,9 @@ __device__ __forceinline__ void cg_body(const PersistSolve& a, Shared& sh, int s
   }
   for (int i = threadIdx.x; i < nr; i += kThreads) {
     a.x[r0 + i] = c.x(i);
-    if constexpr (CL) {
-      if (!done) {
-        a.r[r0 + i] = c.r(i);
+    if (!done) {
+      a.r[r0 + i] = c.r(i);
+      if constexpr (CL) {
         a.q[r0 + i] = c.q(i);
         a.v[r0 + i] = c.v(i);
       }

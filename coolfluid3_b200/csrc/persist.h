@@ -35,6 +35,9 @@ struct PersistSolve {
   // grid form.  BiCGStab: residual, shadow residual, q = p - omega v, v; CG:
   // residual, -, the direction's two buffers.
   double *r = nullptr, *rh = nullptr, *q = nullptr, *v = nullptr;
+  // Grid form, two-level: second copies of r and (BiCGStab) q, and A p or A sh, which
+  // the restrictions read; point Jacobi: r, q and null.
+  double *r2 = nullptr, *q2 = nullptr, *t = nullptr;
   // coarse space of the two-level preconditioners (nc = 0: point Jacobi, or
   // nothing where jacobi is false)
   bool jacobi = true;
@@ -43,7 +46,7 @@ struct PersistSolve {
   const int32_t* agg_ptr = nullptr;
   const int32_t* agg_rows = nullptr;
   const double* ainv = nullptr;
-  double* cvec = nullptr;
+  double* cvec = nullptr;  // 2 * nc
   double* yvec = nullptr;  // 2 * nc: the corrections of the two products of an iteration
   double* part = nullptr;  // kPersistPartials block partials (grid form)
   double* dctl = nullptr;
