@@ -62,12 +62,14 @@ struct ufem_nssi_handle {
   int nbox = 0;
   bool coarse_ready = false;
   bool coarse_ok = false;
+  int widest = 0;  // most neighbours of a node (0: not counted yet)
 };
 
 namespace ufem {
 namespace {
 
 constexpr int kSIThreads = 128;
+constexpr int kSILanes = 8;  // lanes of a node in the velocity matrix kernel
 
 // Inputs every element routine reads.
 struct SIArgs {
@@ -170,20 +172,29 @@ __device__ __forceinline__ constexpr int n_gauss2() { return D == 2 ? 3 : 4; }
 // Velocity matrix T + theta dt M (VelocityAssembly, MatrixAssembly.hpp:52-149):
 // T the consistent mass (order-2 rule) on the diagonal component blocks,
 // M = nu_c grad N^T grad N (diagonal blocks) + tau_bulk dN/dx_i^T dN/dx_j (all
-// blocks) at the centroid; tau from u_adv.  One thread per node writes its
-// dim rows (zeroed first; ZeroLSS).
+// blocks) at the centroid; tau from u_adv.
+//
+// Eight lanes per node, an element each, add to the node's dim rows in shared memory
+// one lane after another, in the order of the elements (the sums are one thread's).
+// A thread per node that added in global memory was bound by its stores: D^2 (D + 1)
+// of them an element, each a write to L2.  32^3 x 6 tetrahedra: 253 -> 109 us.
 template <int D>
 __global__ void __launch_bounds__(kSIThreads) si_velocity_matrix_kernel(SIArgs A, const int64_t* __restrict__ rowptr,
-                                                                        double* __restrict__ vals) {
+                                                                        double* __restrict__ vals, int widest) {
   constexpr int n = D + 1;
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= A.N) return;
+  extern __shared__ double si_rows[];  // kSIThreads / kSILanes nodes x widest row block
+  const int64_t i = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) / kSILanes;
+  const int sub = threadIdx.x % kSILanes;
+  const unsigned lanes = 0xffu << (threadIdx.x & 24);  // the node's lanes
+  if (i >= A.N) return;                                // all of them
   const KParams<double> kp = make_kparams<double>(A.p);
-  const int64_t S = A.start[i + 1] - A.start[i];
-  const int64_t r0 = rowptr[i * D];
-  for (int64_t q = r0; q < r0 + int64_t(D) * D * S; ++q) vals[q] = 0.0;
+  const int S = int(A.start[i + 1] - A.start[i]);
+  double* rows = si_rows + int(threadIdx.x / kSILanes) * widest * (D * D);
+  for (int q = sub; q < D * D * S; q += kSILanes) rows[q] = 0.0;
   const double thdt = kp.theta * kp.dt;
-  for (int32_t p = A.row_inc[i]; p < A.row_inc[i + 1]; ++p) {
+  const int32_t p1 = A.row_inc[i + 1];
+  for (int32_t p0 = A.row_inc[i]; p0 < p1; p0 += kSILanes) {
+    const int32_t p = min(p0 + sub, p1 - 1);  // (the lanes past the last element add nothing)
     const int64_t e = A.inc_elem[p];
     const uint32_t info = A.inc_info[p];
     const int a = int(info >> 24);
@@ -207,27 +218,35 @@ __global__ void __launch_bounds__(kSIThreads) si_velocity_matrix_kernel(SIArgs A
 #pragma unroll
     for (int k = 0; k < D; ++k) Ga[k] = sel<n>(g.G[k], a);
     const double lapc = w1 * g.nu_c, bulkc = w1 * g.tbu;
+    for (int turn = 0; turn < min(kSILanes, p1 - p0); ++turn) {
+      __syncwarp(lanes);
+      if (turn == sub) {
 #pragma unroll
-    for (int b = 0; b < n; ++b) {
-      const int slot = int((info >> (6 * b)) & 63u);
-      double dot = 0.0;
+        for (int b = 0; b < n; ++b) {
+          const int slot = int((info >> (6 * b)) & 63u);
+          double dot = 0.0;
 #pragma unroll
-      for (int k = 0; k < D; ++k) dot += Ga[k] * g.G[k][b];
-      const double lap = lapc * dot;
+          for (int k = 0; k < D; ++k) dot += Ga[k] * g.G[k][b];
+          const double lap = lapc * dot;
 #pragma unroll
-      for (int r = 0; r < D; ++r) {
-        const double br = bulkc * Ga[r];
-        double* row = vals + r0 + int64_t(r) * D * S + int64_t(slot) * D;
+          for (int r = 0; r < D; ++r) {
+            const double br = bulkc * Ga[r];
+            double* row = rows + (r * S + slot) * D;
 #pragma unroll
-        for (int c = 0; c < D; ++c) {
-          const double bulk = br * g.G[c][b];
-          const double M = (r == c) ? lap + bulk : bulk;
-          const double T = (r == c) ? Tm[b] : 0.0;
-          row[c] += T + thdt * M;
+            for (int c = 0; c < D; ++c) {
+              const double bulk = br * g.G[c][b];
+              const double M = (r == c) ? lap + bulk : bulk;
+              const double T = (r == c) ? Tm[b] : 0.0;
+              row[c] += T + thdt * M;
+            }
+          }
         }
       }
     }
   }
+  __syncwarp(lanes);
+  const int64_t r0 = rowptr[i * D];
+  for (int q = sub; q < D * D * S; q += kSILanes) vals[r0 + q] = rows[q];
 }
 
 // Pressure matrix theta (tau_ps + dt) grad N^T grad N (PressureSystem.cpp:110-140),
@@ -741,8 +760,17 @@ int zero_bc_dofs(ufem_ns_handle* sys, double* v, cudaStream_t s) {
 
 template <int D>
 int launch_velocity_matrix(ufem_nssi_handle* h, cudaStream_t s) {
-  si_velocity_matrix_kernel<D><<<si_blocks(h->base->N), kSIThreads, 0, s>>>(make_args(h->base), h->us->d_rowptr,
-                                                                            h->us->d_vals);
+  // the rows of a block's nodes in shared memory: up to 72 KB (slots have six bits).
+  // Always that limit, not this handle's size: other handles launch from other threads.
+  const std::vector<int64_t>& start = h->base->start_h;
+  if (h->widest == 0)
+    for (size_t i = 0; i + 1 < start.size(); ++i) h->widest = std::max(h->widest, int(start[i + 1] - start[i]));
+  const size_t smem = size_t(kSIThreads / kSILanes) * h->widest * D * D * sizeof(double);
+  if (smem > 48 * 1024)
+    UFEM_CUDA_TRY(cudaFuncSetAttribute(si_velocity_matrix_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       int(kSIThreads / kSILanes * 64 * D * D * sizeof(double))));
+  si_velocity_matrix_kernel<D><<<si_blocks(h->base->N * kSILanes), kSIThreads, smem, s>>>(
+      make_args(h->base), h->us->d_rowptr, h->us->d_vals, h->widest);
   UFEM_CUDA_TRY(cudaGetLastError());
   return identity_rows(h->us, s);
 }

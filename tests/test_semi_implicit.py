@@ -401,3 +401,36 @@ def test_two_level_pressure_preconditioner():
         for k in range(3):
             G.add_velocity_dirichlet(walls, k, 0.0)
         G.step(1)
+
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("spokes", [6, 30, 61])
+def test_velocity_matrix_of_a_node_with_many_neighbours(dim, spokes):
+    """Elements around one node (2D) or one edge (3D): rows of one to eight turns of
+    eight lanes, up to the 63 neighbours a row's slots have room for."""
+    ang = 2 * np.pi * np.arange(spokes) / spokes
+    ring = np.c_[np.cos(ang), np.sin(ang)]
+    k = np.arange(spokes)
+    if dim == 2:
+        c = np.vstack([[[0.0, 0.0]], ring])
+        t = np.c_[0 * k, 1 + k, 1 + (k + 1) % spokes]
+    else:
+        c = np.vstack([[[0.0, 0.0, -0.5], [0.0, 0.0, 0.5]], np.c_[ring, 0.1 * np.sin(3 * ang)]])
+        t = np.c_[0 * k, 0 * k + 1, 2 + k, 2 + (k + 1) % spokes]
+    t = np.ascontiguousarray(t, dtype=np.uint32)
+    N = len(c)
+    rng = np.random.default_rng(3)
+    nu = 0.01 * (1.0 + 0.5 * rng.random(N))
+    up = rng.standard_normal((N, dim + 1))
+    lin = np.tile(up[:, :dim], (1, 4)) + 0.05 * rng.standard_normal((N, 4 * dim))
+    G, S = _pair(c, t, dim)
+    with G:
+        for X in (G, S):
+            X.initial_conditions(up[:, :dim].copy(), nu, up[:, dim].copy())
+            X.set_state(up, lin, nu)
+        G.assemble_velocity_matrix()
+        rp, ci, uv, _, _ = G.system("velocity")
+        assert np.diff(rp).max() == dim * (spokes + dim - 1)
+        assert row_scaled_error(uv, S.velocity_matrix(), rp) <= 1e-12
