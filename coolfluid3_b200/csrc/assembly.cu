@@ -19,6 +19,7 @@
 #include <type_traits>
 
 #include "internal.h"
+#include "dirichlet.cuh"
 #include "element.cuh"
 
 namespace ufem {
@@ -1133,93 +1134,30 @@ __global__ void build_csr_kernel(int64_t N, int neq, const int64_t* __restrict__
   if (i == N - 1) rowptr[N * neq] = int64_t(neq) * neq * start[N];
 }
 
-// Symmetric Dirichlet, part 1: per-step values v = value - old for the first
-// and last application of every constrained dof.
-__global__ void dirichlet_values_kernel(int64_t nbc, int neq, const int64_t* __restrict__ bc_dof,
-                                        const double* __restrict__ first, const double* __restrict__ state,
-                                        double* __restrict__ vfirst) {
-  const int64_t u = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (u >= nbc) return;
-  const int64_t dof = bc_dof[u];
-  const int64_t node = dof / neq;
-  const int comp = int(dof - node * neq);
-  vfirst[u] = __dsub_rn(first[u], state[4 * node + comp]);
-}
-
-// Part 2: rows that are not constrained move their constrained columns to the
-// RHS in first-application order (the order of the sequential reference).
-// Eight lanes per row, four rows per warp: the lanes load eight of the row's
-// constrained entries at a time, the terms are added to the RHS one by one in
-// first-application order (the rounding of the sequential form: no FMA, no
-// reassociation), then the lanes zero the entries.
-__global__ void dirichlet_columns_kernel(int64_t nrows, const int64_t* __restrict__ fix_row,
-                                         const int64_t* __restrict__ fix_ptr, const int64_t* __restrict__ fix_pos,
-                                         const int32_t* __restrict__ fix_bc, const double* __restrict__ vfirst,
-                                         double* __restrict__ vals, float* __restrict__ vals32,
-                                         double* __restrict__ rhs) {
-  constexpr unsigned FULL = 0xffffffffu;
-  const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if ((t >> 5) * 4 >= nrows) return;  // whole warp
-  const int64_t q = t >> 3;
-  const int sub = int(t & 7), gbase = int(threadIdx.x & 31) & ~7;
-  const bool valid = q < nrows;
-  int64_t row = 0, k0 = 0;
-  int len = 0;
-  double r = 0.0;
-  if (valid) {
-    row = fix_row[q];
-    k0 = fix_ptr[q];
-    len = int(fix_ptr[q + 1] - k0);
-    r = rhs[row];
-  }
-  int maxlen = len;  // the warp's longest row: every lane runs the same shuffles
-  maxlen = max(maxlen, __shfl_xor_sync(FULL, maxlen, 8));
-  maxlen = max(maxlen, __shfl_xor_sync(FULL, maxlen, 16));
-  for (int kb = 0; kb < maxlen; kb += 8) {
-    const int n = len - kb;  // this row's terms left
-    double term = 0.0;
-    int64_t pos = -1;
-    if (sub < n) {
-      pos = fix_pos[k0 + kb + sub];
-      term = __dmul_rn(-vals[pos], vfirst[fix_bc[k0 + kb + sub]]);
-    }
-    for (int j = 0; j < 8; ++j) {  // added one by one, in first-application order
-      const double tj = __shfl_sync(FULL, term, gbase + j);
-      if (j < n) r = __dadd_rn(r, tj);
-    }
-    if (sub < n) {
-      vals[pos] = 0.0;
-      if (vals32) vals32[pos] = 0.0f;
-    }
-  }
-  if (valid && sub == 0) rhs[row] = r;
-}
-
-// Part 3: constrained rows become identity rows; rhs = sol = last value - old.
-// Eight lanes per constrained dof: the lanes zero the row (the diagonal entry is
-// written 1 in the same pass, so no ordering between lanes is needed).
-__global__ void dirichlet_rows_kernel(int64_t nbc, int neq, const int64_t* __restrict__ bc_dof,
-                                      const double* __restrict__ last, const int64_t* __restrict__ bc_diag,
-                                      const int64_t* __restrict__ rowptr, const double* __restrict__ state,
-                                      double* __restrict__ vals, float* __restrict__ vals32,
-                                      double* __restrict__ rhs, double* __restrict__ sol) {
-  const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int64_t u = t >> 3;  // eight lanes per constrained dof
-  const int sub = int(t & 7);
-  if (u >= nbc) return;
-  const int64_t dof = bc_dof[u];
-  const int64_t diag = bc_diag[u];
-  for (int64_t p = rowptr[dof] + sub; p < rowptr[dof + 1]; p += 8) {
-    const double v = (p == diag) ? 1.0 : 0.0;
-    vals[p] = v;
-    if (vals32) vals32[p] = float(v);
-  }
-  if (sub == 0) {
-    const int64_t node = dof / neq;
-    const int comp = int(dof - node * neq);
-    const double v = __dsub_rn(last[u], state[4 * node + comp]);
-    rhs[dof] = v;
-    sol[dof] = v;
+// Symmetric Dirichlet: the first column_blocks blocks move the constrained columns
+// of the other rows to the RHS, the rest write the constrained rows, eight lanes
+// per row.  In one launch: on small meshes the pass is bound by launches.  Three
+// launches (values, columns, rows) took 1.7, 2.9 and 2.6 us with the gaps between
+// them; assembly and conditions of 64 x 64 x 2 triangles 24.5 -> 16.3 us, of
+// 17^3 x 6 tetrahedra 36.9 -> 30.4 us.
+__global__ void __launch_bounds__(256) dirichlet_kernel(int column_blocks, DirichletPlan bp,
+                                                        const int64_t* __restrict__ rowptr,
+                                                        const double* __restrict__ state, double* __restrict__ vals,
+                                                        float* __restrict__ vals32, double* __restrict__ rhs,
+                                                        double* __restrict__ sol) {
+  if (int(blockIdx.x) < column_blocks) {
+    const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if ((t >> 5) * 4 >= bp.nfix_rows) return;  // whole warp
+    const int64_t q = t >> 3;
+    const bool valid = q < bp.nfix_rows;
+    const int64_t k0 = valid ? bp.fix_ptr[q] : 0;
+    dirichlet_columns(valid, valid ? bp.fix_row[q] : 0, k0, valid ? int(bp.fix_ptr[q + 1] - k0) : 0, bp.fix_pos,
+                      bp.fix_bc, bp.bc_at, bp.bc_first, state, vals, vals32, rhs);
+  } else {
+    const int64_t u = (int64_t(blockIdx.x - column_blocks) * blockDim.x + threadIdx.x) >> 3;
+    if (u < bp.nbc)
+      dirichlet_row(u, bp.bc_dof, bp.bc_at, bp.bc_first, bp.bc_last, bp.bc_diag, rowptr, state, vals, vals32, rhs, sol,
+                    bp.vfirst);
   }
 }
 
@@ -1684,18 +1622,9 @@ int launch_neumann(ufem_ns_handle* h, cudaStream_t s) {
 int launch_dirichlet(ufem_ns_handle* h, cudaStream_t s) {
   const DirichletPlan& bp = h->bcp;
   if (bp.nbc == 0) return UFEM_OK;
-  dirichlet_values_kernel<<<unsigned((bp.nbc + 255) / 256), 256, 0, s>>>(bp.nbc, h->neq, bp.bc_dof, bp.bc_first,
-                                                                         h->d_state, bp.vfirst);
-  UFEM_CUDA_TRY(cudaGetLastError());
-  if (bp.nfix_rows > 0) {
-    dirichlet_columns_kernel<<<unsigned((bp.nfix_rows * 8 + 255) / 256), 256, 0, s>>>(
-        bp.nfix_rows, bp.fix_row, bp.fix_ptr, bp.fix_pos, bp.fix_bc, bp.vfirst, h->d_vals, h->d_vals32, h->d_rhs);
-    UFEM_CUDA_TRY(cudaGetLastError());
-  }
-  dirichlet_rows_kernel<<<unsigned((bp.nbc * 8 + 255) / 256), 256, 0, s>>>(bp.nbc, h->neq, bp.bc_dof, bp.bc_last,
-                                                                            bp.bc_diag,
-                                                        h->d_rowptr, h->d_state, h->d_vals, h->d_vals32, h->d_rhs,
-                                                        h->d_sol);
+  const int64_t cb = (bp.nfix_rows * 8 + 255) / 256, rb = (bp.nbc * 8 + 255) / 256;
+  dirichlet_kernel<<<unsigned(cb + rb), 256, 0, s>>>(int(cb), bp, h->d_rowptr, h->d_state, h->d_vals, h->d_vals32,
+                                                     h->d_rhs, h->d_sol);
   UFEM_CUDA_TRY(cudaGetLastError());
   return UFEM_OK;
 }

@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "dirichlet.cuh"
 #include "persist.h"
 #include "spmv_node.cuh"
 
@@ -82,6 +83,7 @@ struct BatchMesh {
   double* sol;
   int64_t nbc, nfix_rows;
   const int64_t* bc_dof;
+  const int32_t* bc_at;
   const double* bc_first;
   const double* bc_last;
   const int64_t* bc_diag;
@@ -183,85 +185,29 @@ __global__ void update_batch_kernel(int64_t total, int nmesh, const int64_t* __r
   M.state[4 * i + dim] = __dadd_rn(M.state[4 * i + dim], M.sol[i * neq + dim]);
 }
 
-// Symmetric Dirichlet over all members, the three passes of the one-mesh form.
-__global__ void dirichlet_values_batch_kernel(int64_t total, int nmesh, const int64_t* __restrict__ bc_prefix,
-                                              const BatchMesh* __restrict__ bm) {
-  const int64_t g = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (g >= total) return;
-  const int m = find_mesh(bc_prefix, nmesh, g);
-  const BatchMesh& M = bm[m];
-  const int64_t u = g - bc_prefix[m];
-  const int64_t dof = M.bc_dof[u];
-  const int64_t node = dof / M.neq;
-  const int comp = int(dof - node * M.neq);
-  M.vfirst[u] = __dsub_rn(M.bc_first[u], M.state[4 * node + comp]);
-}
-
-__global__ void dirichlet_columns_batch_kernel(int64_t total, int nmesh, const int64_t* __restrict__ fix_prefix,
-                                               const BatchMesh* __restrict__ bm) {
-  constexpr unsigned FULL = 0xffffffffu;
-  const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;  // 8 lanes per row, as the one-mesh kernel
-  if ((t >> 5) * 4 >= total) return;  // whole warp
-  const int64_t g = t >> 3;
-  const int sub = int(t & 7), gbase = int(threadIdx.x & 31) & ~7;
-  const bool valid = g < total;
-  const int m = valid ? find_mesh(fix_prefix, nmesh, g) : 0;
-  const BatchMesh& M = bm[m];
-  int64_t row = 0, k0 = 0;
-  int len = 0;
-  double r = 0.0;
-  if (valid) {
-    const int64_t q = g - fix_prefix[m];
-    row = M.fix_row[q];
-    k0 = M.fix_ptr[q];
-    len = int(M.fix_ptr[q + 1] - k0);
-    r = M.rhs[row];
-  }
-  int maxlen = len;
-  maxlen = max(maxlen, __shfl_xor_sync(FULL, maxlen, 8));
-  maxlen = max(maxlen, __shfl_xor_sync(FULL, maxlen, 16));
-  for (int kb = 0; kb < maxlen; kb += 8) {
-    const int n = len - kb;
-    double term = 0.0;
-    int64_t pos = -1;
-    if (sub < n) {
-      pos = M.fix_pos[k0 + kb + sub];
-      term = __dmul_rn(-M.vals[pos], M.vfirst[M.fix_bc[k0 + kb + sub]]);
-    }
-    for (int j = 0; j < 8; ++j) {  // first-application order
-      const double tj = __shfl_sync(FULL, term, gbase + j);
-      if (j < n) r = __dadd_rn(r, tj);
-    }
-    if (sub < n) {
-      M.vals[pos] = 0.0;
-      if (M.vals32) M.vals32[pos] = 0.0f;
-    }
-  }
-  if (valid && sub == 0) M.rhs[row] = r;
-}
-
-__global__ void dirichlet_rows_batch_kernel(int64_t total, int nmesh, const int64_t* __restrict__ bc_prefix,
-                                            const BatchMesh* __restrict__ bm) {
-  const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int64_t g = t >> 3;  // eight lanes per constrained dof
-  const int sub = int(t & 7);
-  if (g >= total) return;
-  const int m = find_mesh(bc_prefix, nmesh, g);
-  const BatchMesh& M = bm[m];
-  const int64_t u = g - bc_prefix[m];
-  const int64_t dof = M.bc_dof[u];
-  const int64_t diag = M.bc_diag[u];
-  for (int64_t p = M.rowptr[dof] + sub; p < M.rowptr[dof + 1]; p += 8) {
-    const double v = (p == diag) ? 1.0 : 0.0;
-    M.vals[p] = v;
-    if (M.vals32) M.vals32[p] = float(v);
-  }
-  if (sub == 0) {
-    const int64_t node = dof / M.neq;
-    const int comp = int(dof - node * M.neq);
-    const double v = __dsub_rn(M.bc_last[u], M.state[4 * node + comp]);
-    M.rhs[dof] = v;
-    M.sol[dof] = v;
+// Symmetric Dirichlet over all members, as dirichlet_kernel's one mesh.
+__global__ void __launch_bounds__(256)
+    dirichlet_batch_kernel(int column_blocks, int64_t total_fix, int64_t total_bc, int nmesh,
+                           const int64_t* __restrict__ fix_prefix, const int64_t* __restrict__ bc_prefix,
+                           const BatchMesh* __restrict__ bm) {
+  if (int(blockIdx.x) < column_blocks) {
+    const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if ((t >> 5) * 4 >= total_fix) return;  // whole warp
+    const int64_t g = t >> 3;
+    const bool valid = g < total_fix;
+    const int m = valid ? find_mesh(fix_prefix, nmesh, g) : 0;
+    const BatchMesh& M = bm[m];
+    const int64_t q = valid ? g - fix_prefix[m] : 0;
+    const int64_t k0 = valid ? M.fix_ptr[q] : 0;
+    dirichlet_columns(valid, valid ? M.fix_row[q] : 0, k0, valid ? int(M.fix_ptr[q + 1] - k0) : 0, M.fix_pos, M.fix_bc,
+                      M.bc_at, M.bc_first, M.state, M.vals, M.vals32, M.rhs);
+  } else {
+    const int64_t g = (int64_t(blockIdx.x - column_blocks) * blockDim.x + threadIdx.x) >> 3;
+    if (g >= total_bc) return;
+    const int m = find_mesh(bc_prefix, nmesh, g);
+    const BatchMesh& M = bm[m];
+    dirichlet_row(g - bc_prefix[m], M.bc_dof, M.bc_at, M.bc_first, M.bc_last, M.bc_diag, M.rowptr, M.state, M.vals,
+                  M.vals32, M.rhs, M.sol, M.vfirst);
   }
 }
 
@@ -966,6 +912,7 @@ int batch_refresh(ufem_batch* b) {
     M.nbc = P.nbc;
     M.nfix_rows = P.nfix_rows;
     M.bc_dof = P.bc_dof;
+    M.bc_at = P.bc_at;
     M.bc_first = P.bc_first;
     M.bc_last = P.bc_last;
     M.bc_diag = P.bc_diag;
@@ -1661,13 +1608,9 @@ int ufem_batch_assemble(ufem_batch* b, void* stream) {
     if (h->bcp.nneu > 0 && (rc = launch_neumann(h, st))) return rc;
   }
   if (b->total_bc > 0) {
-    dirichlet_values_batch_kernel<<<blocks_for(b->total_bc, 256), 256, 0, st>>>(b->total_bc, b->nmesh,
-                                                                                 b->d_bc_prefix, b->d_mesh);
-    if (b->total_fix > 0)
-      dirichlet_columns_batch_kernel<<<blocks_for(b->total_fix * 8, 256), 256, 0, st>>>(b->total_fix, b->nmesh,
-                                                                                         b->d_fix_prefix, b->d_mesh);
-    dirichlet_rows_batch_kernel<<<blocks_for(b->total_bc * 8, 256), 256, 0, st>>>(b->total_bc, b->nmesh,
-                                                                                   b->d_bc_prefix, b->d_mesh);
+    const unsigned cb = b->total_fix > 0 ? blocks_for(b->total_fix * 8, 256) : 0;
+    dirichlet_batch_kernel<<<cb + blocks_for(b->total_bc * 8, 256), 256, 0, st>>>(
+        int(cb), b->total_fix, b->total_bc, b->nmesh, b->d_fix_prefix, b->d_bc_prefix, b->d_mesh);
     UFEM_CUDA_TRY(cudaGetLastError());
   }
   return UFEM_OK;

@@ -171,7 +171,7 @@ int check_device() {
 }
 
 void free_bc_plan(DirichletPlan& b) {
-  dfree(b.bc_dof); dfree(b.bc_first); dfree(b.bc_last); dfree(b.bc_diag);
+  dfree(b.bc_dof); dfree(b.bc_at); dfree(b.bc_first); dfree(b.bc_last); dfree(b.bc_diag);
   dfree(b.fix_row); dfree(b.fix_ptr); dfree(b.fix_pos); dfree(b.fix_bc); dfree(b.vfirst);
   dfree(b.neu_dof); dfree(b.neu_ptr); dfree(b.neu_val);
   dfree(b.fn_first); dfree(b.fn_last); dfree(b.fn_code); dfree(b.fn_off); dfree(b.fn_const);
@@ -311,13 +311,17 @@ int build_bc_plan(ufem_ns_handle* h) {
   bp.nbc = int64_t(dofs.size());
   bp.nfix_rows = int64_t(frow.size());
   bp.nfix = int64_t(fixes.size());
-  if ((rc = dmalloc(&bp.bc_dof, dofs.size(), "bc_dof")) || (rc = dmalloc(&bp.bc_first, dofs.size(), "bc_first")) ||
+  if ((rc = dmalloc(&bp.bc_dof, dofs.size(), "bc_dof")) || (rc = dmalloc(&bp.bc_at, dofs.size(), "bc_at")) ||
+      (rc = dmalloc(&bp.bc_first, dofs.size(), "bc_first")) ||
       (rc = dmalloc(&bp.bc_last, dofs.size(), "bc_last")) || (rc = dmalloc(&bp.bc_diag, dofs.size(), "bc_diag")) ||
       (rc = dmalloc(&bp.vfirst, dofs.size(), "vfirst")) || (rc = dmalloc(&bp.fix_row, frow.size(), "fix_row")) ||
       (rc = dmalloc(&bp.fix_ptr, fptr.size(), "fix_ptr")) || (rc = dmalloc(&bp.fix_pos, fpos.size(), "fix_pos")) ||
       (rc = dmalloc(&bp.fix_bc, fbc.size(), "fix_bc")))
     return rc;
   UFEM_CUDA_TRY(cudaMemcpy(bp.bc_dof, dofs.data(), dofs.size() * 8, cudaMemcpyHostToDevice));
+  std::vector<int32_t> at(dofs.size());
+  for (size_t u = 0; u < dofs.size(); ++u) at[u] = int32_t(dofs[u] / h->neq * 4 + dofs[u] % h->neq);
+  UFEM_CUDA_TRY(cudaMemcpy(bp.bc_at, at.data(), at.size() * 4, cudaMemcpyHostToDevice));
   UFEM_CUDA_TRY(cudaMemcpy(bp.bc_first, first.data(), first.size() * 8, cudaMemcpyHostToDevice));
   UFEM_CUDA_TRY(cudaMemcpy(bp.bc_last, last.data(), last.size() * 8, cudaMemcpyHostToDevice));
   UFEM_CUDA_TRY(cudaMemcpy(bp.bc_diag, diag.data(), diag.size() * 8, cudaMemcpyHostToDevice));

@@ -97,6 +97,7 @@ struct DirichletPlan {
   int64_t nfix_rows = 0;       // non-BC rows holding BC columns
   int64_t nfix = 0;            // entries moved to the RHS
   int64_t* bc_dof = nullptr;   // nbc
+  int32_t* bc_at = nullptr;    // nbc: place of the dof in the state records
   double* bc_first = nullptr;  // value of the first application (moves columns)
   double* bc_last = nullptr;   // value of the last application (sets row/rhs/sol)
   int64_t* bc_diag = nullptr;  // CSR position of the diagonal of each BC row
