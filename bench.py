@@ -450,7 +450,7 @@ def run_ours(args, rank, world, local):
                    "assembly_kernel": {"variant": asm_variant, "warps_per_cta": asm_warps,
                                        "autotuned": tuned is not None,
                                        "tuned_ms": None if tuned is None else round(tuned["ms"], 4)}},
-        "gpu_launches": (1 + asm_launches + 3) * args.steps,  # linearize, assembly, 3 Dirichlet kernels
+        "gpu_launches": (1 + asm_launches + 1) * args.steps,  # linearize, assembly, the Dirichlet kernel
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4), "peak_kind": peak_kind,
                      "traffic": traffic_bytes, "algorithmic_bytes": B, "kernel_ms": round(kern_ms, 4)},
