@@ -1817,6 +1817,8 @@ int coupled_coarse_build(ufem_ns_handle* h, int max_side_2d, int max_side_3d) {
   if (!pos.empty()) UFEM_CUDA_TRY(cudaMemcpy(kw.cp_pos, pos.data(), pos.size() * 8, cudaMemcpyHostToDevice));
   UFEM_CUDA_TRY(cudaMemcpy(kw.cp_seg, seg.data(), seg.size() * 4, cudaMemcpyHostToDevice));
   if (!dst.empty()) UFEM_CUDA_TRY(cudaMemcpy(kw.cp_dst, dst.data(), dst.size() * 4, cudaMemcpyHostToDevice));
+  // small copies may return before they land, and the caller's stream does not wait for them
+  UFEM_CUDA_TRY(cudaStreamSynchronize(nullptr));
   kw.cp_nseg = int(dst.size());
   kw.nc = nc;
   return UFEM_OK;
