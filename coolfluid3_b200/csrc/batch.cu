@@ -962,6 +962,7 @@ int batch_refresh(ufem_batch* b) {
   UFEM_CUDA_TRY(cudaMemcpy(b->d_mesh, bm.data(), bm.size() * sizeof(BatchMesh), cudaMemcpyHostToDevice));
   UFEM_CUDA_TRY(cudaMemcpy(b->d_bc_prefix, bcp.data(), bcp.size() * 8, cudaMemcpyHostToDevice));
   UFEM_CUDA_TRY(cudaMemcpy(b->d_fix_prefix, fxp.data(), fxp.size() * 8, cudaMemcpyHostToDevice));
+  UFEM_CUDA_TRY(uploads_landed());
   b->active_dirty = false;
   return UFEM_OK;
 }

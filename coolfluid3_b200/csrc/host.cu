@@ -254,7 +254,10 @@ int build_bc_plan(ufem_ns_handle* h) {
   ++bp.version;
   int rc;
   if ((rc = build_neumann_plan(h))) return rc;
-  if (h->bcs.empty()) return UFEM_OK;
+  if (h->bcs.empty()) {
+    if (bp.nneu > 0) UFEM_CUDA_TRY(uploads_landed());
+    return UFEM_OK;
+  }
   const int neq = h->neq;
   std::vector<int32_t> uid(size_t(h->nrows), -1);
   std::vector<int64_t> dofs;
@@ -351,6 +354,7 @@ int build_bc_plan(ufem_ns_handle* h) {
     UFEM_CUDA_TRY(cudaMemcpy(bp.fix_pos, fpos.data(), fpos.size() * 8, cudaMemcpyHostToDevice));
     UFEM_CUDA_TRY(cudaMemcpy(bp.fix_bc, fbc.data(), fbc.size() * 4, cudaMemcpyHostToDevice));
   }
+  UFEM_CUDA_TRY(uploads_landed());
   return UFEM_OK;
 }
 
@@ -1042,6 +1046,7 @@ int ufem_ns_get_state(ufem_ns_handle* h, double* up, double* lin) {
 int ufem_ns_set_solution(ufem_ns_handle* h, const double* sol) {
   if (!h || !sol) return set_error(UFEM_ERR_ARG, "NULL argument");
   UFEM_CUDA_TRY(cudaMemcpy(h->d_sol, sol, size_t(h->nrows) * 8, cudaMemcpyHostToDevice));
+  UFEM_CUDA_TRY(uploads_landed());
   return UFEM_OK;
 }
 

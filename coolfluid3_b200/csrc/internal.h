@@ -35,6 +35,11 @@ using DeviceLock = std::lock_guard<std::recursive_mutex>;
       return ::ufem::set_error(UFEM_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(_e)); \
   } while (0)
 
+// Waits for the legacy stream.  A call that copies to the device with cudaMemcpy (from
+// pageable memory: small copies may return before they land) or zeroes with cudaMemset
+// ends with this, since the streams that callers pass do not wait for the legacy one.
+inline cudaError_t uploads_landed() { return cudaStreamSynchronize(nullptr); }
+
 // Scalar parameters of the element expression, passed to kernels by value.
 struct NSParams {
   double theta, inv_theta, dt, invdt, rho, inv_rho;

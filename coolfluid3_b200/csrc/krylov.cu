@@ -1092,6 +1092,7 @@ int ensure_work(ufem_ns_handle* h, int m, bool need32, bool bicg) {
   if (!kw.cg_counter) {
     if ((rc = dalloc(&kw.cg_counter, 1))) return rc;
     UFEM_CUDA_TRY(cudaMemset(kw.cg_counter, 0, sizeof(int)));
+    UFEM_CUDA_TRY(uploads_landed());
   }
   if ((rc = dalloc(&kw.w, nd)) || (rc = dalloc(&kw.z, nd)) || (rc = dalloc(&kw.t, nd)) || (rc = dalloc(&kw.r, nd)) ||
       (rc = dalloc(&kw.dinv, ndinv)) || (rc = dalloc(&kw.part, npart)) ||
@@ -1817,8 +1818,7 @@ int coupled_coarse_build(ufem_ns_handle* h, int max_side_2d, int max_side_3d) {
   if (!pos.empty()) UFEM_CUDA_TRY(cudaMemcpy(kw.cp_pos, pos.data(), pos.size() * 8, cudaMemcpyHostToDevice));
   UFEM_CUDA_TRY(cudaMemcpy(kw.cp_seg, seg.data(), seg.size() * 4, cudaMemcpyHostToDevice));
   if (!dst.empty()) UFEM_CUDA_TRY(cudaMemcpy(kw.cp_dst, dst.data(), dst.size() * 4, cudaMemcpyHostToDevice));
-  // small copies may return before they land, and the caller's stream does not wait for them
-  UFEM_CUDA_TRY(cudaStreamSynchronize(nullptr));
+  UFEM_CUDA_TRY(uploads_landed());
   kw.cp_nseg = int(dst.size());
   kw.nc = nc;
   return UFEM_OK;
@@ -2110,6 +2110,7 @@ int krylov_set_coarse(ufem_ns_handle* h, const std::vector<int32_t>& agg, int nc
   UFEM_CUDA_TRY(cudaMemcpy(kw.agg, agg.data(), agg.size() * 4, cudaMemcpyHostToDevice));
   UFEM_CUDA_TRY(cudaMemcpy(kw.agg_ptr, ptr.data(), ptr.size() * 4, cudaMemcpyHostToDevice));
   if (!rows.empty()) UFEM_CUDA_TRY(cudaMemcpy(kw.agg_rows, rows.data(), rows.size() * 4, cudaMemcpyHostToDevice));
+  UFEM_CUDA_TRY(uploads_landed());
   kw.nc = nc;
   return UFEM_OK;
 }

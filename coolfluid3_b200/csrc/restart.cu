@@ -214,6 +214,7 @@ int ufem_ns_read_restart(ufem_ns_handle* h, const char* path, double* current_ti
     UFEM_CUDA_TRY(cudaMemset(h->d_sol, 0, size_t(h->nrows) * 8));
   else if (h->d_sol)
     UFEM_CUDA_TRY(cudaMemcpy(h->d_sol, sol.data(), size_t(h->nrows) * 8, cudaMemcpyHostToDevice));
+  UFEM_CUDA_TRY(uploads_landed());
   h->time = std::strtod(attr(restart, "current_time").c_str(), nullptr);  // Time::current_time
   if (current_time) *current_time = h->time;
   if (time_step) *time_step = std::strtod(attr(restart, "time_step").c_str(), nullptr);

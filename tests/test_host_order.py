@@ -1,0 +1,97 @@
+"""What the library's host code asks of the device and in which order, on the CPU: each
+test runs in a child process whose CUDA runtime is tests/fake_cudart.cpp."""
+import os
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+
+
+@pytest.fixture(scope="session")
+def runtime(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("fake") / "fake_cudart.so")
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", os.path.join(cuda, "include"), "-I",
+                    os.path.join(ROOT, "coolfluid3_b200", "csrc"), os.path.join(HERE, "fake_cudart.cpp"), "-o", so],
+                   check=True)
+    return so
+
+
+PREAMBLE = """
+import ctypes, sys
+import numpy as np
+from coolfluid3_b200 import Batch, NavierStokes, NavierStokesSemiImplicit, UfemError
+from coolfluid3_b200 import problems as P
+fake = ctypes.CDLL(sys.argv[1])
+STREAM = 4096  # any stream but the legacy one
+
+def solver(dim, n, **kw):
+    pb = P.make_problem(dim, n)
+    ns = NavierStokes(pb.coords, pb.conn, dt=pb.dt, use_specializations=False, **kw)
+    ns.set_state(pb.up, pb.lin, pb.nu)
+    ns.add_dirichlet(pb.bc_nodes, pb.bc_comps, pb.bc_values)
+    return ns, pb
+
+def check(what):
+    assert fake.fake_faults() == 0, what + ": a stream was given work beside an upload in flight"
+    assert fake.fake_pending() == 0, what + ": returned with an upload in flight"
+"""
+
+
+def run(runtime, body):
+    env = dict(os.environ, LD_PRELOAD=runtime, PYTHONPATH=ROOT)
+    p = subprocess.run([sys.executable, "-c", PREAMBLE + textwrap.dedent(body), runtime], env=env, cwd=ROOT,
+                       capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stdout + p.stderr
+
+
+def test_uploads_land_before_other_streams_read_them(runtime, tmp_path):
+    """The static lists, condition plans, batch tables, coarse spaces and solutions that
+    calls upload: nothing of them is in flight when another stream is given work or
+    the call returns."""
+    run(runtime, f"""
+    ns, pb = solver(2, 12)
+    check("create")
+    ns.add_dirichlet_function(pb.bc_nodes[:3], 0, "x*t")
+    ns.add_neumann(pb.conn[:1, :2].astype(np.uint32), 2, 0.5)
+    ns.assemble(STREAM)
+    ns.apply_dirichlet(STREAM)
+    check("conditions")
+    for kr in (dict(precond="jacobi"), dict(precond="two_level_coupled"), dict(method="gmres", precond="jacobi")):
+        ns.prepare_solve(**kr)
+        check("prepare_solve")
+        ns.solve(STREAM, raise_on_failure=False, max_iters=4, **kr)
+        check("solve")
+    ns.set_solution(np.ones(ns.nb_rows))
+    check("set_solution")
+    ns.write_restart(r"{tmp_path}/r.cfg", time_step=0.1)
+    ns.read_restart(r"{tmp_path}/r.cfg")
+    check("read_restart")
+
+    members = [solver(2, n)[0] for n in (6, 9)]
+    b = Batch(members)
+    check("batch")
+    for pre in ("jacobi", "two_level_coupled"):
+        b.assemble(STREAM)
+        check("batch assemble")
+        b.solve(STREAM, precond=pre, max_iters=4)
+        check("batch solve")
+    b.set_active([True, False])
+    b.assemble(STREAM)
+    check("batch with a held member")
+
+    for dim, n in ((2, 20), (3, 8)):
+        pb = P.make_problem(dim, n)
+        si = NavierStokesSemiImplicit(pb.coords, pb.conn, dt=pb.dt, theta=0.5)
+        check("semi-implicit create")
+        si.initial_conditions(pb.up[:, :dim], 1e-2)
+        si.add_velocity_dirichlet(pb.bc_nodes[:4], 0, np.zeros(4))
+        si.add_pressure_dirichlet(np.array([0]), np.zeros(1))
+        check("semi-implicit conditions")
+        si.step(2, stream=STREAM)
+        check("semi-implicit step")
+    """)
