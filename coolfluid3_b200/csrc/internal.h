@@ -208,6 +208,7 @@ struct ufem_ns_handle {
   ufem::DirichletPlan bcp;
   ufem::StagePipe pipe;
   ufem::KrylovWork* kw = nullptr;
+  int persist_polls = -1;               // limit of a one-launch solve's barriers (below 0: kPersistPolls)
   bool vals32_valid = false;            // d_vals32 holds the current system (written by the assembly)
 
   // transfer staging (reference field layouts <-> padded node records)

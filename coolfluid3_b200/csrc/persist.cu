@@ -39,7 +39,8 @@
 //
 // All sums run in fixed orders, so a solve is deterministic; FP64 throughout,
 // FP32 only in the stored values of the mixed forms.  Grid barriers wait a
-// bounded time: one that runs out sets a flag the host turns into an error.
+// bounded time: one that runs out sets a flag that ends this launch and those
+// queued after it, and that the host turns into an error.
 #include "persist.h"
 
 #include <algorithm>
@@ -55,7 +56,6 @@ constexpr int kThreads = 512;  // one block an SM: 128 registers a thread
 constexpr int kWarps = kThreads / 32;
 constexpr int kClusterMax = 16;  // the non-portable cluster size
 constexpr unsigned FULL = 0xffffffffu;
-constexpr int kSpinLimit = 1 << 23;  // polls of one barrier (seconds) before giving up
 
 extern __shared__ __align__(16) unsigned char g_smem[];
 
@@ -232,7 +232,7 @@ struct Ctx {
           const int target = epoch * blocks;
           int spins = 0, late = 0;
           while (ld_acquire(a.ictl + kFlagBarrier) < target)
-            if (++spins > kSpinLimit) {
+            if (++spins > a.polls) {
               late = 1;
               break;
             }
@@ -766,7 +766,7 @@ __device__ __forceinline__ bool within(double rr, double limit) {
 template <int NEQ, typename MT, bool CL>
 __device__ __forceinline__ void bicgstab_body(const PersistSolve& a, Shared& sh, int smem_bytes, int rank, int blocks,
                                               bool first, int iters) {
-  if (!first && a.ictl[0]) return;  // every block of the solve reads the same flag
+  if (!first && (a.ictl[0] || a.ictl[kFlagLate])) return;  // every block of the solve reads the same flags
   Ctx<NEQ, MT, CL> c{a, sh, rank, blocks};
   setup(c, smem_bytes);
   const int nr = c.rows(), r0 = c.n0 * NEQ;
@@ -953,10 +953,10 @@ __device__ __forceinline__ void bicgstab_body(const PersistSolve& a, Shared& sh,
     a.dctl[kEst] = sqrt(rr);
     a.dctl[kRho] = rho;
     a.dctl[kHnext] = beta;
-    if (done) a.dctl[kTrue] = sqrt(tr);
+    if (done && !late) a.dctl[kTrue] = sqrt(tr);
     a.ictl[2] = status;
     a.ictl[3] = count;
-    a.ictl[0] = done;
+    a.ictl[0] = done && !late;
   }
   if (late && threadIdx.x == 0) a.ictl[kFlagLate] = 1;
   if constexpr (CL) cluster_sync();  // no block leaves while another may read its shared memory
@@ -965,7 +965,7 @@ __device__ __forceinline__ void bicgstab_body(const PersistSolve& a, Shared& sh,
 template <int NEQ, typename MT, bool CL>
 __device__ __forceinline__ void cg_body(const PersistSolve& a, Shared& sh, int smem_bytes, int rank, int blocks,
                                         bool first, int iters) {
-  if (!first && a.ictl[0]) return;
+  if (!first && (a.ictl[0] || a.ictl[kFlagLate])) return;
   Ctx<NEQ, MT, CL> c{a, sh, rank, blocks};
   setup(c, smem_bytes);
   const int nr = c.rows(), r0 = c.n0 * NEQ;
@@ -1103,10 +1103,10 @@ __device__ __forceinline__ void cg_body(const PersistSolve& a, Shared& sh, int s
     a.dctl[kEst] = sqrt(rr);
     a.dctl[kRho] = rho;
     a.dctl[kOmega] = beta;
-    if (done) a.dctl[kTrue] = sqrt(tr);
+    if (done && !late) a.dctl[kTrue] = sqrt(tr);
     a.ictl[2] = status;
     a.ictl[3] = count;
-    a.ictl[0] = done;
+    a.ictl[0] = done && !late;
   }
   if (late && threadIdx.x == 0) a.ictl[kFlagLate] = 1;
   if constexpr (CL) cluster_sync();
@@ -1145,10 +1145,10 @@ int launch(const PersistSolve& a, const PersistPlan& plan, bool first, int iters
   UFEM_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemMax)));
   if (CL) {
     UFEM_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    if (first) UFEM_CUDA_TRY(cudaMemsetAsync(a.ictl + kFlagLate, 0, sizeof(int), s));
-  } else {
-    UFEM_CUDA_TRY(cudaMemsetAsync(a.ictl + kFlagLate, 0, 2 * sizeof(int), s));
   }
+  // the barrier counter of every launch; a late barrier stays on record to the solve's end
+  if (first) UFEM_CUDA_TRY(cudaMemsetAsync(a.ictl + kFlagLate, 0, 2 * sizeof(int), s));
+  else if (!CL) UFEM_CUDA_TRY(cudaMemsetAsync(a.ictl + kFlagBarrier, 0, sizeof(int), s));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(unsigned(plan.blocks));
   cfg.blockDim = dim3(kThreads);

@@ -19,6 +19,7 @@ constexpr int kFlagLate = 4, kFlagBarrier = 5;
 constexpr int kPersistMaxBlocks = 148;
 constexpr int kPersistSlots = 8;
 constexpr int kPersistPartials = kPersistSlots * kPersistMaxBlocks;
+constexpr int kPersistPolls = 1 << 23;  // polls of a grid barrier (seconds) before it gives up
 // One solve of A x = b on a node graph (the point-CSR values of the assembled
 // system); every vector has N * neq entries.
 struct PersistSolve {
@@ -53,6 +54,7 @@ struct PersistSolve {
   int* ictl = nullptr;
   double tol = 0.0, alpha_max = 0.0;
   int maxit = 0;
+  int polls = kPersistPolls;
 };
 
 // Launch plan of a system: the form, its blocks and their shared memory.

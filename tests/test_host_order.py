@@ -95,3 +95,26 @@ def test_uploads_land_before_other_streams_read_them(runtime, tmp_path):
         si.step(2, stream=STREAM)
         check("semi-implicit step")
     """)
+
+
+def test_a_late_barrier_of_any_launch_is_an_error(runtime):
+    """A solve expected to take 600 iterations queues three launches (80 x 80 cells: the
+    grid form) before the host looks: a barrier that ran out of time in the first, a
+    middle or the last of them is an error, and the solve after it starts afresh."""
+    run(runtime, """
+    ns, pb = solver(2, 80)
+    ns.assemble(STREAM)
+    ns.apply_dirichlet(STREAM)
+    kr = dict(precond="jacobi", max_iters=3000)
+    for late in (0, 1, 2):
+        fake.fake_solves(600, -1)
+        assert ns.solve(STREAM, **kr)["iterations"] == 600
+        fake.fake_solves(600, late)
+        try:
+            ns.solve(STREAM, **kr)
+        except UfemError as e:
+            assert "barrier" in str(e)
+        else:
+            raise AssertionError(f"launch {late} was late and the solve succeeded")
+        assert fake.fake_launches() == 3
+    """)
