@@ -1087,7 +1087,7 @@ int ensure_work(ufem_ns_handle* h, int m, bool need32, bool bicg) {
   const int M = kw.m;
   const size_t nd = size_t(n);
   const size_t ndinv = size_t(h->N) * h->neq * h->neq;
-  const size_t npart = std::max(size_t(M + 2) * kw.nblk, size_t(2) * kCGMaxBlocks);
+  const size_t npart = std::max({size_t(M + 2) * kw.nblk, size_t(2) * kCGMaxBlocks, size_t(kPersistPartials)});
   int rc;
   if (!kw.cg_counter) {
     if ((rc = dalloc(&kw.cg_counter, 1))) return rc;
@@ -2175,12 +2175,13 @@ void krylov_free(ufem_ns_handle* h) {
 // Allocation-free solve.  Its Krylov vectors, block partials and scalars live
 // in one fixed array of this file instead of memory obtained from cudaMalloc.
 // Layout (doubles): 9 vectors of UFEM_NOALLOC_MAX_ROWS (r, r^, p, v, s, t, p^,
-// s^, inverse diagonal), 2 * kMaxPartials partials, 16 scalars, 8 for the
-// integer flags.
+// s^, inverse diagonal), 2 * kMaxPartials partials (a one-launch solve's
+// kPersistPartials among them), 16 scalars, 8 for the integer flags.
 // ---------------------------------------------------------------------------
 constexpr int64_t kNoAllocRows = UFEM_NOALLOC_MAX_ROWS;
 constexpr int kMaxPartials = kRedBlocksMax;  // the largest block count red_blocks gives
 constexpr int64_t kNoAllocDoubles = 9 * kNoAllocRows + 2 * kMaxPartials + 16 + 8;
+static_assert(2 * kMaxPartials >= kPersistPartials, "the partials of a one-launch solve have the same place");
 
 static __device__ __align__(256) double g_noalloc_scratch[kNoAllocDoubles];
 
