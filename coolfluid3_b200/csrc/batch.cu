@@ -836,11 +836,8 @@ struct ufem_batch {
   cudaGraphExec_t block_exec[3] = {nullptr, nullptr, nullptr};
   cudaStream_t capture_stream = nullptr;
   int block_pkind[3] = {-1, -1, -1};
-  // One-cluster solves of the members that fit one (persist.cu): their plans per
-  // operator type, with the coarse sizes they were made for, the device list of
+  // One-cluster solves of the members that fit one (persist.cu): the device list of
   // solves, and the solves' scalars and flags (16 and 8 a member).
-  std::vector<PersistPlan> plan[2];
-  std::vector<int> plan_nc[2];
   PersistSolve* d_solves = nullptr;
   double* p_dctl = nullptr;
   int* p_ictl = nullptr;
@@ -1049,10 +1046,6 @@ int solve_in_clusters(ufem_batch* b, int pkind, double tol, int maxit, double* x
                       std::vector<int>& solved, cudaStream_t st) {
   constexpr bool f32 = std::is_same<MT, float>::value;
   const int n = b->nmesh;
-  std::vector<PersistPlan>& plan = b->plan[f32];
-  std::vector<int>& plan_nc = b->plan_nc[f32];
-  plan.resize(size_t(n));
-  plan_nc.resize(size_t(n), -1);
   std::vector<PersistSolve> list;
   std::vector<int64_t> off(size_t(n) + 1, 0);
   for (int m = 0; m < n; ++m) off[size_t(m) + 1] = off[size_t(m)] + b->members[m]->nrows;
@@ -1069,13 +1062,10 @@ int solve_in_clusters(ufem_batch* b, int pkind, double tol, int maxit, double* x
     Group g{blocks, int(list.size()), 0, 0};
     for (int m = 0; m < n; ++m) {
       if (!todo[m]) continue;
-      const ufem_ns_handle* h = b->members[m];
+      ufem_ns_handle* h = b->members[m];
       const CoarseView cv = pkind == 4 && m < int(b->coarse.size()) ? b->coarse[m] : CoarseView{};
-      if (plan_nc[m] != cv.nc) {
-        plan[m] = persist_plan(h->start_h.data(), h->adj_h.data(), h->N, h->neq, f32, cv.nc);
-        plan_nc[m] = cv.nc;
-      }
-      if (plan[m].form != kPersistCluster || plan[m].blocks != blocks) continue;
+      const PersistPlan& plan = persist_plan_of(h, f32, cv.nc);
+      if (plan.form != kPersistCluster || plan.blocks != blocks) continue;
       PersistSolve a;
       a.N = h->N;
       a.neq = h->neq;
@@ -1103,7 +1093,7 @@ int solve_in_clusters(ufem_batch* b, int pkind, double tol, int maxit, double* x
       a.maxit = maxit;
       list.push_back(a);
       ++g.count;
-      g.smem = std::max(g.smem, plan[m].smem);
+      g.smem = std::max(g.smem, plan.smem);
       solved[m] = 1;
     }
     if (g.count > 0) groups.push_back(g);

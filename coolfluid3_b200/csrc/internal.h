@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "../../include/ufem_b200.h"
+#include "persist.h"
 
 namespace ufem {
 
@@ -208,6 +209,15 @@ struct ufem_ns_handle {
   ufem::DirichletPlan bcp;
   ufem::StagePipe pipe;
   ufem::KrylovWork* kw = nullptr;
+  // One-launch solves (persist.cu): the plans of this system per operator type (FP64,
+  // FP32), without a coarse space and with one, and the coarse sizes they are for.
+  ufem::PersistPlan pplan[2][2];
+  int pplan_nc[2][2] = {{-1, -1}, {-1, -1}};
+  // Iterations of the previous BiCGStab and CG solves per operator type: how many are
+  // given to the device before the host's first look at the done flag, so a solve like
+  // the last one runs few iterations past its convergence and waits few times.
+  int bicg_expect[2] = {0, 0};
+  int cg_expect[2] = {0, 0};
   int persist_polls = -1;               // limit of a one-launch solve's barriers (below 0: kPersistPolls)
   bool vals32_valid = false;            // d_vals32 holds the current system (written by the assembly)
 

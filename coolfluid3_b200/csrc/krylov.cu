@@ -56,15 +56,6 @@ struct KrylovWork {
   };
   CGGraph cg_graph[2];
   CGGraph bicg_graph[2];   // the same for BiCGStab
-  // Iterations of the previous BiCGStab solve per operator type: the host's
-  // first look at the done flag comes after that many (rounded down to a
-  // graph block), so a solve like the last one launches few iterations past
-  // its convergence.
-  int bicg_expect[2] = {0, 0};
-  int cg_expect[2] = {0, 0};   // the same for CG
-  // One-launch solves (persist.cu) per operator type: the plan of this system.
-  PersistPlan pplan[2];
-  int pplan_nc[2] = {-1, -1};  // the coarse aggregates it has room for (-1: no plan yet)
   bool use_graph = true;   // false for the allocation-free solve (instantiation allocates)
   cudaStream_t capture_stream = nullptr;
   int cg_nblk = 0;             // blocks of the fused CG kernels (more than nblk: they are latency-bound)
@@ -1306,15 +1297,6 @@ int gmres(ufem_ns_handle* h, const MT* vals, const BT* b, VT* x, VT* V, VT* w, V
   }
 }
 
-// The persistent solver's plan for this system and operator type (persist.cu).
-const PersistPlan& persist_plan_of(ufem_ns_handle* h, KrylovWork& kw, bool f32, int nc) {
-  if (kw.pplan_nc[f32] != nc) {
-    kw.pplan[f32] = persist_plan(h->start_h.data(), h->adj_h.data(), h->N, h->neq, f32, nc);
-    kw.pplan_nc[f32] = nc;
-  }
-  return kw.pplan[f32];
-}
-
 // Runs a one-launch solve to its end: kPersistIters iterations a launch (the
 // other streams' kernels get the SMs in between), as many launches as the
 // previous solve needed before the host's first look at the flags.
@@ -1397,7 +1379,7 @@ int bicgstab(ufem_ns_handle* h, KrylovWork& kw, const MT* vals, const BT* b, VT*
   const double alpha_max = std::is_same<VT, float>::value ? 1e20 : 1e150;
   if (pkind != 2) {
     const bool f32 = std::is_same<MT, float>::value;
-    const PersistPlan& plan = persist_plan_of(h, kw, f32, pkind == 3 || pkind == 4 ? kw.nc : 0);
+    const PersistPlan& plan = persist_plan_of(h, f32, pkind == 3 || pkind == 4 ? kw.nc : 0);
     if (plan.form != kPersistNone) {
       PersistSolve a = persist_args<MT>(h, kw, vals, b, x, pkind, tol, maxit);
       a.r = r;
@@ -1409,7 +1391,7 @@ int bicgstab(ufem_ns_handle* h, KrylovWork& kw, const MT* vals, const BT* b, VT*
       a.q2 = two ? ph : p;
       a.t = tv;
       a.alpha_max = alpha_max;
-      return solve_persist(kw, a, plan, false, kw.bicg_expect[f32], st, res);
+      return solve_persist(kw, a, plan, false, h->bicg_expect[f32], st, res);
     }
   }
   if ((rc = setup_precond<VT, MT>(h, pkind, vals, dinv, st))) return rc;
@@ -1501,7 +1483,7 @@ int bicgstab(ufem_ns_handle* h, KrylovWork& kw, const MT* vals, const BT* b, VT*
   // long solves, little overshoot on short ones or ones like the last
   // (iterations after convergence return at once on the device flag, so the
   // cadence changes no result).
-  int& expect = kw.bicg_expect[std::is_same<MT, float>::value ? 1 : 0];
+  int& expect = h->bicg_expect[std::is_same<MT, float>::value ? 1 : 0];
   int check = std::max(kBlock, expect / kBlock * kBlock);
   for (int it = 0, next = kBlock; it < maxit; it += check, check = next, next = std::min(2 * next, 64)) {
     for (int k = 0; k < check; k += kBlock) {
@@ -1602,7 +1584,7 @@ int cg(ufem_ns_handle* h, KrylovWork& kw, const MT* vals, const BT* b, VT* x, VT
   int rc;
   if (pkind != 2) {
     const bool f32 = std::is_same<MT, float>::value;
-    const PersistPlan& plan = persist_plan_of(h, kw, f32, pkind == 3 || pkind == 4 ? kw.nc : 0);
+    const PersistPlan& plan = persist_plan_of(h, f32, pkind == 3 || pkind == 4 ? kw.nc : 0);
     if (plan.form != kPersistNone) {
       PersistSolve a = persist_args<MT>(h, kw, vals, b, x, pkind, tol, maxit);
       a.r = r;
@@ -1610,7 +1592,7 @@ int cg(ufem_ns_handle* h, KrylovWork& kw, const MT* vals, const BT* b, VT* x, VT
       a.v = z;
       a.r2 = a.nc > 0 ? dinv : r;
       a.t = q;
-      return solve_persist(kw, a, plan, true, kw.cg_expect[f32], st, res);
+      return solve_persist(kw, a, plan, true, h->cg_expect[f32], st, res);
     }
   }
   if ((rc = setup_precond<VT, MT>(h, pkind, vals, dinv, st))) return rc;
@@ -1665,7 +1647,7 @@ int cg(ufem_ns_handle* h, KrylovWork& kw, const MT* vals, const BT* b, VT* x, VT
   }
   // first look at the done flag after the previous solve's iteration count
   // (rounded down to a block), then after 1, 2, 4 and at most 8 more blocks
-  int& expect = kw.cg_expect[std::is_same<MT, float>::value ? 1 : 0];
+  int& expect = h->cg_expect[std::is_same<MT, float>::value ? 1 : 0];
   int reps = std::max(1, expect / kCGBlock);
   for (int it = 0, next = 1; it < maxit; it += reps * kCGBlock, reps = next, next = std::min(2 * next, 8)) {
     for (int k = 0; k < reps; ++k) UFEM_CUDA_TRY(cudaGraphLaunch(gr.exec, st));
@@ -1856,12 +1838,18 @@ int krylov_prepare(ufem_ns_handle* h, const ufem_krylov_opts* ko, int batched) {
     if (o.mixed != 0 && (rc = dalloc(&h->d_vals32, size_t(h->nnz)))) return rc;
   }
   KrylovWork& kw = *h->kw;
-  if (o.precond == 4 && h->neq > 1) {
+  const bool two = o.precond == 4 && h->neq > 1;
+  if (two) {
     const int s2 = batched ? kBatchCoarseSide2D : kCoarseSide2D, s3 = batched ? kBatchCoarseSide3D : kCoarseSide3D;
     if ((kw.cp_bc_version != h->bc_list_version || kw.cp_caps != s2 * 1000 + s3) &&
         (rc = coupled_coarse_build(h, s2, s3)))
       return rc;
   }
+  // the plan of the first solve: FP64 operator, or FP32 in the inner solves of the mixed
+  // forms (in a batch: of the matrix-free one)
+  const bool f32 = batched ? o.mixed == 2 : o.mixed != 0;
+  if (o.method != 0 && o.precond != 2 && o.precond != 3 && !(batched && o.mixed == 1))
+    persist_plan_of(h, f32, two ? kw.nc : 0);
   return UFEM_OK;
 }
 

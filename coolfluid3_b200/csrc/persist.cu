@@ -1210,7 +1210,8 @@ int launch_any(const PersistSolve& a, const PersistPlan& plan, bool first, int i
 
 }  // namespace
 
-PersistPlan persist_plan(const int64_t* start_h, const int32_t* adj_h, int64_t N, int neq, bool f32, int nc) {
+// start_h, adj_h: the node graph on the host; nc: aggregates of the coarse space.
+static PersistPlan persist_plan(const int64_t* start_h, const int32_t* adj_h, int64_t N, int neq, bool f32, int nc) {
   PersistPlan p;
   int dev = 0, sms = 0, coop = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -1272,6 +1273,16 @@ PersistPlan persist_plan(const int64_t* start_h, const int32_t* adj_h, int64_t N
     p.form = kPersistGrid;
     p.blocks = G;
     p.smem = kSmemMax;  // what the lists and vectors leave holds values
+  }
+  return p;
+}
+
+const PersistPlan& persist_plan_of(ufem_ns_handle* h, bool f32, int nc) {
+  PersistPlan& p = h->pplan[f32][nc > 0];
+  int& planned = h->pplan_nc[f32][nc > 0];
+  if (planned != nc) {
+    p = persist_plan(h->start_h.data(), h->adj_h.data(), h->N, h->neq, f32, nc);
+    planned = nc;
   }
   return p;
 }

@@ -5,6 +5,8 @@
 
 #include <cstdint>
 
+struct ufem_ns_handle;
+
 namespace ufem {
 
 // Scalar slots of a solve's dctl array, shared with the multi-launch solvers.
@@ -69,8 +71,9 @@ struct PersistPlan {
   size_t smem = 0;
 };
 
-// start_h, adj_h: the node graph on the host; nc: aggregates of the coarse space.
-PersistPlan persist_plan(const int64_t* start_h, const int32_t* adj_h, int64_t N, int neq, bool f32, int nc);
+// The handle's plan for its FP64 or FP32 operator and nc aggregates of a coarse space,
+// made where it is first asked for (a walk over the graph on the host) and kept.
+const PersistPlan& persist_plan_of(ufem_ns_handle* h, bool f32, int nc);
 // Up to `iters` iterations (first: from the initial residual of x; otherwise
 // continuing the stored state).  When the solve ends in this launch, the true
 // residual norm is left in dctl[kTrue].

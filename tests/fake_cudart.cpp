@@ -7,7 +7,9 @@
 //    next legacy copy waits for the earlier ones, a synchronisation for all; work
 //    given to another stream while one is in flight is counted as a fault;
 //  - one-launch Krylov solves: a launch of persist_kernel reports the end of its
-//    solve in the flags, or, where the test says so, that its barrier ran out of time.
+//    solve in the flags, or, where the test says so, that its barrier ran out of time;
+//    the plans made for them are counted (each asks once whether the device can do
+//    cooperative launches).
 //
 // A device-to-host copy of a single double reads 1.
 #include <cuda_runtime.h>
@@ -19,7 +21,7 @@
 
 namespace {
 int g_pending = 0, g_faults = 0;
-int g_launches = 0, g_late_at = -1, g_iters = 1;
+int g_launches = 0, g_late_at = -1, g_iters = 1, g_plans = 0;
 void landed() { g_pending = 0; }
 void uses(cudaStream_t s) {
   if (s != nullptr && g_pending > 0) ++g_faults;
@@ -36,6 +38,11 @@ int fake_faults() {
   return f;
 }
 int fake_launches() { return g_launches; }
+int fake_plans() {
+  const int n = g_plans;
+  g_plans = 0;
+  return n;
+}
 // The launches of one-launch solves from now on report `iters` iterations and the end
 // of the solve; the one numbered late_at (from 0; -1: none) a late barrier instead.
 void fake_solves(int iters, int late_at) {
@@ -114,6 +121,7 @@ cudaError_t cudaGetDeviceProperties_v2(cudaDeviceProp* p, int) {
 }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
   *v = a == cudaDevAttrMultiProcessorCount ? 148 : 1;
+  if (a == cudaDevAttrCooperativeLaunch) ++g_plans;
   return cudaSuccess;
 }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void*, int, size_t, unsigned) {

@@ -118,3 +118,38 @@ def test_a_late_barrier_of_any_launch_is_an_error(runtime):
             raise AssertionError(f"launch {late} was late and the solve succeeded")
         assert fake.fake_launches() == 3
     """)
+
+
+@pytest.mark.parametrize("precond", ["jacobi", "two_level_coupled"])
+def test_a_system_is_planned_once(runtime, precond):
+    """The plan of a one-launch solve (a walk over the graph on the host) is made by
+    prepare_solve, and by nothing after it: not the first solve, not a solve without
+    allocation, not a new batch with the same members."""
+    run(runtime, f"""
+    from coolfluid3_b200 import _native, krylov_options
+    kr = dict(precond="{precond}", max_iters=20)
+    ns, _ = solver(2, 80)
+    ns.prepare_solve(**kr)
+    assert fake.fake_plans() == 1
+    ns.assemble()
+    ns.apply_dirichlet()
+    ns.solve(**kr)
+    assert fake.fake_plans() == 0
+    st = _native.KrylovStatus()
+    plain = krylov_options(precond="jacobi", max_iters=20)
+    for k in range(3):
+        _native.lib().ufem_ns_solve_noalloc(ns.handle, ctypes.byref(plain), ctypes.byref(st), None)
+    assert fake.fake_plans() == (0 if "{precond}" == "jacobi" else 1)
+
+    for mixed in (False, "matrix_free"):
+        ms = [solver(2, n)[0] for n in (8, 80)]
+        for m in ms:
+            m.prepare_solve(batched=True, mixed=mixed, **kr)
+        assert fake.fake_plans() == 2
+        for k in range(2):
+            b = Batch(ms)
+            b.assemble()
+            b.solve(mixed=mixed, **kr)
+            b.close()
+        assert fake.fake_plans() == 0
+    """)
