@@ -695,8 +695,9 @@ __global__ void zero_x_if_b0_kernel(const Chunk* __restrict__ chunks, const Batc
 }
 
 __global__ void zero_batch_kernel(const Chunk* __restrict__ chunks, const BatchMesh* __restrict__ bm,
-                                  double* __restrict__ a, double* __restrict__ b) {
+                                  double* __restrict__ a, double* __restrict__ b, const int* __restrict__ ictl) {
   const Chunk c = chunks[blockIdx.x];
+  if (ictl[c.mesh * kIc + fDone]) return;
   const int64_t off = bm[c.mesh].row_off;
 #pragma unroll 4
   for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x) {
@@ -841,10 +842,11 @@ struct ufem_batch {
   PersistSolve* d_solves = nullptr;
   double* p_dctl = nullptr;
   int* p_ictl = nullptr;
-  std::vector<int> p_flags;
+  PersistSolve* h_solves = nullptr;  // pinned
+  int* p_flags = nullptr;  // pinned host copy of p_ictl
   // launches of different cluster sizes run beside each other
-  cudaStream_t side[4] = {};
-  cudaEvent_t fork = nullptr, join[4] = {};
+  cudaStream_t side[5] = {};
+  cudaEvent_t fork = nullptr, join[5] = {};
   // matrix-free refinement (mixed = 2): the members' FP64 residuals, the inner
   // solve's right-hand sides (residual / its norm) and corrections
   double *mfr = nullptr, *mfb = nullptr, *mfz = nullptr;
@@ -871,6 +873,8 @@ void batch_free(ufem_batch* b) {
   dfr(b->d_solves); dfr(b->p_dctl); dfr(b->p_ictl);
   if (b->h_dctl) cudaFreeHost(b->h_dctl);
   if (b->h_ictl) cudaFreeHost(b->h_ictl);
+  if (b->p_flags) cudaFreeHost(b->p_flags);
+  if (b->h_solves) cudaFreeHost(b->h_solves);
   delete b;
 }
 
@@ -1034,39 +1038,47 @@ int residual_b(ufem_batch* b, double* x, double* bw, bool init_rh, bool skip_don
   return UFEM_OK;
 }
 
-// Solves the members in `todo` that fit one cluster, one cluster each, all at once
-// (launches by cluster size); the others are left in `todo`.  The choice and the
-// arithmetic depend on the member alone.  The chunk kernels are bound by launches
+// Starts the solves of the members in `todo` that fit one cluster, one cluster each, all
+// at once (launches by cluster size): solved[m] is set and todo[m] cleared.  The choice
+// and the arithmetic depend on the member alone.  The chunk kernels are bound by launches
 // (55 us an iteration for 8 members of 40^2 cells, 27 blocks busy); in a cluster an
-// iteration costs its four barriers and the member's product, about 9 us, and
-// clusters need no one else: 10.2 -> 1.9 ms a time step of those 8 members.  solved[m] is set, and p_flags holds their
-// flags (8 ints a member: done, -, status, iterations).
+// iteration costs its barriers (three; seven with the coarse correction) and the member's
+// products, about 9 us, and clusters need no one else: 10.2 -> 1.9 ms a time step of those
+// 8 members.  Where members are left for the chunk kernels, `st` stays free for them and
+// every launch goes to a side stream; otherwise the largest clusters run on `st`.  The side
+// streams start after what `st` holds; end_clusters makes `st` wait for them.
 template <typename MT>
-int solve_in_clusters(ufem_batch* b, int pkind, double tol, int maxit, double* xw, double* bw, std::vector<int>& todo,
-                      std::vector<int>& solved, cudaStream_t st) {
+int start_clusters(ufem_batch* b, int pkind, double tol, int maxit, double* xw, double* bw, std::vector<int>& todo,
+                   std::vector<int>& solved, int* aside, cudaStream_t st) {
   constexpr bool f32 = std::is_same<MT, float>::value;
   const int n = b->nmesh;
-  std::vector<PersistSolve> list;
   std::vector<int64_t> off(size_t(n) + 1, 0);
   for (int m = 0; m < n; ++m) off[size_t(m) + 1] = off[size_t(m)] + b->members[m]->nrows;
   int rc;
-  if (!b->d_solves && ((rc = dmal(&b->d_solves, size_t(n))) || (rc = dmal(&b->p_dctl, size_t(16) * n)) ||
-                       (rc = dmal(&b->p_ictl, size_t(8) * n))))
-    return rc;
+  if (!b->h_solves) {
+    if ((!b->d_solves && (rc = dmal(&b->d_solves, size_t(n)))) || (!b->p_dctl && (rc = dmal(&b->p_dctl, size_t(16) * n))) ||
+        (!b->p_ictl && (rc = dmal(&b->p_ictl, size_t(8) * n))))
+      return rc;
+    DeviceLock lk(device_mutex());
+    if (!b->p_flags) UFEM_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&b->p_flags), sizeof(int) * 8 * n));
+    UFEM_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&b->h_solves), sizeof(PersistSolve) * n));
+  }
+  int count = 0;  // solves listed
   struct Group {
     int blocks, first, count;
     size_t smem;
   };
   std::vector<Group> groups;
   for (int blocks = 1; blocks <= 16; blocks *= 2) {
-    Group g{blocks, int(list.size()), 0, 0};
+    Group g{blocks, count, 0, 0};
     for (int m = 0; m < n; ++m) {
       if (!todo[m]) continue;
       ufem_ns_handle* h = b->members[m];
       const CoarseView cv = pkind == 4 && m < int(b->coarse.size()) ? b->coarse[m] : CoarseView{};
       const PersistPlan& plan = persist_plan_of(h, f32, cv.nc);
       if (plan.form != kPersistCluster || plan.blocks != blocks) continue;
-      PersistSolve a;
+      PersistSolve& a = b->h_solves[count++];
+      a = PersistSolve{};
       a.N = h->N;
       a.neq = h->neq;
       a.start = h->d_start;
@@ -1091,49 +1103,54 @@ int solve_in_clusters(ufem_batch* b, int pkind, double tol, int maxit, double* x
       a.tol = tol;
       a.alpha_max = 1e150;
       a.maxit = maxit;
-      list.push_back(a);
       ++g.count;
       g.smem = std::max(g.smem, plan.smem);
       solved[m] = 1;
     }
     if (g.count > 0) groups.push_back(g);
   }
-  if (list.empty()) return UFEM_OK;
-  UFEM_CUDA_TRY(cudaMemcpyAsync(b->d_solves, list.data(), list.size() * sizeof(PersistSolve), cudaMemcpyHostToDevice, st));
+  if (count == 0) return UFEM_OK;
+  bool rest = false;
+  for (int m = 0; m < n; ++m) {
+    if (solved[m]) todo[m] = 0;
+    rest = rest || todo[m];
+  }
+  UFEM_CUDA_TRY(cudaMemcpyAsync(b->d_solves, b->h_solves, count * sizeof(PersistSolve), cudaMemcpyHostToDevice, st));
   UFEM_CUDA_TRY(cudaMemsetAsync(b->p_ictl, 0, sizeof(int) * 8 * n, st));
-  // the largest clusters on `st`, the other sizes on side streams that start after
-  // what `st` holds and that `st` waits for
-  if (groups.size() > 1) {
+  const int nside = int(groups.size()) - (rest ? 0 : 1);
+  if (nside > 0) {
     DeviceLock lk(device_mutex());
     int prio = 0;
     UFEM_CUDA_TRY(cudaStreamGetPriority(st, &prio));
     if (!b->fork) UFEM_CUDA_TRY(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
-    for (size_t k = 0; k + 1 < groups.size(); ++k) {
+    for (int k = 0; k < nside; ++k) {
       if (!b->side[k]) UFEM_CUDA_TRY(cudaStreamCreateWithPriority(&b->side[k], cudaStreamNonBlocking, prio));
       if (!b->join[k]) UFEM_CUDA_TRY(cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming));
     }
     UFEM_CUDA_TRY(cudaEventRecord(b->fork, st));
   }
-  rc = UFEM_OK;
-  for (size_t k = groups.size(); k-- > 0;) {
-    const Group& g = groups[k];
-    const bool aside = k + 1 < groups.size();
-    const cudaStream_t q = aside ? b->side[k] : st;
-    if (aside) UFEM_CUDA_TRY(cudaStreamWaitEvent(q, b->fork, 0));
-    const int lrc = persist_bicgstab_members(b->d_solves + g.first, g.count, b->neq, f32, g.blocks, g.smem,
-                                             std::max(1, maxit), q);
-    if (lrc) rc = lrc;
-    if (aside) {
+  for (int k = int(groups.size()) - 1; k >= 0; --k) {
+    const Group& g = groups[size_t(k)];
+    const cudaStream_t q = k < nside ? b->side[k] : st;
+    if (k < nside) UFEM_CUDA_TRY(cudaStreamWaitEvent(q, b->fork, 0));
+    rc = persist_bicgstab_members(b->d_solves + g.first, g.count, b->neq, f32, g.blocks, g.smem, std::max(1, maxit), q);
+    if (k < nside) {
       UFEM_CUDA_TRY(cudaEventRecord(b->join[k], q));
-      UFEM_CUDA_TRY(cudaStreamWaitEvent(st, b->join[k], 0));
+      ++*aside;
     }
+    if (rc) return rc;
   }
-  if (rc) return rc;
-  b->p_flags.resize(size_t(8) * n);
-  UFEM_CUDA_TRY(cudaMemcpyAsync(b->p_flags.data(), b->p_ictl, sizeof(int) * 8 * n, cudaMemcpyDeviceToHost, st));
+  return UFEM_OK;
+}
+
+// `st` waits for the side streams' solves (also where their call fails: they use the
+// members' arrays), whose flags land in p_flags (8 ints a member: done, -, status,
+// iterations).
+int end_clusters(ufem_batch* b, int aside, cudaStream_t st) {
+  for (int k = 0; k < 5; ++k)
+    if (aside > 0 && b->join[k]) UFEM_CUDA_TRY(cudaStreamWaitEvent(st, b->join[k], 0));
+  UFEM_CUDA_TRY(cudaMemcpyAsync(b->p_flags, b->p_ictl, sizeof(int) * 8 * b->nmesh, cudaMemcpyDeviceToHost, st));
   UFEM_CUDA_TRY(cudaStreamSynchronize(st));
-  for (int m = 0; m < n; ++m)
-    if (solved[m]) todo[m] = 0;
   return UFEM_OK;
 }
 
@@ -1147,18 +1164,19 @@ int bicgstab_chunks(ufem_batch* b, int pkind, double tol, int maxit, bool use_ou
   const unsigned nc = unsigned(b->nchunks);
   const unsigned gm = blocks_for(int64_t(b->nmesh) * 32, 256);
   int rc;
-  // every mesh takes part in the set-up (flags are reset by the init kernel)
-  if (use_outer)  // flags prepared by the caller in the host mirror: fOuter set, the rest zero
+  // every mesh takes part in the set-up (flags are reset by the init kernel), except
+  // those that arrive done: they are being solved elsewhere
+  if (use_outer)  // flags prepared by the caller in the host mirror: fOuter, and fDone as well where solved elsewhere
     UFEM_CUDA_TRY(cudaMemcpyAsync(b->ictl, b->h_ictl, sizeof(int) * kIc * b->nmesh, cudaMemcpyHostToDevice, st));
   else
     UFEM_CUDA_TRY(cudaMemsetAsync(b->ictl, 0, sizeof(int) * kIc * b->nmesh, st));
   if (pkind == 1 || pkind == 4)
     jacobi_batch_kernel<MT><<<nc, kThreads, 0, st>>>(b->d_chunks, b->d_mesh, b->dinv, b->ictl);
   // the initial residual is FP64 in a mixed solve (residual replacement)
-  if ((rc = reliable ? residual_b<double, XL, BL>(b, xw, bw, true, false, st)
-                     : residual_b<MT, XL, BL>(b, xw, bw, true, false, st)))
+  if ((rc = reliable ? residual_b<double, XL, BL>(b, xw, bw, true, true, st)
+                     : residual_b<MT, XL, BL>(b, xw, bw, true, true, st)))
     return rc;
-  zero_batch_kernel<<<nc, kThreads, 0, st>>>(b->d_chunks, b->d_mesh, b->p, b->v);
+  zero_batch_kernel<<<nc, kThreads, 0, st>>>(b->d_chunks, b->d_mesh, b->p, b->v, b->ictl);
   bicg_init_batch_kernel<<<gm, 256, 0, st>>>(b->nmesh, b->d_cprefix, b->part, b->nchunks, b->dctl, b->ictl, tol,
                                              maxit, use_outer ? 1 : 0);
   zero_x_if_b0_kernel<XL><<<nc, kThreads, 0, st>>>(b->d_chunks, b->d_mesh, xw, b->dctl, b->ictl, use_outer ? 1 : 0);
@@ -1236,9 +1254,11 @@ int bicgstab_chunks(ufem_batch* b, int pkind, double tol, int maxit, bool use_ou
   return UFEM_OK;
 }
 
-// The same with the members that fit one cluster solved there, and the others, if
-// any, by the chunk kernels.  Leaves every member's flags in b->ictl.  The mixed form
-// with residual replacement (`reliable`) runs in the chunk kernels alone.
+// The same with the members that fit one cluster solved there, and the others, if any,
+// by the chunk kernels beside them (one after the other, 8 members of 55 to 90 cells a
+// side took 26.8 ms a step, 24.6 with the chunk kernels alone).  Leaves every member's
+// flags in b->ictl.  The mixed form with residual replacement (`reliable`) runs in the
+// chunk kernels alone.
 template <typename MT, int XL, int BL>
 int bicgstab_b(ufem_batch* b, int pkind, double tol, int maxit, bool use_outer, int slot, cudaStream_t st,
                bool reliable = false, double* xw = nullptr, double* bw = nullptr) {
@@ -1250,23 +1270,25 @@ int bicgstab_b(ufem_batch* b, int pkind, double tol, int maxit, bool use_outer, 
       outer[m] = b->h_ictl[m * kIc + fOuter];
       todo[m] = outer[m] ? 0 : 1;
     }
-  int rc;
-  if ((rc = solve_in_clusters<MT>(b, pkind, tol, maxit, xw, bw, todo, solved, st))) return rc;
+  int aside = 0, rc = start_clusters<MT>(b, pkind, tol, maxit, xw, bw, todo, solved, &aside, st);
   bool any_solved = false, rest = false;
   for (int m = 0; m < n; ++m) {
     any_solved = any_solved || solved[m];
     rest = rest || todo[m];
   }
-  if (!any_solved) return bicgstab_chunks<MT, XL, BL>(b, pkind, tol, maxit, use_outer, slot, st, false, xw, bw);
-  if (rest) {
+  if (!rc && !any_solved)
+    return bicgstab_chunks<MT, XL, BL>(b, pkind, tol, maxit, use_outer, slot, st, false, xw, bw);
+  if (!rc && rest) {
     for (int m = 0; m < n; ++m) {
       for (int q = 0; q < kIc; ++q) b->h_ictl[m * kIc + q] = 0;
       b->h_ictl[m * kIc + fOuter] = todo[m] ? 0 : 1;
+      b->h_ictl[m * kIc + fDone] = solved[m];
     }
-    if ((rc = bicgstab_chunks<MT, XL, BL>(b, pkind, tol, maxit, true, slot, st, false, xw, bw))) return rc;
-    UFEM_CUDA_TRY(cudaMemcpyAsync(b->h_ictl, b->ictl, sizeof(int) * kIc * n, cudaMemcpyDeviceToHost, st));
-    UFEM_CUDA_TRY(cudaStreamSynchronize(st));
-  } else {
+    rc = bicgstab_chunks<MT, XL, BL>(b, pkind, tol, maxit, true, slot, st, false, xw, bw);
+  }
+  const int erc = end_clusters(b, aside, st);
+  if (rc || erc) return rc ? rc : erc;
+  if (!rest) {  // (the chunk kernels' loop leaves its members' flags in h_ictl)
     for (int m = 0; m < n; ++m)
       for (int q = 0; q < kIc; ++q) b->h_ictl[m * kIc + q] = 0;
   }

@@ -9,23 +9,30 @@
 //  - one-launch Krylov solves: a launch of persist_kernel reports the end of its
 //    solve in the flags, or, where the test says so, that its barrier ran out of time;
 //    the plans made for them are counted (each asks once whether the device can do
-//    cooperative launches).
+//    cooperative launches);
+//  - what the streams are given: a graph (G), one-cluster solves of a batch (C), a
+//    wait of the host (S).
 //
 // A device-to-host copy of a single double reads 1.
 #include <cuda_runtime.h>
 
 #include <cstdlib>
 #include <cstring>
+#include <string>
 
 #include "persist.h"
 
 namespace {
 int g_pending = 0, g_faults = 0;
 int g_launches = 0, g_late_at = -1, g_iters = 1, g_plans = 0;
+std::string g_log;
+constexpr uintptr_t kTestStream = 4096;  // the stream that tests pass
 void landed() { g_pending = 0; }
 void uses(cudaStream_t s) {
   if (s != nullptr && g_pending > 0) ++g_faults;
 }
+// upper case on the test's stream, lower case on another
+void note(char c, cudaStream_t s) { g_log += reinterpret_cast<uintptr_t>(s) == kTestStream ? c : char(c + 32); }
 }  // namespace
 
 extern "C" {
@@ -42,6 +49,12 @@ int fake_plans() {
   const int n = g_plans;
   g_plans = 0;
   return n;
+}
+const char* fake_log() {
+  static std::string out;
+  out.swap(g_log);
+  g_log.clear();
+  return out.c_str();
 }
 // The launches of one-launch solves from now on report `iters` iterations and the end
 // of the solve; the one numbered late_at (from 0; -1: none) a late barrier instead.
@@ -87,6 +100,7 @@ cudaError_t cudaDeviceSynchronize() {
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) {
   if (s == nullptr) landed();
+  note('S', s);
   return cudaSuccess;
 }
 cudaError_t cudaLaunchKernel(const void*, dim3, dim3, void**, size_t, cudaStream_t st) {
@@ -95,7 +109,10 @@ cudaError_t cudaLaunchKernel(const void*, dim3, dim3, void**, size_t, cudaStream
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void*, void** args) {
   uses(c->stream);
-  if (*static_cast<int*>(args[1]) != int(c->dynamicSmemBytes)) return cudaSuccess;  // not persist_kernel
+  if (*static_cast<int*>(args[1]) != int(c->dynamicSmemBytes)) {  // not persist_kernel: its form for batches
+    note('C', c->stream);
+    return cudaSuccess;
+  }
   const ufem::PersistSolve& a = *static_cast<const ufem::PersistSolve*>(args[0]);
   const bool late = g_launches++ == g_late_at;
   if (late) a.ictl[ufem::kFlagLate] = 1;
@@ -184,6 +201,7 @@ cudaError_t cudaGraphExecDestroy(cudaGraphExec_t e) {
 }
 cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t s) {
   uses(s);
+  note('G', s);
   return cudaSuccess;
 }
 

@@ -153,3 +153,26 @@ def test_a_system_is_planned_once(runtime, precond):
             b.close()
         assert fake.fake_plans() == 0
     """)
+
+
+def test_batch_members_of_both_forms_run_beside_each_other(runtime):
+    """Members that fit a cluster and members that do not, in one batch: the clusters go to
+    streams of their own and the others' iterations are given to the caller's stream
+    before the host waits for anything; without such others the largest clusters run on
+    the caller's stream."""
+    run(runtime, """
+    fake.fake_log.restype = ctypes.c_char_p
+    kr = dict(precond="jacobi", max_iters=8)
+    def log(sizes):
+        b = Batch([solver(2, n)[0] for n in sizes])
+        b.assemble(STREAM)
+        fake.fake_log()
+        b.solve(STREAM, **kr)
+        return fake.fake_log().decode()
+    both = log([6, 140, 20])
+    first = min(both.index(c) for c in "cC" if c in both)
+    assert "C" not in both
+    assert "G" in both[first:].split("S")[0], both
+    small = log([6, 20])
+    assert "C" in small and "G" not in small.split("C")[1].split("S")[0], small
+    """)
