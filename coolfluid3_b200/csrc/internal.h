@@ -218,7 +218,7 @@ struct ufem_ns_handle {
   // the last one runs few iterations past its convergence and waits few times.
   int bicg_expect[2] = {0, 0};
   int cg_expect[2] = {0, 0};
-  int persist_polls = -1;               // limit of a one-launch solve's barriers (below 0: kPersistPolls)
+  bool persist_stuck = false;           // PersistSolve::stuck of the handle's solves
   bool vals32_valid = false;            // d_vals32 holds the current system (written by the assembly)
 
   // transfer staging (reference field layouts <-> padded node records)

@@ -1362,7 +1362,7 @@ PersistSolve persist_args(const ufem_ns_handle* h, const KrylovWork& kw, const M
   a.ictl = kw.ictl;
   a.tol = tol;
   a.maxit = maxit;
-  if (h->persist_polls >= 0) a.polls = h->persist_polls;
+  a.stuck = h->persist_stuck;
   return a;
 }
 
@@ -2200,9 +2200,9 @@ int noalloc_scratch(double** out) {
 
 }  // namespace ufem
 
-// For tests of the error path: polls after which a barrier of the handle's one-launch
-// solves gives up (below 0: the usual limit).
-extern "C" void ufem_ns_limit_barriers(ufem_ns_handle* h, int polls) { h->persist_polls = polls; }
+// For tests of the error path: the grid barriers of the handle's one-launch solves wait for
+// an arrival that never comes, and run out of time.
+extern "C" void ufem_ns_stick_barriers(ufem_ns_handle* h, int on) { h->persist_stuck = on != 0; }
 
 extern "C" int ufem_ns_solve_noalloc(ufem_ns_handle* h, const ufem_krylov_opts* kopts, ufem_krylov_status* status,
                                      void* stream) {

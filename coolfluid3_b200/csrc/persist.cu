@@ -232,7 +232,7 @@ struct Ctx {
           const int target = epoch * blocks;
           int spins = 0, late = 0;
           while (ld_acquire(a.ictl + kFlagBarrier) < target)
-            if (++spins > a.polls) {
+            if (++spins > kPersistPolls) {
               late = 1;
               break;
             }
@@ -1148,7 +1148,8 @@ int launch(const PersistSolve& a, const PersistPlan& plan, bool first, int iters
   }
   // the barrier counter of every launch; a late barrier stays on record to the solve's end
   if (first) UFEM_CUDA_TRY(cudaMemsetAsync(a.ictl + kFlagLate, 0, 2 * sizeof(int), s));
-  else if (!CL) UFEM_CUDA_TRY(cudaMemsetAsync(a.ictl + kFlagBarrier, 0, sizeof(int), s));
+  if (!CL && (!first || a.stuck))
+    UFEM_CUDA_TRY(cudaMemsetAsync(a.ictl + kFlagBarrier, a.stuck ? 0xff : 0, sizeof(int), s));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(unsigned(plan.blocks));
   cfg.blockDim = dim3(kThreads);

@@ -21,17 +21,17 @@ def system(dim, n, **kw):
     return ns
 
 
-def limit_barriers(ns, polls):
-    f = _native.lib().ufem_ns_limit_barriers
+def stick_barriers(ns, on):
+    f = _native.lib().ufem_ns_stick_barriers
     f.argtypes, f.restype = [ctypes.c_void_p, ctypes.c_int], None
-    f(ns._h, polls)
+    f(ns._h, on)
 
 
 @pytest.mark.parametrize("precond", ["jacobi", "two_level_coupled"])
 def test_a_barrier_that_runs_out_ends_the_solve_with_an_error(precond):
-    """96 x 96 cells (the grid form).  A barrier that gives up at its first look ends the
-    launch and those queued behind it (the solve before took more than one), the call
-    fails, and the next solve gives the bits of the first."""
+    """96 x 96 cells (the grid form).  A barrier that waits in vain gives up after some
+    seconds, which ends its launch and those queued behind it (the solve before took more
+    than one), the call fails, and the next solve gives the bits of the first."""
     ns = system(2, 96)
     start = ns.solution()
     kr = dict(precond=precond, tol=1e-11, max_iters=6000)
@@ -39,10 +39,10 @@ def test_a_barrier_that_runs_out_ends_the_solve_with_an_error(precond):
     x = ns.solution()
     assert precond != "jacobi" or st["iterations"] > 256
     ns.set_solution(start)
-    limit_barriers(ns, 0)
+    stick_barriers(ns, 1)
     with pytest.raises(UfemError, match="barrier"):
         ns.solve(**kr)
-    limit_barriers(ns, -1)
+    stick_barriers(ns, 0)
     ns.set_solution(start)
     again = ns.solve(**kr)
     assert again["iterations"] == st["iterations"]
