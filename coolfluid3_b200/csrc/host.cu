@@ -106,26 +106,21 @@ void dfree(T*& p) {
 }
 
 // The warp kernel's static lists; a second pass writes the contributor lists of
-// items with more than 7 contributors, where there are any.
+// items with more than 7 contributors, where there are any.  The transfer staging
+// holds the counter: freeing one would wait for the whole device.
 int build_assembly_lists(ufem_ns_handle* h, cudaStream_t s) {
-  unsigned* used = nullptr;
-  int rc;
-  if ((rc = dmalloc(&used, 1, "list counter"))) return rc;
+  unsigned* used = reinterpret_cast<unsigned*>(h->d_stage);
   unsigned n = 0;
-  cudaError_t ce = cudaMemsetAsync(used, 0, sizeof(unsigned), s);
-  if (ce == cudaSuccess && (rc = launch_assembly_items(h, used, s)) == UFEM_OK) {
-    ce = cudaMemcpyAsync(&n, used, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
-    if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
-    if (ce == cudaSuccess && n > 0 && (rc = dmalloc(&h->d_over, n, "long item lists")) == UFEM_OK) {
-      h->over_bytes = n;
-      ce = cudaMemsetAsync(used, 0, sizeof(unsigned), s);
-      if (ce == cudaSuccess && (rc = launch_assembly_items(h, used, s)) == UFEM_OK) ce = cudaStreamSynchronize(s);
-    }
-  }
-  dfree(used);
-  if (rc) return rc;
-  if (ce != cudaSuccess) return set_error(UFEM_ERR_CUDA, std::string("assembly lists: ") + cudaGetErrorString(ce));
-  return UFEM_OK;
+  int rc;
+  UFEM_CUDA_TRY(cudaMemsetAsync(used, 0, sizeof(unsigned), s));
+  if ((rc = launch_assembly_items(h, used, s))) return rc;
+  UFEM_CUDA_TRY(cudaMemcpyAsync(&n, used, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+  UFEM_CUDA_TRY(cudaStreamSynchronize(s));
+  if (n == 0) return UFEM_OK;
+  if ((rc = dmalloc(&h->d_over, n, "long item lists"))) return rc;
+  h->over_bytes = n;
+  UFEM_CUDA_TRY(cudaMemsetAsync(used, 0, sizeof(unsigned), s));
+  return launch_assembly_items(h, used, s);  // (the caller waits for the stream)
 }
 
 int validate_options(const ufem_ns_options* o) {

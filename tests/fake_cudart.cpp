@@ -11,7 +11,8 @@
 //    the plans made for them are counted (each asks once whether the device can do
 //    cooperative launches);
 //  - what the streams are given: a graph (G), one-cluster solves of a batch (C), a
-//    wait of the host (S).
+//    wait of the host (S);
+//  - frees, each of which waits for the whole device.
 //
 // A device-to-host copy of a single double reads 1.
 #include <cuda_runtime.h>
@@ -24,7 +25,7 @@
 
 namespace {
 int g_pending = 0, g_faults = 0;
-int g_launches = 0, g_late_at = -1, g_iters = 1, g_plans = 0;
+int g_launches = 0, g_late_at = -1, g_iters = 1, g_plans = 0, g_frees = 0;
 std::string g_log;
 constexpr uintptr_t kTestStream = 4096;  // the stream that tests pass
 void landed() { g_pending = 0; }
@@ -50,6 +51,11 @@ int fake_plans() {
   g_plans = 0;
   return n;
 }
+int fake_frees() {
+  const int n = g_frees;
+  g_frees = 0;
+  return n;
+}
 const char* fake_log() {
   static std::string out;
   out.swap(g_log);
@@ -68,6 +74,7 @@ void fake_solves(int iters, int late_at) {
 cudaError_t cudaMalloc(void** p, size_t n) { return (*p = std::calloc(n + 32, 1)) ? cudaSuccess : cudaErrorMemoryAllocation; }
 cudaError_t cudaMallocHost(void** p, size_t n) { return cudaMalloc(p, n); }
 cudaError_t cudaFree(void* p) {
+  if (p) ++g_frees;
   std::free(p);
   return cudaSuccess;
 }

@@ -176,3 +176,13 @@ def test_batch_members_of_both_forms_run_beside_each_other(runtime):
     small = log([6, 20])
     assert "C" in small and "G" not in small.split("C")[1].split("S")[0], small
     """)
+
+
+def test_creation_does_not_free(runtime):
+    """Building a handle does not hold up what other threads have on the device: it frees
+    nothing (a free waits for all of it)."""
+    run(runtime, """
+    fake.fake_frees()
+    kept = [solver(dim, n, precision=p) for dim, n in ((2, 12), (3, 5)) for p in ("fp64", "fp32")]
+    assert fake.fake_frees() == 0
+    """)
