@@ -1175,6 +1175,13 @@ void fill_params(const ufem_ns_handle* h, NSParams& p) {
   p.has_force = h->d_force != nullptr;
 }
 
+// Without rows of more than 24 incidences the 24-lane plan serves the "warp" variant of
+// tetrahedra too: less staging a warp leaves the L1 more of the SM's array (the rows'
+// values are the same bits under both plans).
+bool warp_takes_24(const ufem_ns_handle* h) {
+  return h->dim == 3 && h->wplan24.big64.nchunks == 0 && h->wplan24.ngroups > 0;
+}
+
 // Whether the handle's element routine is the general one (another tau than METRIC).
 bool assembly_general(const ufem_ns_handle* h) { return h->opt.use_specializations == 0 && h->opt.supg_type != 1; }
 
@@ -1213,13 +1220,22 @@ int launch_chunk_g(const ufem_ns_handle* h, const AssemblyPlan& plan, const NSPa
   return UFEM_OK;
 }
 
+// f with the element routine of the handle as a type; the specialised form has one only.
+template <bool SPEC, typename F>
+int with_gen(const ufem_ns_handle* h, F&& f) {
+  if constexpr (!SPEC)
+    if (assembly_general(h)) return f(std::true_type{});
+  return f(std::false_type{});
+}
+
 template <int D, typename T, int CH, bool SPEC>
 int launch_chunk_t(const ufem_ns_handle* h, const AssemblyPlan& plan, const NSParams& p, cudaStream_t s,
                    bool write32) {
   if (plan.nchunks == 0) return UFEM_OK;
   if (plan.cap != CH) return set_error(UFEM_ERR_STATE, "assembly plan does not match the kernel width");
-  return assembly_general(h) ? launch_chunk_g<D, T, CH, SPEC, true>(h, plan, p, s, write32)
-                             : launch_chunk_g<D, T, CH, SPEC, false>(h, plan, p, s, write32);
+  return with_gen<SPEC>(h, [&](auto gen) {
+    return launch_chunk_g<D, T, CH, SPEC, decltype(gen)::value>(h, plan, p, s, write32);
+  });
 }
 
 // Resident CTAs of a kernel on the current device (persistent-warp grids).
@@ -1265,21 +1281,17 @@ int launch_assembly_t(ufem_ns_handle* h, cudaStream_t s, bool write32) {
   constexpr bool f32 = std::is_same<T, float>::value;
   if (h->asm_variant == kAsmChunk) return launch_chunk_t<D, T, CH, SPEC>(h, f32 ? h->plan32 : h->plan64, p, s, write32);
   int rc;
-  // Without rows of more than 24 incidences the 24-lane plan serves the "warp"
-  // variant too: less staging a warp leaves the L1 more of the SM's array (the rows'
-  // values are the same bits under both plans).
-  const bool w24 = D == 3 && (h->asm_variant == kAsmWarp24 || (h->wplan24.big64.nchunks == 0 && h->wplan24.ngroups > 0));
+  const bool w24 = D == 3 && (h->asm_variant == kAsmWarp24 || warp_takes_24(h));
   const WarpPlan& wp = w24 ? h->wplan24 : h->wplan;
   AsmDesc one;  // this handle's descriptor, passed as a kernel parameter
   fill_desc(h, write32, one, &wp);
-  auto run = [&](auto gen) {
+  rc = with_gen<SPEC>(h, [&](auto gen) {
     constexpr bool G = decltype(gen)::value;
     if constexpr (D == 3) {
       if (w24) return launch_warp_w<D, T, SPEC, G, false, 24>(h->asm_warps, wp.ngroups, 1, nullptr, nullptr, one, s);
     }
     return launch_warp_w<D, T, SPEC, G, false, 32>(h->asm_warps, wp.ngroups, 1, nullptr, nullptr, one, s);
-  };
-  rc = one.gen ? run(std::true_type{}) : run(std::false_type{});
+  });
   if (rc) return rc;
   return launch_chunk_t<D, T, CH, SPEC>(h, f32 ? wp.big32 : wp.big64, p, s, write32);
 }
@@ -1315,7 +1327,8 @@ int set_smem_attr_g() {
 template <int D, typename T, int CH, bool SPEC>
 int set_smem_attr() {
   const int rc = set_smem_attr_g<D, T, CH, SPEC, false>();
-  return rc ? rc : set_smem_attr_g<D, T, CH, SPEC, true>();
+  if constexpr (SPEC) return rc;
+  else return rc ? rc : set_smem_attr_g<D, T, CH, SPEC, true>();
 }
 
 // ---------------------------------------------------------------------------
@@ -1430,13 +1443,13 @@ int launch_residual_t(ufem_ns_handle* h, const double* dxp, double* res, cudaStr
   NSParams p;
   fill_params(h, p);
   if (h->plan64.cap != CH) return set_error(UFEM_ERR_STATE, "chunk plan does not match the residual kernel width");
-  const bool gen = !SPEC && h->opt.supg_type != 1;
-  auto kernel = gen ? ns_residual_kernel<D, CH, SPEC, true> : ns_residual_kernel<D, CH, SPEC, false>;
-  kernel<<<h->plan64.nchunks, CH, 0, s>>>(h->plan64.chunks, h->d_row_inc, h->d_inc_elem, h->d_inc_info,
-                                          reinterpret_cast<const int4*>(h->d_conn), h->d_coords, h->d_uadv,
-                                          h->d_state, h->d_force, p, dxp, res);
-  UFEM_CUDA_TRY(cudaGetLastError());
-  return UFEM_OK;
+  return with_gen<SPEC>(h, [&](auto gen) {
+    ns_residual_kernel<D, CH, SPEC, decltype(gen)::value><<<h->plan64.nchunks, CH, 0, s>>>(
+        h->plan64.chunks, h->d_row_inc, h->d_inc_elem, h->d_inc_info, reinterpret_cast<const int4*>(h->d_conn),
+        h->d_coords, h->d_uadv, h->d_state, h->d_force, p, dxp, res);
+    UFEM_CUDA_TRY(cudaGetLastError());
+    return int(UFEM_OK);
+  });
 }
 
 constexpr int kChunk2D = 256;
@@ -1488,8 +1501,9 @@ int launch_batch_t(int warps, int kinds, int ngroups, int nmesh, const AsmDesc* 
   int rc;
   if ((kinds & 1) && (rc = launch_warp_w<D, T, SPEC, false, true>(warps, ngroups, nmesh, d_descs, d_gprefix, AsmDesc{}, s)))
     return rc;
-  if ((kinds & 2) && (rc = launch_warp_w<D, T, SPEC, true, true>(warps, ngroups, nmesh, d_descs, d_gprefix, AsmDesc{}, s)))
-    return rc;
+  if constexpr (!SPEC)
+    if ((kinds & 2) && (rc = launch_warp_w<D, T, SPEC, true, true>(warps, ngroups, nmesh, d_descs, d_gprefix, AsmDesc{}, s)))
+      return rc;
   return UFEM_OK;
 }
 }  // namespace

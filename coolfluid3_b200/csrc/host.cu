@@ -937,7 +937,7 @@ int ufem_ns_device_bytes(const ufem_ns_handle* h, int64_t* bytes) {
   b += krylov_device_bytes(h);  // solver workspace allocated so far (none for a batch member's vectors)
   if (h->pipe.buf[0]) b += 2 * (N * (h->neq + 4 * h->dim + 1) + R) * 8;  // overlapped-transfer buffers, once used
   if (h->d_tie) b += h->ntie * 8;
-  b += h->bcp.nbc * 40 + h->bcp.nfix_rows * 16 + h->bcp.nfix * 12;
+  b += h->bcp.nbc * 44 + h->bcp.nfix_rows * 16 + h->bcp.nfix * 12;
   *bytes = b;
   return UFEM_OK;
 }
@@ -1190,7 +1190,7 @@ int ufem_ns_tune_assembly(ufem_ns_handle* h, void* stream, int32_t reps, int32_t
   const bool w32 = h->d_vals32 != nullptr;
   struct Cand { int variant, warps; };
   std::vector<Cand> cands = {{kAsmWarp, 2}, {kAsmWarp, 4}, {kAsmWarp, 8}, {kAsmChunk, 4}};
-  if (h->dim == 3) {
+  if (h->dim == 3 && !warp_takes_24(h)) {  // (otherwise the same launches)
     cands.push_back({kAsmWarp24, 2});
     cands.push_back({kAsmWarp24, 4});
   }

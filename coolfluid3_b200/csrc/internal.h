@@ -244,6 +244,7 @@ void fill_desc(const ufem_ns_handle* h, bool write32, AsmDesc& d, const WarpPlan
 // (the lists are written where d_over is allocated).
 int launch_assembly_items(ufem_ns_handle* h, unsigned* over_used, cudaStream_t s);
 bool assembly_general(const ufem_ns_handle* h);
+bool warp_takes_24(const ufem_ns_handle* h);
 // Warp assembly of many meshes in one persistent launch per kind of element routine
 // (kinds: bit 0 METRIC, bit 1 general; same dim and precision;
 // rows with more than 32 incidences go through each mesh's chunk plan).
