@@ -219,6 +219,7 @@ struct ufem_ns_handle {
   int bicg_expect[2] = {0, 0};
   int cg_expect[2] = {0, 0};
   bool persist_stuck = false;           // PersistSolve::stuck of the handle's solves
+  int persist_iters = 256;              // iterations a launch of a one-launch solve runs
   bool vals32_valid = false;            // d_vals32 holds the current system (written by the assembly)
 
   // transfer staging (reference field layouts <-> padded node records)

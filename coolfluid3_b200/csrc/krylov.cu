@@ -1297,18 +1297,18 @@ int gmres(ufem_ns_handle* h, const MT* vals, const BT* b, VT* x, VT* V, VT* w, V
   }
 }
 
-// Runs a one-launch solve to its end: kPersistIters iterations a launch (the
-// other streams' kernels get the SMs in between), as many launches as the
-// previous solve needed before the host's first look at the flags.
-constexpr int kPersistIters = 256;
-int solve_persist(KrylovWork& kw, const PersistSolve& a, const PersistPlan& plan, bool use_cg, int& expect,
-                  cudaStream_t st, SolveResult& res) {
+// Runs a one-launch solve to its end: 256 iterations a launch (the other streams'
+// kernels get the SMs in between), as many launches as the previous solve needed
+// before the host's first look at the flags.
+int solve_persist(const ufem_ns_handle* h, KrylovWork& kw, const PersistSolve& a, const PersistPlan& plan, bool use_cg,
+                  int& expect, cudaStream_t st, SolveResult& res) {
+  const int per = h->persist_iters;
   res = SolveResult();
   int rc;
   bool first = true;
-  for (int reps = 1 + std::max(0, expect - 1) / kPersistIters, run = 0; run < a.maxit || first; reps = 1) {
-    for (int k = 0; k < reps; ++k, run += kPersistIters) {
-      rc = use_cg ? persist_cg(a, plan, first, kPersistIters, st) : persist_bicgstab(a, plan, first, kPersistIters, st);
+  for (int reps = 1 + std::max(0, expect - 1) / per, run = 0; run < a.maxit || first; reps = 1) {
+    for (int k = 0; k < reps; ++k, run += per) {
+      rc = use_cg ? persist_cg(a, plan, first, per, st) : persist_bicgstab(a, plan, first, per, st);
       if (rc) return rc;
       first = false;
     }
@@ -1391,7 +1391,7 @@ int bicgstab(ufem_ns_handle* h, KrylovWork& kw, const MT* vals, const BT* b, VT*
       a.q2 = two ? ph : p;
       a.t = tv;
       a.alpha_max = alpha_max;
-      return solve_persist(kw, a, plan, false, h->bicg_expect[f32], st, res);
+      return solve_persist(h, kw, a, plan, false, h->bicg_expect[f32], st, res);
     }
   }
   if ((rc = setup_precond<VT, MT>(h, pkind, vals, dinv, st))) return rc;
@@ -1592,7 +1592,7 @@ int cg(ufem_ns_handle* h, KrylovWork& kw, const MT* vals, const BT* b, VT* x, VT
       a.v = z;
       a.r2 = a.nc > 0 ? dinv : r;
       a.t = q;
-      return solve_persist(kw, a, plan, true, h->cg_expect[f32], st, res);
+      return solve_persist(h, kw, a, plan, true, h->cg_expect[f32], st, res);
     }
   }
   if ((rc = setup_precond<VT, MT>(h, pkind, vals, dinv, st))) return rc;
@@ -2199,6 +2199,9 @@ int noalloc_scratch(double** out) {
 }  // namespace
 
 }  // namespace ufem
+
+// For tests of solves that take several launches: the iterations of each.
+extern "C" void ufem_ns_launch_iterations(ufem_ns_handle* h, int iters) { h->persist_iters = iters; }
 
 // For tests of the error path: the grid barriers of the handle's one-launch solves wait for
 // an arrival that never comes, and run out of time.

@@ -1192,4 +1192,7 @@ int64_t ufem_nssi_device_bytes(const ufem_nssi_handle* h) {
   return bytes + N * (3 * D + 2) * 8;  // inner-loop vectors
 }
 
+// For tests of solves that take several launches: the iterations of each.
+void ufem_nssi_launch_iterations(ufem_nssi_handle* h, int iters) { h->us->persist_iters = h->ps->persist_iters = iters; }
+
 }  // extern "C"
