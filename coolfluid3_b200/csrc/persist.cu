@@ -1224,6 +1224,27 @@ int launch_any(const PersistSolve& a, const PersistPlan& plan, bool first, int i
 
 }  // namespace
 
+// Whether the device can run a cluster of C blocks (a part of one may not hold 16 SMs that
+// share a cluster); every kernel of the cluster form needs the same of it.
+static bool cluster_runs(int C, size_t smem) {
+  auto kernel = persist_kernel<false, 4, double, true>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemMax)) != cudaSuccess ||
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+    return false;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(C));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = unsigned(C);
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int n = 0;
+  return cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0;
+}
+
 // start_h, adj_h: the node graph on the host; nc: aggregates of the coarse space.
 static PersistPlan persist_plan(const int64_t* start_h, const int32_t* adj_h, int64_t N, int neq, bool f32, int nc) {
   PersistPlan p;
@@ -1276,6 +1297,7 @@ static PersistPlan persist_plan(const int64_t* start_h, const int32_t* adj_h, in
     if (C < kClusterMax && N > int64_t(C) * per * 2) continue;
     if (size_t(bytes / C) > kSmemMax) continue;
     if (const size_t s = needs(C, true)) {
+      if (!cluster_runs(C, s)) continue;
       p.form = kPersistCluster;
       p.blocks = C;
       p.smem = s;

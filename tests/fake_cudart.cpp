@@ -11,7 +11,7 @@
 //    the plans made for them are counted (each asks once whether the device can do
 //    cooperative launches);
 //  - what the streams are given: a graph (G), one-cluster solves of a batch (C), a
-//    wait of the host (S);
+//    cluster (P) or a grid (R) that solves one system, a wait of the host (S);
 //  - frees, each of which waits for the whole device.
 //
 // A device-to-host copy of a single double reads 1.
@@ -25,7 +25,7 @@
 
 namespace {
 int g_pending = 0, g_faults = 0;
-int g_launches = 0, g_late_at = -1, g_iters = 1, g_plans = 0, g_frees = 0;
+int g_launches = 0, g_late_at = -1, g_iters = 1, g_plans = 0, g_frees = 0, g_clusters = 8;
 std::string g_log;
 constexpr uintptr_t kTestStream = 4096;  // the stream that tests pass
 void landed() { g_pending = 0; }
@@ -56,6 +56,8 @@ int fake_frees() {
   g_frees = 0;
   return n;
 }
+// Clusters that the device can run at once.
+void fake_clusters(int n) { g_clusters = n; }
 const char* fake_log() {
   static std::string out;
   out.swap(g_log);
@@ -121,6 +123,7 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void*, void**
     return cudaSuccess;
   }
   const ufem::PersistSolve& a = *static_cast<const ufem::PersistSolve*>(args[0]);
+  note(c->attrs[0].id == cudaLaunchAttributeCooperative ? 'R' : 'P', c->stream);
   const bool late = g_launches++ == g_late_at;
   if (late) a.ictl[ufem::kFlagLate] = 1;
   a.ictl[0] = late ? 0 : 1;
@@ -150,6 +153,10 @@ cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
 }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void*, int, size_t, unsigned) {
   *n = 1;
+  return cudaSuccess;
+}
+cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void*, const cudaLaunchConfig_t*) {
+  *n = g_clusters;
   return cudaSuccess;
 }
 cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return cudaSuccess; }

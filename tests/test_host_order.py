@@ -186,3 +186,27 @@ def test_creation_does_not_free(runtime):
     kept = [solver(dim, n, precision=p) for dim, n in ((2, 12), (3, 5)) for p in ("fp64", "fp32")]
     assert fake.fake_frees() == 0
     """)
+
+
+def test_a_device_without_room_for_a_cluster_solves_on_the_grid(runtime):
+    """A system that would take one cluster goes to the grid where the device cannot run the
+    cluster, and a batch's members to the chunk kernels."""
+    run(runtime, """
+    fake.fake_log.restype = ctypes.c_char_p
+    def solved(clusters):
+        fake.fake_clusters(clusters)
+        ns, _ = solver(2, 12)
+        ns.assemble(STREAM)
+        ns.apply_dirichlet(STREAM)
+        fake.fake_log()
+        ns.solve(STREAM, precond="jacobi")
+        one = fake.fake_log().decode()
+        b = Batch([solver(2, 12)[0]])
+        b.assemble(STREAM)
+        b.solve(STREAM, precond="jacobi", max_iters=8)
+        return one, fake.fake_log().decode()
+    one, batch = solved(8)
+    assert "P" in one and "C" in batch and "G" not in batch
+    one, batch = solved(0)
+    assert "R" in one and "P" not in one and "C" not in batch and "G" in batch
+    """)
