@@ -9,7 +9,8 @@
 // invdt*T + theta*A and the neq entries of -A*x + a -- and stages it in shared
 // memory.  Phase 2: one thread per (row, neighbour slot, equation) sums the
 // staged contributions of the row's incidences in ascending element order (the
-// order in which the reference adds them) and writes each CSR value exactly
+// order in which the reference adds them; the warp kernel's tetrahedra: another
+// fixed order of the row's elements) and writes each CSR value exactly
 // once, coalesced.  No floating-point atomics, no element matrices in HBM.
 #include <cuda_runtime.h>
 
@@ -699,8 +700,10 @@ __global__ void __launch_bounds__(CH) ns_assembly_kernel(
 // static words instead of masks built by shared-memory atomics, and the smaller
 // staging leaves room for 16 warps (128 registers) where 12 fitted.  64^3 x 6 on a
 // B200, before -> after: FP64 generic 0.737 -> 0.591 ms, specialised 0.843 -> 0.530,
-// FP32 generic 0.545 -> 0.457; 301^2 x 2 triangles in random order, FP64 generic 52.0
-// -> 51.5 us, specialised 53.3 -> 45.4.
+// FP32 generic 0.545 -> 0.457; 301^2 x 2 triangles in random order, FP64 generic 45.6
+// -> 42.2 us, specialised 50.1 -> 41.7, FP32 42.1 -> 43.3 and 41.5 -> 43.3 (the words and
+// diagonal places are 50 MB more to read at 1000^2, and FP32 writes two copies of the
+// values).
 // ---------------------------------------------------------------------------
 constexpr size_t kDescSlot = (sizeof(AsmDesc) + 15) / 16 * 16;
 
@@ -715,8 +718,9 @@ constexpr size_t warp_stage_bytes() {
 // Resident-CTA hints (register budgets): warps an SM.  64^3 x 6, generic, 4-warp
 // CTAs: FP64 0.595 ms at 16 warps, 0.737 at 12 and 0.771 at 20 (spills); FP32 0.480 at
 // 16, 0.457 at 20.  The batched 3D FP64 kernel spills at 16 (its descriptors are in
-// shared memory), so it keeps 12.  Triangles, FP64: 51.5 us at 16, 60-76 at 20-24 (spills);
-// FP32 51.7 at 16, 48 at 24.
+// shared memory), so it keeps 12.  Triangles, FP64: 16 (20 and 24 spill and take a fifth to
+// a half longer); FP32, 1000^2 in natural order with the conditions: 497 us at 16 warps,
+// 455 at 20, 442 at 24 and 28.
 template <int D, typename T, bool BATCH, int WPB>
 constexpr int warp_min_blocks() {
   const int warps = D == 3 ? (sizeof(T) == 4 ? 20 : (BATCH ? 12 : 16)) : (sizeof(T) == 4 ? 24 : 16);

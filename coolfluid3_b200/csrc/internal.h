@@ -51,7 +51,8 @@ struct NSParams {
 };
 
 // Row-owner assembly plans.  Incidences (row node, element) are sorted by
-// (row node, element id), so each CSR entry is summed in element order.
+// (row node, element id), so each CSR entry is summed in an order that depends on
+// its row's elements alone (the chunk kernel's and the triangles': ascending).
 //  - chunk plan: ranges of whole rows whose incidences fit one CTA of `cap`
 //    threads (one thread per incidence);
 //  - warp plan: ranges of consecutive rows with at most 32 incidences in total,

@@ -31,11 +31,19 @@
 //
 // What bounds it: barriers and the latency of each phase, not bytes.  An
 // iteration, launches against this: 64 x 64 x 2 triangles, BiCGStab with point
-// Jacobi, 27 -> 9.3 us (cluster of 16); 24^3 x 6 tetrahedra, two-level BiCGStab,
-// 46 -> 22 us; 32^3 x 6, two-level CG of the pressure 29 -> 12 us, CG of the
-// velocity 24 -> 15 us (grid).  (With the restriction after the update and its own
+// Jacobi, 27 -> 9.1 us (cluster of 16); 24^3 x 6 tetrahedra, two-level BiCGStab,
+// 46 -> 21 us; 32^3 x 6, two-level CG of the pressure 29 -> 12.8 us, CG of the
+// velocity 24 -> 16.3 us (grid).  (With the restriction after the update and its own
 // barrier, and the coarse sums' last rows one at a time, the two-level forms took 27
 // and 13.5 us.)
+//
+// A block's rows are a range of node numbers, so a scattered numbering costs: a block
+// then touches 7 (triangles) to 14 (tetrahedra) times its own nodes instead of 2 to 5,
+// copies as many more a product, and has less room for values.  28^3 x 6 in random
+// order: point Jacobi 32.5 us an iteration (natural 23.0; launches 43.5), two-level
+// 45.0 (32.5; 67).  From 32^3 x 6 or 260^2 x 2 in random order the lists and vectors
+// no longer fit, and the launches take the system (natural order: up to the 96 MB of
+// persist_plan, triangles up to 360^2).
 //
 // All sums run in fixed orders, so a solve is deterministic; FP64 throughout,
 // FP32 only in the stored values of the mixed forms.  Grid barriers wait a
@@ -1253,9 +1261,12 @@ static PersistPlan persist_plan(const int64_t* start_h, const int32_t* adj_h, in
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop)
     return p;
-  // Above 96 MB of values the matrix streams from HBM and the launches' share is
-  // small (0.235 ms an iteration at 514 MB, 0.18 ms of it the products); the
-  // multi-launch products then run with more loads in flight.
+  // Above 96 MB of values the matrix no longer stays in L2 beside the rest, and the
+  // multi-launch products, with more loads in flight, make up for their launches.
+  // Tetrahedra in natural order, point Jacobi, us an iteration (launches / one): 36^3 x 6
+  // (89 MB) 60.5 / 43.9, 37^3 (96.3 MB) 61.4 / 54.8, 38^3 (104 MB) 64.3 / 65.1, 40^3
+  // (121 MB) 71.8 / 76.4.  Most systems end earlier, where a block's vectors and lists do
+  // not fit (needs, below).
   const int64_t vb = int64_t(neq) * neq * (f32 ? 4 : 8);
   const int npw = 32 / neq, sb = slice_bytes(neq, f32 ? 4 : 8);
   const int64_t bytes = start_h[N] * vb;

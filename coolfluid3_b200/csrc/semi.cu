@@ -26,7 +26,8 @@
 // lumped mass inverse) are node-major arrays of the same row numbering.
 //
 // Every element quantity is evaluated by the thread that owns the row (one
-// thread per node, its incidences in ascending element order), so each global
+// thread per node, its incidences in ascending element order; eight lanes a node
+// that add in that order for the velocity matrix), so each global
 // entry is a sum over elements in the order the reference adds them: no
 // atomics, deterministic results.  Linked (periodic) nodes keep identity rows
 // with a zero right-hand side; their values are copied from the master row
