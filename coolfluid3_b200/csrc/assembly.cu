@@ -701,9 +701,8 @@ __global__ void __launch_bounds__(CH) ns_assembly_kernel(
 // staging leaves room for 16 warps (128 registers) where 12 fitted.  64^3 x 6 on a
 // B200, before -> after: FP64 generic 0.737 -> 0.591 ms, specialised 0.843 -> 0.530,
 // FP32 generic 0.545 -> 0.457; 301^2 x 2 triangles in random order, FP64 generic 45.6
-// -> 42.2 us, specialised 50.1 -> 41.7, FP32 42.1 -> 43.3 and 41.5 -> 43.3 (the words and
-// diagonal places are 50 MB more to read at 1000^2, and FP32 writes two copies of the
-// values).
+// -> 42.2 us, specialised 50.1 -> 41.7; FP32 elements with the conditions 61.2 -> 51.5 and
+// 60.8 -> 49.3.
 // ---------------------------------------------------------------------------
 constexpr size_t kDescSlot = (sizeof(AsmDesc) + 15) / 16 * 16;
 
@@ -719,11 +718,12 @@ constexpr size_t warp_stage_bytes() {
 // CTAs: FP64 0.595 ms at 16 warps, 0.737 at 12 and 0.771 at 20 (spills); FP32 0.480 at
 // 16, 0.457 at 20.  The batched 3D FP64 kernel spills at 16 (its descriptors are in
 // shared memory), so it keeps 12.  Triangles, FP64: 16 (20 and 24 spill and take a fifth to
-// a half longer); FP32, 1000^2 in natural order with the conditions: 497 us at 16 warps,
-// 455 at 20, 442 at 24 and 28.
+// a half longer); FP32: 24 (fewer took longer: 455 us at 20 and 497 at 16 where 24 took
+// 442), batched 20 (at 24 the generic form spills: 8 meshes of 300^2 in random order 371
+// us, 326 at 20).
 template <int D, typename T, bool BATCH, int WPB>
 constexpr int warp_min_blocks() {
-  const int warps = D == 3 ? (sizeof(T) == 4 ? 20 : (BATCH ? 12 : 16)) : (sizeof(T) == 4 ? 24 : 16);
+  const int warps = D == 3 ? (sizeof(T) == 4 ? 20 : (BATCH ? 12 : 16)) : (sizeof(T) == 4 ? (BATCH ? 20 : 24) : 16);
   return warps / WPB > 0 ? warps / WPB : 1;
 }
 
@@ -865,45 +865,49 @@ __device__ __forceinline__ void reduce_rows_3d(const T* stage, const int* s_off,
 }
 
 // ... triangles: a lane an entry of the diagonal blocks and the RHS rows (summed
-// over the row's lanes), then a lane an off-diagonal block.
+// over the row's lanes), then a lane an off-diagonal block.  The values of a group are
+// one run of the CSR: with FP32 elements a group of usual size (five rows of six
+// elements, at most 32 off-diagonal blocks) puts them together over its records and
+// writes the run, FP64 and FP32 copy, lane by lane.  Written where they are summed, 24 and
+// 12 bytes a lane and row, every sector goes to L2 in three parts.  1000^2 in natural
+// order, with the conditions: FP32 generic 448 -> 406 us, specialised 437 -> 395, random
+// order 512 -> 481; FP64 elements, with one copy and fewer warps to hide the second pass
+// over shared memory behind, lose by it (471 -> 537) and write directly.
 template <typename T, typename F>
-__device__ __forceinline__ void reduce_rows_2d(const T* stage, const int* s_off, const int* s_start, int R, int row0,
+__device__ __forceinline__ void reduce_rows_2d(T* stage, const int* s_off, const int* s_start, int R, int row0,
                                                int64_t gstart, const unsigned long long* __restrict__ words,
                                                unsigned long long word, const AsmDesc& d, F&& next) {
   using L = RecordLayout<2, T>;
   constexpr int LS = L::pitch;
+  constexpr bool kRun = std::is_same<T, float>::value;
+  constexpr int kRows = 5, kBlocks = 32;  // of a group written as a run
+  static_assert((kRows + kBlocks) * 9 * sizeof(double) <= size_t(32) * LS * sizeof(T), "the run fits the records' place");
   const int lane = threadIdx.x & 31;
   double* __restrict__ vals = d.vals;
   float* __restrict__ vals32 = d.vals32;
-  for (int it = lane; it < R * 12; it += 32) {
+  const int nslot = s_start[R] - R;
+  const bool run = kRun && R <= kRows && nslot <= kBlocks;  // warp-uniform
+  double* out = reinterpret_cast<double*>(stage);
+  auto diagonal = [&](int it, bool& rhs, int64_t& pos) {  // entry it of the rows' 12: its sum and CSR or RHS place
     const int rl = it / 12, dl = it - rl * 12;
     const int64_t row = row0 + rl;
     const int er = dl / 3, ec = dl - er * 3;
-    int64_t pos = 0;
-    if (dl < 9) pos = __ldg(d.diagpos + row * 3 + er) - er + ec;
+    rhs = dl >= 9;
+    pos = rhs ? row * 3 + (dl - 9) : __ldg(d.diagpos + row * 3 + er) - er + ec;
     const T* q = stage + (dl < 9 ? dl : L::sums + dl - 9);
     double acc = 0.0;
     const int ke = s_off[rl + 1];
 #pragma unroll 4
     for (int k = s_off[rl]; k < ke; ++k) acc += double(q[k * LS]);
-    if (dl < 9) {
-      __stcs(vals + pos, acc);
-      if (vals32 != nullptr) __stcs(vals32 + pos, float(acc));
-    } else {
-      __stcs(d.rhs + row * 3 + (dl - 9), acc);
-    }
-  }
-  next();
-  const int nslot = s_start[R] - R;
-  for (int it = lane; it < nslot; it += 32) {
-    if (it >= 32) word = __ldg(words + it);
+    return acc;
+  };
+  auto off_diagonal = [&](double (&acc)[9], int64_t& pos, int& step) {  // the block of `word`, its place and row step
     const bool over = (word >> 63) != 0;
     const int rl = (int(word >> 58) - row0) & 31;
     const int slot = int(word >> 52) & 63;
     const int cnt = over ? int(word >> 32) & 0xff : int(word >> 49) & 7;
     const uint8_t* more = d.over + uint32_t(word);
     const T* base = stage + s_off[rl] * LS;
-    double acc[9];
 #pragma unroll
     for (int e = 0; e < 9; ++e) acc[e] = 0.0;
     unsigned long long list = word;
@@ -914,15 +918,69 @@ __device__ __forceinline__ void reduce_rows_2d(const T* stage, const int* s_off,
 #pragma unroll
       for (int e = 0; e < 9; ++e) acc[e] += double(q[e]);
     }
-    const int S = s_start[rl + 1] - s_start[rl];
-    const int64_t base0 = 9 * (gstart + s_start[rl]) + slot * 3;
+    pos = 9 * (gstart + s_start[rl]) + slot * 3;
+    step = (s_start[rl + 1] - s_start[rl]) * 3;
+  };
+  if (run) {
+    double dv[2] = {0.0, 0.0}, acc[9];
+    int at[3] = {-1, -1, 0}, step = 0;
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+      if (lane + 32 * q < R * 12) {
+        bool rhs;
+        int64_t pos;
+        dv[q] = diagonal(lane + 32 * q, rhs, pos);
+        if (rhs) __stcs(d.rhs + pos, dv[q]);
+        else at[q] = int(pos - 9 * gstart);
+      }
+    next();
+    if (lane < nslot) {
+      int64_t pos;
+      off_diagonal(acc, pos, step);
+      at[2] = int(pos - 9 * gstart);
+    }
+    __syncwarp();  // the records are summed
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+      if (at[q] >= 0) out[at[q]] = dv[q];
+    if (lane < nslot)
+#pragma unroll
+      for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) out[at[2] + r * step + c] = acc[r * 3 + c];
+    __syncwarp();
+    const int n = 9 * s_start[R];
+    for (int i = lane; i < n; i += 32) {
+      const double v = out[i];
+      __stcs(vals + 9 * gstart + i, v);
+      if (vals32 != nullptr) __stcs(vals32 + 9 * gstart + i, float(v));
+    }
+    return;
+  }
+  for (int it = lane; it < R * 12; it += 32) {
+    bool rhs;
+    int64_t pos;
+    const double acc = diagonal(it, rhs, pos);
+    if (rhs) {
+      __stcs(d.rhs + pos, acc);
+    } else {
+      __stcs(vals + pos, acc);
+      if (vals32 != nullptr) __stcs(vals32 + pos, float(acc));
+    }
+  }
+  next();
+  for (int it = lane; it < nslot; it += 32) {
+    if (it >= 32) word = __ldg(words + it);
+    double acc[9];
+    int64_t pos;
+    int step;
+    off_diagonal(acc, pos, step);
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const int64_t pos = base0 + int64_t(r) * S * 3 + c;
-        __stcs(vals + pos, acc[r * 3 + c]);
-        if (vals32 != nullptr) __stcs(vals32 + pos, float(acc[r * 3 + c]));
+        __stcs(vals + pos + r * step + c, acc[r * 3 + c]);
+        if (vals32 != nullptr) __stcs(vals32 + pos + r * step + c, float(acc[r * 3 + c]));
       }
   }
 }
