@@ -865,49 +865,45 @@ __device__ __forceinline__ void reduce_rows_3d(const T* stage, const int* s_off,
 }
 
 // ... triangles: a lane an entry of the diagonal blocks and the RHS rows (summed
-// over the row's lanes), then a lane an off-diagonal block.  The values of a group are
-// one run of the CSR: with FP32 elements a group of usual size (five rows of six
-// elements, at most 32 off-diagonal blocks) puts them together over its records and
-// writes the run, FP64 and FP32 copy, lane by lane.  Written where they are summed, 24 and
-// 12 bytes a lane and row, every sector goes to L2 in three parts.  1000^2 in natural
-// order, with the conditions: FP32 generic 448 -> 406 us, specialised 437 -> 395, random
-// order 512 -> 481; FP64 elements, with one copy and fewer warps to hide the second pass
-// over shared memory behind, lose by it (471 -> 537) and write directly.
+// over the row's lanes), then a lane an off-diagonal block.
 template <typename T, typename F>
-__device__ __forceinline__ void reduce_rows_2d(T* stage, const int* s_off, const int* s_start, int R, int row0,
+__device__ __forceinline__ void reduce_rows_2d(const T* stage, const int* s_off, const int* s_start, int R, int row0,
                                                int64_t gstart, const unsigned long long* __restrict__ words,
                                                unsigned long long word, const AsmDesc& d, F&& next) {
   using L = RecordLayout<2, T>;
   constexpr int LS = L::pitch;
-  constexpr bool kRun = std::is_same<T, float>::value;
-  constexpr int kRows = 5, kBlocks = 32;  // of a group written as a run
-  static_assert((kRows + kBlocks) * 9 * sizeof(double) <= size_t(32) * LS * sizeof(T), "the run fits the records' place");
   const int lane = threadIdx.x & 31;
   double* __restrict__ vals = d.vals;
   float* __restrict__ vals32 = d.vals32;
-  const int nslot = s_start[R] - R;
-  const bool run = kRun && R <= kRows && nslot <= kBlocks;  // warp-uniform
-  double* out = reinterpret_cast<double*>(stage);
-  auto diagonal = [&](int it, bool& rhs, int64_t& pos) {  // entry it of the rows' 12: its sum and CSR or RHS place
+  for (int it = lane; it < R * 12; it += 32) {
     const int rl = it / 12, dl = it - rl * 12;
     const int64_t row = row0 + rl;
     const int er = dl / 3, ec = dl - er * 3;
-    rhs = dl >= 9;
-    pos = rhs ? row * 3 + (dl - 9) : __ldg(d.diagpos + row * 3 + er) - er + ec;
+    int64_t pos = 0;
+    if (dl < 9) pos = __ldg(d.diagpos + row * 3 + er) - er + ec;
     const T* q = stage + (dl < 9 ? dl : L::sums + dl - 9);
     double acc = 0.0;
     const int ke = s_off[rl + 1];
 #pragma unroll 4
     for (int k = s_off[rl]; k < ke; ++k) acc += double(q[k * LS]);
-    return acc;
-  };
-  auto off_diagonal = [&](double (&acc)[9], int64_t& pos, int& step) {  // the block of `word`, its place and row step
+    if (dl < 9) {
+      __stcs(vals + pos, acc);
+      if (vals32 != nullptr) __stcs(vals32 + pos, float(acc));
+    } else {
+      __stcs(d.rhs + row * 3 + (dl - 9), acc);
+    }
+  }
+  next();
+  const int nslot = s_start[R] - R;
+  for (int it = lane; it < nslot; it += 32) {
+    if (it >= 32) word = __ldg(words + it);
     const bool over = (word >> 63) != 0;
     const int rl = (int(word >> 58) - row0) & 31;
     const int slot = int(word >> 52) & 63;
     const int cnt = over ? int(word >> 32) & 0xff : int(word >> 49) & 7;
     const uint8_t* more = d.over + uint32_t(word);
     const T* base = stage + s_off[rl] * LS;
+    double acc[9];
 #pragma unroll
     for (int e = 0; e < 9; ++e) acc[e] = 0.0;
     unsigned long long list = word;
@@ -918,70 +914,93 @@ __device__ __forceinline__ void reduce_rows_2d(T* stage, const int* s_off, const
 #pragma unroll
       for (int e = 0; e < 9; ++e) acc[e] += double(q[e]);
     }
-    pos = 9 * (gstart + s_start[rl]) + slot * 3;
-    step = (s_start[rl + 1] - s_start[rl]) * 3;
-  };
-  if (run) {
-    double dv[2] = {0.0, 0.0}, acc[9];
-    int at[3] = {-1, -1, 0}, step = 0;
-#pragma unroll
-    for (int q = 0; q < 2; ++q)
-      if (lane + 32 * q < R * 12) {
-        bool rhs;
-        int64_t pos;
-        dv[q] = diagonal(lane + 32 * q, rhs, pos);
-        if (rhs) __stcs(d.rhs + pos, dv[q]);
-        else at[q] = int(pos - 9 * gstart);
-      }
-    next();
-    if (lane < nslot) {
-      int64_t pos;
-      off_diagonal(acc, pos, step);
-      at[2] = int(pos - 9 * gstart);
-    }
-    __syncwarp();  // the records are summed
-#pragma unroll
-    for (int q = 0; q < 2; ++q)
-      if (at[q] >= 0) out[at[q]] = dv[q];
-    if (lane < nslot)
-#pragma unroll
-      for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) out[at[2] + r * step + c] = acc[r * 3 + c];
-    __syncwarp();
-    const int n = 9 * s_start[R];
-    for (int i = lane; i < n; i += 32) {
-      const double v = out[i];
-      __stcs(vals + 9 * gstart + i, v);
-      if (vals32 != nullptr) __stcs(vals32 + 9 * gstart + i, float(v));
-    }
-    return;
-  }
-  for (int it = lane; it < R * 12; it += 32) {
-    bool rhs;
-    int64_t pos;
-    const double acc = diagonal(it, rhs, pos);
-    if (rhs) {
-      __stcs(d.rhs + pos, acc);
-    } else {
-      __stcs(vals + pos, acc);
-      if (vals32 != nullptr) __stcs(vals32 + pos, float(acc));
-    }
-  }
-  next();
-  for (int it = lane; it < nslot; it += 32) {
-    if (it >= 32) word = __ldg(words + it);
-    double acc[9];
-    int64_t pos;
-    int step;
-    off_diagonal(acc, pos, step);
+    const int S = s_start[rl + 1] - s_start[rl];
+    const int64_t base0 = 9 * (gstart + s_start[rl]) + slot * 3;
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        __stcs(vals + pos + r * step + c, acc[r * 3 + c]);
-        if (vals32 != nullptr) __stcs(vals32 + pos + r * step + c, float(acc[r * 3 + c]));
+        const int64_t pos = base0 + int64_t(r) * S * 3 + c;
+        __stcs(vals + pos, acc[r * 3 + c]);
+        if (vals32 != nullptr) __stcs(vals32 + pos, float(acc[r * 3 + c]));
       }
+  }
+}
+
+// Triangles with FP32 elements.  The values of a group are one run of the CSR: a group of
+// usual size (five rows of six elements, at most 32 off-diagonal blocks) puts them
+// together over its records and writes the run, FP64 and FP32 copy, lane by lane.
+// Written where they are summed, 24 and 12 bytes a lane and row, every sector goes to L2
+// in three parts.  1000^2 in natural order, with the conditions: generic 448 -> 402 us,
+// specialised 437 -> 395, random order 512 -> 474.  FP64 elements, with one copy and fewer
+// warps to hide the second pass over shared memory behind, lose by it (471 -> 537) and
+// write directly.
+template <typename F>
+__device__ __forceinline__ void reduce_run_2d(float* stage, const int* s_off, const int* s_start, int R, int row0,
+                                              int64_t gstart, const unsigned long long* __restrict__ words,
+                                              unsigned long long word, const AsmDesc& d, F&& next) {
+  using L = RecordLayout<2, float>;
+  constexpr int LS = L::pitch;
+  constexpr int kRows = 5, kBlocks = 32;
+  static_assert((kRows + kBlocks) * 9 * sizeof(double) <= size_t(32) * LS * sizeof(float), "the run fits the records' place");
+  const int lane = threadIdx.x & 31;
+  const int nslot = s_start[R] - R;
+  if (R > kRows || nslot > kBlocks) {  // the whole warp
+    reduce_rows_2d<float>(stage, s_off, s_start, R, row0, gstart, words, word, d, next);
+    return;
+  }
+  double dv[2] = {0.0, 0.0}, acc[9];
+  int at[3] = {-1, -1, 0}, step = 0;  // places in the run
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int it = lane + 32 * h;
+    if (it >= R * 12) continue;
+    const int rl = it / 12, dl = it - rl * 12;
+    const int64_t row = row0 + rl;
+    const int er = dl / 3, ec = dl - er * 3;
+    if (dl < 9) at[h] = int(__ldg(d.diagpos + row * 3 + er) - er + ec - 9 * gstart);
+    const float* q = stage + (dl < 9 ? dl : L::sums + dl - 9);
+    const int ke = s_off[rl + 1];
+#pragma unroll 4
+    for (int k = s_off[rl]; k < ke; ++k) dv[h] += double(q[k * LS]);
+    if (dl >= 9) __stcs(d.rhs + row * 3 + (dl - 9), dv[h]);
+  }
+  next();
+  if (lane < nslot) {
+    const bool over = (word >> 63) != 0;
+    const int rl = (int(word >> 58) - row0) & 31;
+    const int cnt = over ? int(word >> 32) & 0xff : int(word >> 49) & 7;
+    const uint8_t* more = d.over + uint32_t(word);
+    const float* base = stage + s_off[rl] * LS;
+#pragma unroll
+    for (int e = 0; e < 9; ++e) acc[e] = 0.0;
+    unsigned long long list = word;
+#pragma unroll 1
+    for (int c = 0; c < cnt; ++c, list >>= 7) {
+      const int id = over ? int(__ldg(more + c)) : int(list & 127u);
+      const float* q = base + (id >> 2) * LS + (id & 3) * 9;
+#pragma unroll
+      for (int e = 0; e < 9; ++e) acc[e] += double(q[e]);
+    }
+    at[2] = 9 * s_start[rl] + (int(word >> 52) & 63) * 3;
+    step = (s_start[rl + 1] - s_start[rl]) * 3;
+  }
+  __syncwarp();  // the records are summed
+  double* out = reinterpret_cast<double*>(stage);
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    if (at[h] >= 0) out[at[h]] = dv[h];
+  if (lane < nslot)
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) out[at[2] + r * step + c] = acc[r * 3 + c];
+  __syncwarp();
+  const int n = 9 * s_start[R];
+  for (int i = lane; i < n; i += 32) {
+    const double v = out[i];
+    __stcs(d.vals + 9 * gstart + i, v);
+    if (d.vals32 != nullptr) __stcs(d.vals32 + 9 * gstart + i, float(v));
   }
 }
 
@@ -1115,8 +1134,11 @@ __global__ void __launch_bounds__(32 * WPB, warp_min_blocks<D, T, BATCH, WPB>())
       reduce_rows_3d<T, KC>(stage, s_off, s_start, R, row0, gstart, words, word, UFEM_DESC(cs),
                             [&] { if (lane < Gn.w) pcn = __ldg(UFEM_DESC(ns).conn + (pea & 0x3fffffffu)); });
     } else {
-      reduce_rows_2d<T>(stage, s_off, s_start, R, row0, gstart, words, word, UFEM_DESC(cs),
-                        [&] { if (lane < Gn.w) pcn = __ldg(UFEM_DESC(ns).conn + (pea & 0x3fffffffu)); });
+      auto next = [&] { if (lane < Gn.w) pcn = __ldg(UFEM_DESC(ns).conn + (pea & 0x3fffffffu)); };
+      if constexpr (std::is_same<T, float>::value)
+        reduce_run_2d(stage, s_off, s_start, R, row0, gstart, words, word, UFEM_DESC(cs), next);
+      else
+        reduce_rows_2d<T>(stage, s_off, s_start, R, row0, gstart, words, word, UFEM_DESC(cs), next);
     }
     if (gn >= ngroups) break;
     g = gn;
